@@ -10,7 +10,7 @@
 //
 // Two kernels:
 //  * kCollideGlobal -- one thread per sorted particle, neighbours read
-//    through the read-only cache.  Used for scenes that do not suit tiling.
+//    through the read-only cache (kCollideBatch is the same over many scenes).
 //  * kCollideTiled  -- a CTA takes 128 consecutive sorted particles, splits
 //    them into row groups (same (y, z) grid row), and for each group stages
 //    in shared memory the 9 neighbour-row windows of the cell tables and the
@@ -160,44 +160,44 @@ __device__ __forceinline__ CellCull makeCull(float3 p, int3 g, float R, const Si
   return c;
 }
 
-// Asynchronous 16-byte copy global -> shared (cp.async, completion per
-// thread by commit groups).
-__device__ __forceinline__ void copyAsync16(float4 *dst, const float4 *src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(__cvta_generic_to_global(src))
-               : "memory");
-}
-__device__ __forceinline__ void copyAsyncCommit() {
-  asm volatile("cp.async.commit_group;\n" ::: "memory");
-}
-template <int kPending>
-__device__ __forceinline__ void copyAsyncWait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(kPending) : "memory");
-}
-
 // Per-thread queue of near partners (shared memory, entry q of thread t at
 // [q * kQueueStride + t]).
-constexpr int kQueueLen = 16;
+constexpr int kQueueLen = 12;
 constexpr int kQueueStride = 128;
-constexpr int kStageLen = 128;  // staged partner positions per warp row buffer
 
-// The 27-cell loop with cell tables and positions read from global memory,
-// in two phases.  The scan over candidates only tests the squared distance
-// (see rejectBound) and queues the partners that may be in contact, with the
-// index of their neighbour cell; the queue is drained in order, where the
-// exact `dist < cd` test and the contact term run.  Contacts are thus
-// computed back to back instead of diverging inside the scan.  Sums: `cf`
-// gathers the terms of the current cell and is added to `force` when a
-// contact of a later cell arrives.  Cells without contacts would add +0.0,
-// which leaves a sum that started at +0.0 unchanged, so the result is the
-// reference's cell-by-cell sum.
+// Range [a, b) of cell h (empty: a == b).
+template <bool kPrefix>
+__device__ __forceinline__ void cellRange(unsigned h, const CellRanges &cells, unsigned n,
+                                          unsigned &a, unsigned &b) {
+  if (kPrefix) {
+    a = __ldg(cells.off + h);
+    b = min(__ldg(cells.off + h + 1), n);
+  } else {
+    a = __ldg(cells.start + h);
+    if (a == kEmpty) {
+      a = 0u;
+      b = 0u;
+    } else {
+      b = min(__ldg(cells.end + h), n);
+    }
+  }
+  if (b < a) b = a;
+}
+
+// The general 27-cell loop (any cell order, any cell tables, rows of any
+// length), for the particles that the mask scan below does not take.  The
+// scan over candidates only tests the squared distance (see rejectBound) and
+// queues the partners that may be in contact, with the index of their
+// neighbour cell; the queue is drained in order, where the exact `dist < cd`
+// test and the contact term run.  Sums: `cf` gathers the terms of the current
+// cell and is added to `force` when a contact of a later cell arrives.  Cells
+// without contacts would add +0.0, which leaves a sum that started at +0.0
+// unchanged, so the result is the reference's cell-by-cell sum.
 template <bool kRadiusFromW, bool kPrefix>
 __device__ __forceinline__ float3 neighbourForceGlobal(
     unsigned i, unsigned n, float3 pos, float3 vel, float ri, int3 g, bool cull,
     const float4 *__restrict__ sortedPos, const float4 *__restrict__ sortedVel,
-    const CellRanges &cells, const SimParams &P, unsigned *qj, unsigned char *qc,
-    float4 *stage = nullptr, unsigned live = 0u) {
+    const CellRanges &cells, const SimParams &P, unsigned *qj, unsigned char *qc) {
   const float cdMono = ri + P.particleRadius;
   const float cdMonoHi2 = rejectBound(cdMono);
   // largest contact distance: r_i + particleRadius (in the radius-from-w
@@ -234,55 +234,17 @@ __device__ __forceinline__ float3 neighbourForceGlobal(
     }
     qn = 0;
   };
-  // queue a near partner j of neighbour cell `cell` (0..26); load(j) gives
-  // the position of sorted particle j (global or the warp's staged copy)
-  auto scanRange = [&](unsigned a, unsigned b, int cellA, unsigned m1, unsigned m2, auto load) {
-    // cells cellA, cellA+1, cellA+2 hold [a, m1), [m1, m2), [m2, b).
-    // Two candidates per iteration: their dependent test chains overlap
-    // (0.778 against 0.810 ms of collide per 4.2M-sphere step early in the
-    // packed job; unrolled by 4, or with more registers by a minimum-blocks
-    // launch bound, it is slower).
-#pragma unroll 2
-    for (unsigned j = a; j < b; j++) {
-      float4 q4 = load(j);
-      float3 rel = make_float3(q4.x - pos.x, q4.y - pos.y, q4.z - pos.z);
-      float d2 = pairDist2(rel);
-      float hi2 = kRadiusFromW ? rejectBound(ri + q4.w) : cdMonoHi2;
-      if (d2 < hi2 && j != i) {
-        if (qn == kQueueLen) drain();
-        qj[qn * kQueueStride] = j;
-        qc[qn * kQueueStride] = (unsigned char)(cellA + (j >= m1) + (j >= m2));
-        ++qn;
-      }
-    }
-  };
-  auto loadGlobal = [&](unsigned j) { return ldg4(sortedPos + j); };
-  // one row's three cells one by one (the x wrap, Morton order or the split
-  // cellStart/cellEnd tables)
-  auto cellRow = [&](int row) {
+#pragma unroll 1
+  for (int row = 0; row < 9; row++) {
     const int z = row / 3 - 1, y = row % 3 - 1;
     const float rowD2 = CellCull::pick(z, cc.zl, cc.zh) + CellCull::pick(y, cc.yl, cc.yh);
-    if (rowD2 > cullR2) return;
-    unsigned h[3], start[3], end[3];
-#pragma unroll
+    if (rowD2 > cullR2) continue;
+#pragma unroll 1
     for (int x = 0; x < 3; x++) {
-      start[x] = kEmpty;
-      if (rowD2 + CellCull::pick(x - 1, cc.xl, cc.xh) <= cullR2) {
-        h[x] = gridHash(g.x + x - 1, g.y + y, g.z + z, P);
-        start[x] = __ldg((kPrefix ? cells.off : cells.start) + h[x]);
-      }
-    }
-#pragma unroll
-    for (int x = 0; x < 3; x++) {
-      if (kPrefix)  // off[h] .. off[h+1]; empty when equal
-        end[x] = start[x] != kEmpty ? min(__ldg(cells.off + h[x] + 1), n) : 0u;
-      else
-        end[x] = start[x] != kEmpty ? min(__ldg(cells.end + h[x]), n) : 0u;
-    }
-#pragma unroll
-    for (int x = 0; x < 3; x++) {
-      const unsigned b = end[x];
-      for (unsigned j = start[x] != kEmpty ? start[x] : 0u; j < b; j++) {
+      if (rowD2 + CellCull::pick(x - 1, cc.xl, cc.xh) > cullR2) continue;
+      unsigned a, b;
+      cellRange<kPrefix>(gridHash(g.x + x - 1, g.y + y, g.z + z, P), cells, n, a, b);
+      for (unsigned j = a; j < b; j++) {
         float4 q4 = ldg4(sortedPos + j);
         float3 rel = make_float3(q4.x - pos.x, q4.y - pos.y, q4.z - pos.z);
         float d2 = pairDist2(rel);
@@ -295,87 +257,279 @@ __device__ __forceinline__ float3 neighbourForceGlobal(
         }
       }
     }
-  };
-  const bool linear = kPrefix && !mortonOrder(P);
-  const unsigned gxm = P.gridSize[0] - 1u;
-  const unsigned xm = (unsigned)(g.x) & gxm;
-  // no x wrap: a row's three cells are consecutive hashes, one range
-  const bool merged = linear && xm >= 1u && xm < gxm;
-  // row `row`'s merged range [a, b), split into its cells at o1 and o2
-  // (a == b: nothing to scan)
-  auto rowRange = [&](int row, unsigned &a, unsigned &b, unsigned &o1, unsigned &o2) {
-    const int z = row / 3 - 1, y = row % 3 - 1;
-    const float rowD2 = CellCull::pick(z, cc.zl, cc.zh) + CellCull::pick(y, cc.yl, cc.yh);
-    a = b = o1 = o2 = 0u;
-    if (merged && rowD2 <= cullR2) {
-      const unsigned h0 = gridHash(g.x - 1, g.y + y, g.z + z, P);
-      const unsigned o0 = __ldg(cells.off + h0);
-      o1 = __ldg(cells.off + h0 + 1);
-      o2 = __ldg(cells.off + h0 + 2);
-      const unsigned o3 = __ldg(cells.off + h0 + 3);
-      a = rowD2 + cc.xl <= cullR2 ? o0 : o1;
-      b = min(rowD2 + cc.xh <= cullR2 ? o3 : o2, n);
+  }
+  drain();
+  force.x = force.x + cf.x;
+  force.y = force.y + cf.y;
+  force.z = force.z + cf.z;
+  return force;
+}
+
+// ---------------------------------------------------------------------------
+// The per-particle scan with hit masks.
+
+// Packed pairs of floats (one instruction for two lanes' worth of FP32).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// The near test of one particle against candidates, conservative: a pair that
+// passes `sqrtf(d2) < cd` is always near.  With e = 2^-24 and s = 1 + 16 e,
+//   c = w s + r_i s >= cd (1 + 13 e)   (three roundings off 16 e),
+//   near: the sign of dz^2 + (dx^2 + (dy^2 - c^2)), one rounding each.
+// A pair in contact has dx^2 + dy^2 + dz^2 <= cd^2 (1 + 5 e) (the roundings of
+// pairDist2 and of the root) and c^2 >= cd^2 (1 + 26 e), so the exact sum is
+// below -21 e cd^2; the roundings before the last are off by at most 3 e c^2
+// together and the last one keeps the sign.  (A NaN may carry a sign too.)
+// The contact test itself runs when the hits are drained.
+template <bool kRadiusFromW>
+struct NearTest {
+  f32x2 nxy, nzr, sel;  // (-x, -y), (-z, r_i s), (1, s)
+  float nz, nc2;        // equal radii: -z and -c^2
+  __device__ __forceinline__ NearTest(float3 p, float ri, float cdMono) {
+    constexpr float s = 1.0f + 1.0f / 1048576.0f;
+    nxy = pack2(-p.x, -p.y);
+    nzr = pack2(-p.z, __fmul_rn(ri, s));
+    sel = pack2(1.0f, s);
+    nz = -p.z;
+    const float c = __fmul_rn(cdMono, s);
+    nc2 = -__fmul_rn(c, c);
+  }
+  // negative where the candidate q is near
+  __device__ __forceinline__ float operator()(float4 q) const {
+    float dx, dy, dz, t;
+    unpack2(add2(pack2(q.x, q.y), nxy), dx, dy);
+    if (kRadiusFromW) {
+      unpack2(fma2(pack2(q.z, q.w), sel, nzr), dz, t);
+      t = -__fmul_rn(t, t);
+    } else {
+      dz = __fadd_rn(q.z, nz);
+      t = nc2;
     }
-  };
-  if (linear && stage) {
-    // The lanes of a warp are consecutive sorted particles, mostly in one
-    // grid row: their ranges of a neighbour row overlap.  The warp copies
-    // the union into shared memory with asynchronous 16-byte copies, and
-    // every lane scans its own range from there.  The copy of row r + 1 is
-    // issued before row r is scanned (two buffers of kStageLen), so it
-    // arrives while row r is scanned.  `live` is every lane of the warp that
-    // calls this function (fixed by a ballot before the call): all of them
-    // take part in each row's reductions and barriers, so a buffer is never
-    // refilled while a lane still reads it.
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned rank = __popc(live & ((1u << lane) - 1u)), lanes = __popc(live);
-    auto issue = [&](unsigned a, unsigned b, float4 *buf, unsigned &lo) {
-      lo = __reduce_min_sync(live, a < b ? a : 0xffffffffu);
-      const unsigned hi = __reduce_max_sync(live, a < b ? b : 0u);
-      const bool staged = lo < hi && hi - lo <= (unsigned)kStageLen;
-      if (staged)
-        for (unsigned t = rank; t < hi - lo; t += lanes) copyAsync16(buf + t, sortedPos + lo + t);
-      copyAsyncCommit();
-      return staged;  // false: the row is read from global memory
-    };
-    unsigned a0, b0, s10, s20, lo0;
-    rowRange(0, a0, b0, s10, s20);
-    bool st0 = issue(a0, b0, stage, lo0);
-#pragma unroll 1
-    for (int row = 0; row < 9; row++) {
-      unsigned a1 = 0, b1 = 0, s11 = 0, s21 = 0, lo1 = 0;
-      bool st1 = false;
-      if (row < 8) {
-        rowRange(row + 1, a1, b1, s11, s21);
-        st1 = issue(a1, b1, stage + ((row + 1) & 1) * kStageLen, lo1);
-        copyAsyncWait<1>();  // this lane's copies of row `row` have landed
+    return fmaf(dz, dz, fmaf(dx, dx, fmaf(dy, dy, t)));
+  }
+};
+
+// The candidates of a particle in one neighbour row (z, y offsets row / 3 - 1,
+// row % 3 - 1), numbered t = 0, 1, ... in the reference's order: those below
+// k1 are in the cell at x offset -1, those from k2 on in the cell at +1.
+// seg.x is the sorted slot of candidate 0 and seg.y = len | k1 << 8 |
+// k2 << 16.  In the grid's first and last column the row's wrapped cell is
+// apart from the other two: then candidate t from the break on (k1 in the
+// first column, k2 in the last) is slot edgeSlot + t instead of seg.x + t.
+constexpr unsigned kSegMax = 255;  // longest row the mask scan takes
+constexpr unsigned kScan = 4;      // candidates loaded and tested together (3 and 6 are slower)
+
+// The nine rows of a particle with grid coordinates g into
+// seg[row * kQueueStride] and edgeSlot[row].  total receives the particles of
+// the 27 cells.  The table loads of all rows are independent.  Returns -1 in
+// the grid's first column, 1 in its last, 0 between, or 2 (seg undefined)
+// when the row structure does not hold: Morton order, an axis with fewer
+// than three cells (rows or cells come up twice there, and with them the
+// particle itself), a row too long for the mask scan, fewer than kScan
+// particles, or cell tables that do not list a row's cells one after the
+// other.
+template <bool kPrefix>
+__device__ __forceinline__ int rowSegments(int3 g, const CellRanges &cells, unsigned n,
+                                           const SimParams &P, const CellCull &cc, float cullR2,
+                                           uint2 *seg, unsigned *edgeSlot, unsigned &total) {
+  const unsigned gx = P.gridSize[0];
+  if (mortonOrder(P) || gx < 3u || P.gridSize[1] < 3u || P.gridSize[2] < 3u || n < kScan)
+    return 2;
+  const unsigned xm = (unsigned)g.x & (gx - 1u);
+  const bool edgeLow = xm == 0u, edgeHigh = xm == gx - 1u;
+  bool ok = true;
+  unsigned yBase[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    yBase[k] = __umul24((unsigned)(g.y + k - 1) & (P.gridSize[1] - 1u), gx);
+  total = 0u;
+#pragma unroll
+  for (int zi = 0; zi < 3; ++zi) {
+    const unsigned zBase = __umul24(
+        __umul24((unsigned)(g.z + zi - 1) & (P.gridSize[2] - 1u), P.gridSize[1]), gx);
+#pragma unroll
+    for (int yi = 0; yi < 3; ++yi) {
+      const int row = zi * 3 + yi;
+      const unsigned h = zBase + yBase[yi] + xm;
+      const float rowD2 = CellCull::pick(zi - 1, cc.zl, cc.zh) + CellCull::pick(yi - 1, cc.yl, cc.yh);
+      const bool low = rowD2 + cc.xl <= cullR2, high = rowD2 + cc.xh <= cullR2;
+      const bool mid = rowD2 <= cullR2;
+      // the cells that are not beyond the wrap: [o0, o1), [o1, o2), [o2, o3)
+      unsigned o0, o1, o2, o3;
+      if (kPrefix) {
+        o1 = __ldg(cells.off + h);
+        o2 = __ldg(cells.off + h + 1);
+        o0 = edgeLow ? o1 : __ldg(cells.off + h - 1);
+        o3 = edgeHigh ? o2 : __ldg(cells.off + h + 2);
       } else {
-        copyAsyncWait<0>();
+        const unsigned s0 = edgeLow ? kEmpty : __ldg(cells.start + h - 1);
+        const unsigned s1 = __ldg(cells.start + h);
+        const unsigned s2 = edgeHigh ? kEmpty : __ldg(cells.start + h + 1);
+        const unsigned e0 = edgeLow ? 0u : __ldg(cells.end + h - 1), e1 = __ldg(cells.end + h);
+        const unsigned e2 = edgeHigh ? 0u : __ldg(cells.end + h + 1);
+        // an empty cell begins and ends where the one before it ends
+        o0 = s0 != kEmpty ? s0 : (s1 != kEmpty ? s1 : (s2 != kEmpty ? s2 : 0u));
+        o1 = s0 != kEmpty ? e0 : o0;
+        o2 = s1 != kEmpty ? e1 : o1;
+        o3 = s2 != kEmpty ? e2 : o2;
+        ok = ok && (s1 == kEmpty || s1 == o1) && (s2 == kEmpty || s2 == o2);
       }
-      __syncwarp(live);  // and every other lane's
-      const float4 *buf = stage + (row & 1) * kStageLen;
-      if (st0)
-        scanRange(a0, b0, row * 3, s10, s20, [&](unsigned j) { return buf[j - lo0]; });
-      else if (merged)
-        scanRange(a0, b0, row * 3, s10, s20, loadGlobal);
-      if (!merged) cellRow(row);
-      __syncwarp(live);  // buffer row & 1 is refilled for row + 2
-      a0 = a1;
-      b0 = b1;
-      s10 = s11;
-      s20 = s21;
-      lo0 = lo1;
-      st0 = st1;
+      ok = ok && o0 <= o1 && o1 <= o2 && o2 <= o3 && o3 <= n;
+      total += o3 - o0;
+      unsigned a = low ? o0 : o1, b = high ? o3 : o2;
+      unsigned k1 = o1 - a, k2 = o2 - a, len = b - a;
+      if (edgeLow || edgeHigh) {
+        unsigned sa, sb;  // the cell beyond the wrap
+        cellRange<kPrefix>(edgeLow ? h + gx - 1u : h + 1u - gx, cells, n, sa, sb);
+        total += sb - sa;
+        const unsigned extra = (edgeLow ? low : high) ? sb - sa : 0u;
+        edgeSlot[row] = edgeLow ? a - extra : sa - len;
+        if (edgeLow) {
+          a = sa;
+          k1 += extra;
+          k2 += extra;
+        }
+        len += extra;
+      }
+      if (!mid) len = 0u;
+      ok = ok && len <= kSegMax;
+      seg[row * kQueueStride] = make_uint2(a, len ? len | (k1 << 8) | (k2 << 16) : 0u);
     }
-  } else {
+  }
+  return ok ? (edgeLow ? -1 : (edgeHigh ? 1 : 0)) : 2;
+}
+
+// The pair forces from the rows in seg.  Candidates are tested 32 at a time
+// into a bit mask -- no branch and no store per hit -- and masks with hits
+// are queued; the drain takes the hits in order (rows, then slots), where
+// the exact test and the contact term run.  Sums as in neighbourForceGlobal.
+// kEdge: the particle may be in the grid's first or last column (edge).
+template <bool kRadiusFromW, bool kEdge>
+__device__ __forceinline__ float3 neighbourForceMask(
+    unsigned i, unsigned n, float3 pos, float3 vel, float ri,
+    const float4 *__restrict__ sortedPos, const float4 *__restrict__ sortedVel,
+    const SimParams &P, const uint2 *seg, const unsigned *edgeSlot, int edge, unsigned *qm, unsigned char *qd) {
+  const float cdMono = ri + P.particleRadius;
+  const NearTest<kRadiusFromW> near(pos, ri, cdMono);
+  float3 force = make_float3(0.0f, 0.0f, 0.0f);
+  float3 cf = make_float3(0.0f, 0.0f, 0.0f);
+  int cfCell = -1;
+  int qn = 0;
+  // where the row's second part begins, and the slot of its candidate "0"
+  auto breakOf = [&](uint2 s) { return edge < 0 ? (s.y >> 8) & 255u : (s.y >> 16) & 255u; };
+  auto drain = [&]() {
+    int e = 0;
+    unsigned mask = 0u, t0 = 0u, row = 0u, cut = 0u, slot2 = 0u;
+    uint2 s = make_uint2(0u, 0u);
+    while (true) {
+      if (mask == 0u) {
+        if (e == qn) break;
+        mask = qm[e * kQueueStride];
+        const unsigned d = qd[e * kQueueStride];
+        ++e;
+        row = d & 15u;
+        t0 = (d >> 4) * 32u;
+        s = seg[row * kQueueStride];
+        if (kEdge) {
+          cut = breakOf(s);
+          slot2 = edge ? edgeSlot[row] : s.x;
+        }
+      }
+      const unsigned t = t0 + (unsigned)(__ffs((int)mask) - 1);
+      mask &= mask - 1u;
+      const unsigned j = t + (kEdge && t >= cut ? slot2 : s.x);
+      const float4 q4 = ldg4(sortedPos + j);
+      const float4 w4 = ldg4(sortedVel + j);
+      const float3 rel = make_float3(q4.x - pos.x, q4.y - pos.y, q4.z - pos.z);
+      const float dist = sqrtf(pairDist2(rel));
+      const float cd = kRadiusFromW ? ri + q4.w : cdMono;
+      if (dist < cd) {
+        const int cell = (int)(row * 3u) + (t >= ((s.y >> 8) & 255u)) + (t >= ((s.y >> 16) & 255u));
+        if (cell != cfCell) {
+          force.x = force.x + cf.x;
+          force.y = force.y + cf.y;
+          force.z = force.z + cf.z;
+          cf = make_float3(0.0f, 0.0f, 0.0f);
+          cfCell = cell;
+        }
+        const float3 f = contactTerm(rel, dist, cd, vel, make_float3(w4.x, w4.y, w4.z),
+                                     P.attraction, P);
+        cf.x = cf.x + f.x;
+        cf.y = cf.y + f.y;
+        cf.z = cf.z + f.z;
+      }
+    }
+    qn = 0;
+  };
 #pragma unroll 1
-    for (int row = 0; row < 9; row++) {
-      if (merged) {
-        unsigned a, b, o1, o2;
-        rowRange(row, a, b, o1, o2);
-        scanRange(a, b, row * 3, o1, o2, loadGlobal);
-      } else {
-        cellRow(row);
+  for (int row = 0; row < 9; ++row) {
+    const uint2 s = seg[row * kQueueStride];
+    const unsigned len = s.y & 255u;
+    unsigned cut = 0u, slot2 = 0u;
+    if (kEdge) {
+      cut = breakOf(s);
+      slot2 = edge ? edgeSlot[row] : s.x;
+    }
+#pragma unroll 1
+    for (unsigned c0 = 0; c0 < len; c0 += 32u) {
+      const unsigned cnt = min(32u, len - c0);
+      unsigned mask = 0u;
+#pragma unroll 1
+      for (unsigned t = 0; t < cnt; t += kScan) {
+        unsigned m = 0u, back = 0u;
+        float4 c[kScan];
+        if (kEdge) {
+#pragma unroll
+          for (unsigned u = 0; u < kScan; ++u) {
+            const unsigned v = c0 + (u ? min(t + u, cnt - 1u) : t);
+            c[u] = ldg4(sortedPos + (v + (v >= cut ? slot2 : s.x)));
+          }
+        } else {
+          // kScan slots on, or the array's last kScan where it ends first
+          const unsigned j = s.x + c0 + t, j0 = min(j, n - kScan);
+          back = j - j0;
+          const float4 *q = sortedPos + j0;
+#pragma unroll
+          for (unsigned u = 0; u < kScan; ++u) c[u] = ldg4(q + u);
+        }
+        // the sign bits, the last candidate's first
+#pragma unroll
+        for (int u = kScan - 1; u >= 0; --u)
+          m = __funnelshift_l(__float_as_uint(near(c[u])), m, 1);
+        mask |= (m >> back) << t;
+      }
+      mask &= 0xffffffffu >> (32u - cnt);  // candidates past the row's end
+      if (row == 4) {  // the particle itself
+        const unsigned self = i - c0 - (kEdge && edge < 0 ? slot2 : s.x);
+        if (self < 32u) mask &= ~(1u << self);
+      }
+      if (mask) {
+        if (qn == kQueueLen) drain();
+        qm[qn * kQueueStride] = mask;
+        qd[qn * kQueueStride] = (unsigned char)((unsigned)row | (c0 >> 1));
+        ++qn;
       }
     }
   }
@@ -384,6 +538,20 @@ __device__ __forceinline__ float3 neighbourForceGlobal(
   force.y = force.y + cf.y;
   force.z = force.z + cf.z;
   return force;
+}
+
+// neighbourForceMask for the lanes of a warp that run together: the version
+// for the grid's edge columns only where one of them is in such a column.
+template <bool kRadiusFromW>
+__device__ __forceinline__ float3 maskForce(
+    unsigned i, unsigned n, float3 pos, float3 vel, float ri,
+    const float4 *__restrict__ sortedPos, const float4 *__restrict__ sortedVel,
+    const SimParams &P, const uint2 *seg, const unsigned *edgeSlot, int edge, unsigned *qm, unsigned char *qd) {
+  if (__any_sync(__activemask(), edge != 0))
+    return neighbourForceMask<kRadiusFromW, true>(i, n, pos, vel, ri, sortedPos, sortedVel, P, seg,
+                                                  edgeSlot, edge, qm, qd);
+  return neighbourForceMask<kRadiusFromW, false>(i, n, pos, vel, ri, sortedPos, sortedVel, P, seg,
+                                                 edgeSlot, 0, qm, qd);
 }
 
 // ---------------------------------------------------------------------------
@@ -408,44 +576,12 @@ struct CrowdList {
   unsigned limit;   // neighbourhood size above which a particle is deferred
 };
 
-// Range [a, b) of cell h (empty: a == b).
-template <bool kPrefix>
-__device__ __forceinline__ void cellRange(unsigned h, const CellRanges &cells, unsigned n,
-                                          unsigned &a, unsigned &b) {
-  if (kPrefix) {
-    a = __ldg(cells.off + h);
-    b = min(__ldg(cells.off + h + 1), n);
-  } else {
-    a = __ldg(cells.start + h);
-    if (a == kEmpty) {
-      a = 0u;
-      b = 0u;
-    } else {
-      b = min(__ldg(cells.end + h), n);
-    }
-  }
-  if (b < a) b = a;
-}
-
-// Particles in the 27 neighbour cells of grid position g.  The nine rows
-// are independent (no early exit), so their table loads overlap.
+// Particles in the 27 neighbour cells of grid position g, where rowSegments
+// has not counted them.
 template <bool kPrefix>
 __device__ __forceinline__ unsigned neighbourhoodCount(int3 g, const CellRanges &cells,
                                                        unsigned n, const SimParams &P) {
   unsigned total = 0;
-  const unsigned gxm = P.gridSize[0] - 1u;
-  const unsigned xm = (unsigned)(g.x) & gxm;
-  if (kPrefix && xm >= 1u && xm < gxm && !mortonOrder(P)) {
-    // no x wrap: each row's three cells are consecutive hashes
-#pragma unroll
-    for (int row = 0; row < 9; row++) {
-      const int z = row / 3 - 1, y = row % 3 - 1;
-      const unsigned h0 = gridHash(g.x - 1, g.y + y, g.z + z, P);
-      const unsigned o0 = __ldg(cells.off + h0), o3 = __ldg(cells.off + h0 + 3);
-      total += o3 > o0 ? o3 - o0 : 0u;
-    }
-    return total;
-  }
 #pragma unroll 1
   for (int row = 0; row < 9; row++) {
     const int z = row / 3 - 1, y = row % 3 - 1;
@@ -459,50 +595,73 @@ __device__ __forceinline__ unsigned neighbourhoodCount(int3 g, const CellRanges 
   return total;
 }
 
+// One thread per sorted particle.  Bound by instruction issue and the ALU
+// pipe, then by L1 latency (4.2M spheres at 30% volume fraction, an earlier
+// form of this scan: 67% issue active, ALU 56%, L1 data 55%, DRAM 6%, 17 of
+// 32 lanes).  So the scan spends 8 instructions on a candidate -- one 16-byte
+// load, packed differences, three multiply-adds, one shift that collects the
+// sign -- with no branch and no store per hit, and all table loads go out
+// before it.  Measured against the kernel it replaced (rows copied to shared
+// memory one after the other, a branch and two stores per near partner), per
+// collide: 4.2M spheres 507 against 748 us, 1M in piles 250 against 395, 1M
+// falling monodisperse 72 against 121.  All lanes scan the same row at a time:
+// skipping a lane's empty rows costs L1 hits (+13%).  64 registers (8 CTAs
+// per SM) against 72: -3%.  Shared memory is kept small because L1 gets the
+// rest of the 256 KB (31 KB per CTA instead of 17: +6%).
 template <int kMode, bool kRadiusFromW, bool kCollider, bool kForceOut, bool kPrefix>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 8)
 kCollideGlobal(float4 *__restrict__ newVel, const float4 *__restrict__ sortedPos,
                const float4 *__restrict__ sortedVel, const unsigned *__restrict__ index,
                CellRanges cells, unsigned n, KParams kp, CollideOut out, bool cull,
-               CrowdList crowd, unsigned *status, bool stageRows) {
+               CrowdList crowd, unsigned *status) {
   __shared__ unsigned qj[kQueueLen * kQueueStride];
   __shared__ unsigned char qc[kQueueLen * kQueueStride];
-  __shared__ float4 sStage[4][2 * kStageLen];  // two row buffers per warp
+  __shared__ uint2 sSeg[9 * kQueueStride];
   const SimParams &P = kp.p;
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  // every lane of the warp reaches the ballot below (the block is whole
-  // warps); lanes past n load nothing
-  const bool active = i < n;
-  const float4 p4 = active ? ldg4(sortedPos + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  const float4 v4 = active ? ldg4(sortedVel + i) : p4;
+  if (i >= n) return;
+  const float4 p4 = ldg4(sortedPos + i);
+  const float4 v4 = ldg4(sortedVel + i);
   const float3 pos = make_float3(p4.x, p4.y, p4.z), vel = make_float3(v4.x, v4.y, v4.z);
   const float ri = kRadiusFromW ? p4.w : P.particleRadius;
   const int3 g = gridPos(pos.x, pos.y, pos.z, P);
-  bool deferred = false;
-  if (active && crowd.groups && neighbourhoodCount<kPrefix>(g, cells, n, P) > crowd.limit) {
-    unsigned a, b;
-    cellRange<kPrefix>(gridHash(g.x, g.y, g.z, P), cells, n, a, b);
-    if (i >= a && i < b) {  // deferred to kCollideCrowd
-      if (((i - a) & 31u) == 0u) {
-        const unsigned k = atomicAdd(crowd.count, 1u);
-        if (k < crowd.cap) crowd.groups[k] = make_uint2(i, min(32u, b - i));
-      }
-      deferred = true;
-    }
-  }
-  if (active && !deferred && kRadiusFromW && !(ri <= P.particleRadius)) {
+  if (kRadiusFromW && !(ri <= P.particleRadius)) {
     atomicOr(status, (unsigned)kStatusRadiusBound);  // the culling bound is broken
     cull = false;
   }
+  uint2 *mySeg = sSeg + threadIdx.x;
+  unsigned edgeSlot[9];
+  // largest contact distance: r_i + particleRadius (in the radius-from-w
+  // mode particleRadius bounds every radius)
+  const CellCull cc = makeCull(pos, g, ri + P.particleRadius, P);
+  const float cullR2 = cull ? cc.r2 : __int_as_float(0x7f800000);  // +inf: no culling
+  unsigned total = 0u;
+  const int edge = rowSegments<kPrefix>(g, cells, n, P, cc, cullR2, mySeg, edgeSlot, total);
+  if (crowd.groups) {
+    if (edge == 2) total = neighbourhoodCount<kPrefix>(g, cells, n, P);
+    if (total > crowd.limit) {
+      unsigned a, b;
+      cellRange<kPrefix>(gridHash(g.x, g.y, g.z, P), cells, n, a, b);
+      if (i >= a && i < b) {  // deferred to kCollideCrowd
+        if (((i - a) & 31u) == 0u) {
+          const unsigned k = atomicAdd(crowd.count, 1u);
+          if (k < crowd.cap) crowd.groups[k] = make_uint2(i, min(32u, b - i));
+        }
+        return;
+      }
+    }
+  }
   // an inert particle's force is +0.0 (inertPos): it scans nothing
-  const bool scan = active && !deferred && !inertPos(pos);
-  const unsigned live = __ballot_sync(0xffffffffu, scan);
-  if (!active || deferred) return;
   float3 force = make_float3(0.0f, 0.0f, 0.0f);
-  if (scan)
-    force = neighbourForceGlobal<kRadiusFromW, kPrefix>(
-        i, n, pos, vel, ri, g, cull, sortedPos, sortedVel, cells, P, qj + threadIdx.x,
-        qc + threadIdx.x, kPrefix && stageRows ? sStage[threadIdx.x >> 5] : nullptr, live);
+  if (!inertPos(pos)) {
+    if (edge != 2)
+      force = maskForce<kRadiusFromW>(i, n, pos, vel, ri, sortedPos, sortedVel, P, mySeg,
+                                      edgeSlot, edge, qj + threadIdx.x, qc + threadIdx.x);
+    else
+      force = neighbourForceGlobal<kRadiusFromW, kPrefix>(i, n, pos, vel, ri, g, cull, sortedPos,
+                                                          sortedVel, cells, P, qj + threadIdx.x,
+                                                          qc + threadIdx.x);
+  }
   finishParticle<kMode, kCollider, kForceOut>(i, n, pos, vel, p4, ri, force, index, newVel,
                                               out, P);
 }
@@ -854,11 +1013,12 @@ bool g_crowdPath = true;  // fcdemSetCrowdPath
 unsigned g_crowdLimit = kCrowdLimit;  // fcdemSetCrowdLimit
 constexpr unsigned kCrowdCtasPerSmDefault = 4;
 unsigned g_crowdCtasPerSm = kCrowdCtasPerSmDefault;  // persistent grid: CTAs per SM
-bool g_stageRows = true;  // kCollideGlobal copies short row unions to shared memory
 
 // The collide configurations fcdemAutotuneCollide chooses from: crowd
 // limit x crowded-kernel CTAs per SM x row staging.  Results are identical
 // for every one; configuration kDefaultCollideConfig is the built-in one.
+// kCollideGlobal reads its rows through L1 whatever stageRows says (see
+// there), so the tuner times the configurations with it set only.
 struct CollideConfig {
   unsigned crowdLimit, ctasPerSm;
   bool stageRows;
@@ -874,7 +1034,6 @@ void applyCollideConfig(int k) {
   const CollideConfig c = collideConfig(k);
   g_crowdLimit = c.crowdLimit;
   g_crowdCtasPerSm = c.ctasPerSm;
-  g_stageRows = c.stageRows;
 }
 
 // The group list for n particles (grown on demand; at most one group per
@@ -916,7 +1075,7 @@ void launchT(bool tiled, bool cull, unsigned n, float4 *newVel, const float4 *sp
     const CrowdList crowd = crowdList(n);
     kCollideGlobal<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix>
         <<<blocks, 128, 0, curStream()>>>(newVel, sp, sv, index, cells, n, kp, out, cull,
-                                          crowd, ctx().dStatus, g_stageRows);
+                                          crowd, ctx().dStatus);
     if (crowd.groups && launchOk())
       kCollideCrowd<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix>
           <<<numSms() * g_crowdCtasPerSm, kCrowdWarps * 32, 0, curStream()>>>(
@@ -935,6 +1094,7 @@ kCollideBatch(const BatchScene *__restrict__ scenes, const unsigned *__restrict_
               const unsigned *__restrict__ off, unsigned n, CollideOut out, unsigned *status) {
   __shared__ unsigned qj[kQueueLen * kQueueStride];
   __shared__ unsigned char qc[kQueueLen * kQueueStride];
+  __shared__ uint2 sSeg[9 * kQueueStride];
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const BatchScene &S = scenes[__ldg(sceneOf + i)];
@@ -951,11 +1111,22 @@ kCollideBatch(const BatchScene *__restrict__ scenes, const unsigned *__restrict_
   }
   CellRanges cells;
   cells.off = off + S.cellBase;
+  uint2 *mySeg = sSeg + threadIdx.x;
+  unsigned edgeSlot[9];
+  const CellCull cc = makeCull(pos, g, ri + P.particleRadius, P);
+  const float cullR2 = cull ? cc.r2 : __int_as_float(0x7f800000);  // +inf: no culling
   float3 force = make_float3(0.0f, 0.0f, 0.0f);
-  if (!inertPos(pos))
-    force = neighbourForceGlobal<kRadiusFromW, true>(i, n, pos, vel, ri, g, cull, sortedPos,
-                                                     sortedVel, cells, P, qj + threadIdx.x,
-                                                     qc + threadIdx.x);
+  if (!inertPos(pos)) {
+    unsigned total = 0u;
+    const int edge = rowSegments<true>(g, cells, n, P, cc, cullR2, mySeg, edgeSlot, total);
+    if (edge != 2)
+      force = maskForce<kRadiusFromW>(i, n, pos, vel, ri, sortedPos, sortedVel, P, mySeg,
+                                      edgeSlot, edge, qj + threadIdx.x, qc + threadIdx.x);
+    else
+      force = neighbourForceGlobal<kRadiusFromW, true>(i, n, pos, vel, ri, g, cull, sortedPos,
+                                                       sortedVel, cells, P, qj + threadIdx.x,
+                                                       qc + threadIdx.x);
+  }
   // collider sphere (particles_kernel.cu:288)
   {
     float3 rel = make_float3(P.colliderPos[0] - pos.x, P.colliderPos[1] - pos.y,
@@ -1142,6 +1313,7 @@ extern "C" int fcdemAutotuneCollide(float *pos, float *vel, float *sortedPos, fl
   float bestT = 3.4e38f, defaultT = 3.4e38f;
   bool ok = true;
   for (int k = 0; k < kNumCollideConfigs && ok; ++k) {
+    if (!collideConfig(k).stageRows) continue;
     applyCollideConfig(k);
     float tot = 0.0f;
     for (int rep = 0; rep < 3 && ok; ++rep) {

@@ -246,8 +246,10 @@ int fcdemSetSortConfig(unsigned numParticles, int config);
 
 /* Collide tuning.  A collide configuration is a crowd limit (256, 384, 512,
  * 768 or 1024 neighbourhood members; fcdemSetCrowdLimit), the CTAs per SM of
- * the crowded-neighbourhood kernel's persistent grid (2, 4 or 8) and whether
- * the per-particle kernel copies short neighbour rows to shared memory;
+ * the crowded-neighbourhood kernel's persistent grid (2, 4 or 8) and
+ * stageRows, which stays part of the numbering but changes nothing: the
+ * per-particle kernel reads neighbour rows through L1, and the tuner times
+ * only the configurations that have it set;
  * results are identical for every one.  fcdemAutotuneCollide times one
  * fcdemUpdate step from the caller's state (the arguments of fcdemUpdate)
  * under each configuration, keeps the fastest -- the default unless another

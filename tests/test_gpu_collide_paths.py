@@ -262,3 +262,51 @@ def test_collide_autotuner_keeps_the_state_and_the_results():
     dem.check("update, default configuration")
     for x, y in zip(tuned, (ds2.pos.cpu().numpy(), ds2.vel.cpu().numpy())):
         np.testing.assert_array_equal(x.view(np.uint32), y.view(np.uint32))
+
+
+def _rows_scene(grid, n, poly, kind, seed):
+    """Scenes at the edges of the row scan: `rows` puts n particles into one
+    column of cells (rows of n candidates), `full` spreads them over the whole
+    grid and past it, so that the first and last columns wrap."""
+    from fullc0ntact_gb300 import scenes
+    radius = 1.0 / 64.0
+    sc = scenes.random_box(n, grid=grid, radius=radius, seed=seed, cell=1.0 / 32.0, poly=poly)
+    rng = np.random.default_rng(seed + 1)
+    if kind == "rows":
+        sc["pos"][:, 0] = rng.uniform(-0.5, -0.5 + 3.0 / 32.0, n)
+        sc["pos"][:, 1:3] = rng.uniform(-0.5, -0.5 + 1.0 / 32.0, (n, 2))
+    else:
+        ext = np.array(grid) / 32.0
+        sc["pos"][:, :3] = np.clip(-1.0 + rng.uniform(-0.02, 1.02, (n, 3)) * ext, -0.98, 0.98)
+    return sc
+
+
+@pytest.mark.parametrize("poly", [False, True])
+@pytest.mark.parametrize("grid,n,kind", [
+    ((64, 64, 64), 1, "rows"), ((64, 64, 64), 3, "rows"), ((64, 64, 64), 4, "rows"),
+    ((64, 64, 64), 5, "rows"), ((64, 64, 64), 31, "rows"), ((64, 64, 64), 33, "rows"),
+    ((64, 64, 64), 129, "rows"), ((64, 64, 64), 255, "rows"), ((64, 64, 64), 256, "rows"),
+    ((64, 64, 64), 700, "rows"), ((4, 4, 4), 300, "full"), ((4, 8, 16), 700, "full"),
+    ((8, 2, 4), 200, "full"), ((2, 8, 8), 300, "full"), ((16, 16, 16), 4001, "full")])
+def test_row_scan_edges_match_oracle(grid, n, kind, poly):
+    """The hit-mask scan and the general loop on rows of 0 to 700 candidates,
+    wrapped columns and aliased axes: bit-exact against the oracle, staged
+    (cellStart/cellEnd) and fused (prefix table)."""
+    from fullc0ntact_gb300 import dem
+    from oracle import oracle as O
+    sc = _rows_scene(grid, n, poly, kind, 100 + n)
+    P = O.SimParams.from_buffer_copy(bytes(sc["params"]))
+    with O.gpu_arithmetic():
+        pos, vel = sc["pos"].copy(), sc["vel"].copy()
+        O.update(P, pos, vel, sc["dt"], 1, poly)  # in place
+    for crowd in (1, 0):
+        dem.lib.fcdemSetCrowdPath(crowd)
+        try:
+            for fused in (False, True):
+                ds = dem.DeviceScene(sc)
+                ds.update(1) if fused else ds.stages()
+                dem.check("row scan")
+                for a, b in ((ds.pos, pos), (ds.vel, vel)):
+                    np.testing.assert_array_equal(a.cpu().numpy(), b)
+        finally:
+            dem.lib.fcdemSetCrowdPath(1)
