@@ -41,3 +41,35 @@ def test_torus_mesh_map_matches_exact_torus():
     assert np.abs(vm[:, 0] - vt[:, 0]).max() <= facet + 1e-5
     far = np.abs(vt[:, 0]) > 2 * facet
     assert np.all(np.sign(vm[far, 0]) == np.sign(vt[far, 0]))
+
+
+@pytest.mark.parametrize("form", ["closed", "shuffled", "unwelded", "open"])
+@pytest.mark.parametrize("nu,nv,cells", [(3, 5, 9), (4, 4, 13), (3, 11, 16), (32, 17, 21)])
+def test_mesh_map_forms_match_fp64_oracle(nu, nv, cells, form):
+    """Cluster remainders (30, 32, 66 and 1,088 triangles), lattices that are no
+    multiple of a brick, triangle order, vertices given once per triangle, and
+    a mesh with a boundary: distance, closest point and winding-number sign."""
+    from fullc0ntact_gb300 import dem, scenes
+    from oracle import mesh_oracle as mo
+    from oracle import oracle as O
+    verts, tris = scenes.torus_mesh(0.3, 0.1, nu, nv)
+    rng = np.random.default_rng(nu * 100 + nv)
+    if form == "open":
+        tris = tris[: len(tris) * 2 // 3]
+    elif form != "closed":
+        tris = rng.permutation(tris)
+    if form == "unwelded":
+        verts, tris = verts[tris.reshape(-1)], np.arange(tris.size, dtype=np.uint32).reshape(-1, 3)
+    m = dem.DistanceMap.from_mesh(verts, tris, cells, 0.05)
+    v = m.vertices()
+    coords = O.lattice_coords(m.vmin, m.cell_size, m.cells).astype(np.float64)
+    d, _ = mo.mesh_distance(coords, verts, tris)
+    assert np.abs(np.abs(v[:, 0]) - np.abs(d)).max() <= 2e-6
+    V = verts.astype(np.float64)
+    wind = mo.winding_number(coords, V[tris[:, 0]], V[tris[:, 1]], V[tris[:, 2]])
+    sure = (np.abs(d) > 1e-5) & (np.abs(wind - 0.5) > 1e-3)
+    assert np.all((v[sure, 0] < 0) == (wind[sure] > 0.5))
+    gcp = v[:, 1:].astype(np.float64)
+    assert np.abs(np.linalg.norm(coords - gcp, axis=1) - np.abs(d)).max() <= 2e-6
+    on, _ = mo.mesh_distance(gcp, verts, tris)
+    assert np.abs(on).max() <= 2e-6
