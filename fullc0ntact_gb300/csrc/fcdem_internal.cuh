@@ -85,6 +85,39 @@ bool cudaOk(cudaError_t e);
 // Checks (and counts) the launch that was just issued.
 bool launchOk();
 
+// Chained launches.  launchChained(true, ...) issues a kernel that may start
+// while the kernel before it on the stream is still running (programmatic
+// stream serialisation), so that its launch latency and its prologue overlap
+// with that kernel's tail.  Every kernel launched this way first calls
+// chainTrigger() (the next one may start), then chainWait(), which returns
+// when the kernels before it are complete and their writes visible, and only
+// then reads or writes what others touch: a kernel's completion thus still
+// implies that of all before it.  Before chainWait() it may read what was
+// complete before the last launch that was not chained.  The first launch of
+// a call is not chained (its inputs come from the caller's work); launched
+// that way the two calls do nothing.
+__device__ __forceinline__ void chainTrigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void chainWait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... Params, class... Args>
+inline void launchChained(bool chained, void (*kernel)(Params...), unsigned blocks, unsigned threads,
+                          size_t smem, Args &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(blocks);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = curStream();
+  cudaLaunchAttribute attr = {};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);  // launchOk() reads the error
+}
+
 // Stage profiling of fcdemUpdate (fcdemSetProfiling): brackets a stage with a
 // CUDA event pair when profiling is on.
 void stageBegin(int stage);

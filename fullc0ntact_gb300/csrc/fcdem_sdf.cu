@@ -9,12 +9,10 @@
 // vector: W0 [H][D], b0 [H], then per further hidden layer W [H][H], b [H],
 // then wOut [H], bOut.  Weight matrices are row-major [out][in].
 //
-//  * training (FP32): kSdfTrain runs forward and backward for a tile of S
-//    samples per CTA with every activation in shared memory; the products are
-//    4x4 register tiles over shared-memory operands; the tile's weight and
-//    bias gradients are added to the batch gradient with atomics; kSdfAdam
-//    applies Adam and refreshes the transposed weight copies the forward
-//    reads;
+//  * training (FP32): kSdfTrain runs forward and backward for tiles of 16
+//    samples per CTA with the weights and every activation in shared memory
+//    and the weight gradients in registers; kSdfReduce adds the CTAs' sums and
+//    applies Adam;
 //  * inference (BF16 weights and activations, FP32 accumulate): kSdfInfer
 //    and the culled integrate give each CTA 128 points.  The first layer
 //    (3 or 11 inputs) and the output layer run on the CUDA cores; each H x H
@@ -24,6 +22,7 @@
 //    layer's operand tile.
 #include <cuda_bf16.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -72,7 +71,6 @@ SdfLayout makeLayout(int D, int H, int L) {
 struct SdfView {
   SdfLayout lay;
   const float *__restrict__ p;   // parameters
-  const float *__restrict__ pT;  // same, weight matrices transposed ([in][out])
   const __nv_bfloat16 *__restrict__ w16;  // hidden layers 1..L-1, tensor-core tiles
   float shift[3], scale[3], outScale;
 };
@@ -135,218 +133,300 @@ kSdfSamples(MapView M, float4 *__restrict__ out, int *__restrict__ shapeOut, int
 }
 
 // ---------------------------------------------------------------------------
-// Training: forward (+ backward) of S = 4096 / H samples per CTA.
+// Training: forward (+ backward) of kTrainS samples per CTA at a time.
+//
+// A mini-batch of the obstacle networks is a few thousand samples, 0.1 GFLOP:
+// what bounds it is how many SMs it reaches and the latency of its chain of
+// layers, so a tile is small (16 samples; a batch of 2,048 is 128 CTAs) and 4 H
+// threads share it, four outputs of one sample each.  The hidden layers'
+// weights sit in shared memory row-major [out][in], rows padded by four floats:
+// the forward product reads rows j, j + H/4, ... (lanes on consecutive rows)
+// and the backward one the columns of a row (lanes on consecutive 16-byte
+// words), both without bank conflicts.  Each thread keeps its 4 x 4 blocks of
+// the weight gradients in registers over the CTA's tiles; the CTA's sums go to
+// its row of `partial`, and kSdfReduce adds the rows in order (no atomics: the
+// same bits every time; the loss alone is summed sample by sample).  3 -> 64 ->
+// 64 -> 64 -> 1, batches of 2,048 samples: 17 us a batch against 67 us with
+// tiles of 64 samples (32 CTAs), weights read from L2 and a gradient added with
+// 277,000 atomics.
+constexpr int kTrainS = 16;
 
-// out[s][j] = bias[j] + sum_k in[s][k] * Wt[k][j] for the S x H tile; thread
-// t owns rows 4*(t / (H/4)) .. +3 and columns 4*(t % (H/4)) .. +3.
-template <int H>
-__device__ __forceinline__ void gemmTile(const float *in, int inStride, int K,
-                                         const float *__restrict__ Wt,
-                                         const float *__restrict__ bias, float *out) {
-  const int t = threadIdx.x;
-  const int j0 = (t % (H / 4)) * 4, s0 = (t / (H / 4)) * 4;
-  float acc[4][4];
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    const float b = bias ? __ldg(bias + j0 + v) : 0.0f;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) acc[u][v] = b;
-  }
-  for (int k = 0; k < K; ++k) {
-    const float4 w = __ldg(reinterpret_cast<const float4 *>(Wt + (size_t)k * H + j0));
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float a = in[(s0 + u) * inStride + k];
-      acc[u][0] = fmaf(a, w.x, acc[u][0]);
-      acc[u][1] = fmaf(a, w.y, acc[u][1]);
-      acc[u][2] = fmaf(a, w.z, acc[u][2]);
-      acc[u][3] = fmaf(a, w.w, acc[u][3]);
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) out[(s0 + u) * H + j0 + v] = acc[u][v];
-}
-
-// g[j][k] += sum_s delta[s][j] * act[s][k] over the tile (k < K, act row
-// stride actStride), then bias g_b[j] += sum_s delta[s][j].
-template <int H>
-__device__ __forceinline__ void weightGrad(const float *delta, const float *act, int actStride,
-                                           int K, int S, float *__restrict__ gW,
-                                           float *__restrict__ gB) {
-  const int t = threadIdx.x;
-  if ((K & 3) == 0) {
-    const int tiles = (H / 4) * (K / 4);
-    for (int e = t; e < tiles; e += blockDim.x) {
-      const int j0 = (e / (K / 4)) * 4, k0 = (e % (K / 4)) * 4;
-      float acc[4][4] = {};
-      for (int s = 0; s < S; ++s) {
-        float dj[4], ak[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          dj[u] = delta[s * H + j0 + u];
-          ak[u] = act[s * actStride + k0 + u];
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(dj[u], ak[v], acc[u][v]);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) atomicAdd(gW + (j0 + u) * K + k0 + v, acc[u][v]);
-    }
-  } else {
-    for (int e = t; e < H * K; e += blockDim.x) {
-      const int j = e / K, k = e % K;
-      float acc = 0.0f;
-      for (int s = 0; s < S; ++s) acc = fmaf(delta[s * H + j], act[s * actStride + k], acc);
-      atomicAdd(gW + e, acc);
-    }
-  }
-  for (int j = t; j < H; j += blockDim.x) {
-    float acc = 0.0f;
-    for (int s = 0; s < S; ++s) acc += delta[s * H + j];
-    atomicAdd(gB + j, acc);
-  }
-}
+// Floats of one row of gradient sums: the parameters, rounded up to 16 bytes
+// (every hidden layer's weights start on 16 bytes in it).
+__host__ __device__ constexpr unsigned partialRow(unsigned total) { return (total + 3u) & ~3u; }
 
 template <int H, int L>
-constexpr size_t trainSmemBytes() {
-  constexpr int S = 4096 / H;
-  return sizeof(float) * ((size_t)S * kSdfMaxInputs + 2 * (size_t)L * S * H + 2 * (size_t)S * H +
-                          2 * (size_t)S);
-}
+struct TrainSmem {
+  static constexpr int kRow = H + 4;
+  float w[L - 1][H][kRow];                 // hidden layers, [out][in]
+  float z[L][kTrainS][kRow];               // pre-activations
+  float a[L][kTrainS][kRow];               // activations
+  float d[2][kTrainS][kRow];               // deltas
+  float x[kTrainS][kSdfMaxInputs];
+  float w0[kSdfMaxInputs][H];              // first layer, [in][out]
+  float b[L][H], wo[H];
+  float dy[kTrainS];
+};
 
-// Sample s of the tile is samples[base + s]: input (x - shift) * scale and
-// the one-hot shape code, target d / outScale, weight 1 + 9 [|d| < band].
-// kBackward: adds invB * the gradient of sum_s w (y - t)^2 to grad and the
-// loss term to *loss; otherwise writes the distance prediction to yOut.
+// Sample s of a tile is samples[base + s]: input (x - shift) * scale and the
+// one-hot shape code, target d / outScale, weight 1 + 9 [|d| < band].
+// kBackward: the CTA's sums of invB * the gradient of sum_s w (y - t)^2 go to
+// partial[blockIdx.x] and the loss terms are added to *lossSum; otherwise
+// writes the distance prediction to yOut.
 template <int H, int L, bool kBackward>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(4 * H, 1)
 kSdfTrain(SdfView net, const float4 *__restrict__ samples, const int *__restrict__ shapes,
-          unsigned n, float band, float invB, float *__restrict__ grad, float *__restrict__ loss,
-          float *__restrict__ yOut) {
-  constexpr int S = 4096 / H;
-  extern __shared__ __align__(16) float smf[];
-  float *X = smf;                              // [S][kSdfMaxInputs]
-  float *Z = X + S * kSdfMaxInputs;            // [L][S][H] pre-activations
-  float *A = Z + L * S * H;                    // [L][S][H] activations
-  float *D0 = A + L * S * H;                   // [S][H] deltas
-  float *D1 = D0 + S * H;
-  float *yv = D1 + S * H;                      // [S]
-  float *dyv = yv + S;                         // [S]
+          unsigned n, float band, float invB, float *__restrict__ partial,
+          float *__restrict__ lossSum, float *__restrict__ yOut) {
+  extern __shared__ __align__(1024) unsigned char smraw[];
+  TrainSmem<H, L> &sm = *reinterpret_cast<TrainSmem<H, L> *>(smraw);
+  constexpr int T = 4 * H, S = kTrainS, Q = H / 4;
+  constexpr int kBlocks = Q * Q / T;  // 4 x 4 weight-gradient blocks per thread and layer
   const SdfLayout &ly = net.lay;
   const int D = ly.D;
   const int t = threadIdx.x;
-  const unsigned base = blockIdx.x * S;
-  for (int e = t; e < S * kSdfMaxInputs; e += blockDim.x) {
-    const int s = e / kSdfMaxInputs, d = e % kSdfMaxInputs;
-    const unsigned idx = base + s;
+  const int row = t / Q, col = t % Q;  // this thread's sample and column group
+  chainTrigger();
+  const unsigned tiles = (n + S - 1) / S;
+  // thread t < 256 stages input t % 16 of sample t / 16, read one tile ahead
+  auto input = [&](unsigned tile) {
+    const int s = t / kSdfMaxInputs, d = t % kSdfMaxInputs;
+    const unsigned idx = tile * S + s;
     float v = 0.0f;
-    if (idx < n && d < D) {
+    if (tile < tiles && t < S * kSdfMaxInputs && idx < n && d < D) {
       const float4 q = __ldg(samples + idx);
       if (d < 3)
         v = ((d == 0 ? q.x : (d == 1 ? q.y : q.z)) - net.shift[d]) * net.scale[d];
       else
         v = (shapes && __ldg(shapes + idx) == d - 3) ? 1.0f : 0.0f;
     }
-    X[e] = v;
+    return v;
+  };
+  float x0 = input(blockIdx.x);
+  chainWait();  // the weights
+#pragma unroll 1
+  for (int l = 1; l < L; ++l) {  // (the layers' weights start on 16 bytes: widths of 64 or 128)
+    const float4 *src = reinterpret_cast<const float4 *>(net.p + ly.wh[l - 1]);
+#pragma unroll 4
+    for (int e = t; e < H * Q; e += T)
+      *reinterpret_cast<float4 *>(&sm.w[l - 1][e / Q][4 * (e % Q)]) = __ldg(src + e);
   }
-  __syncthreads();
-  gemmTile<H>(X, kSdfMaxInputs, D, net.pT + ly.w0, net.p + ly.b0, Z);
-  __syncthreads();
-  for (int e = t; e < S * H; e += blockDim.x) A[e] = silu(Z[e]);
-  __syncthreads();
-  for (int l = 1; l < L; ++l) {
-    gemmTile<H>(A + (l - 1) * S * H, H, H, net.pT + ly.wh[l - 1], net.p + ly.bh[l - 1],
-                Z + l * S * H);
-    __syncthreads();
-    for (int e = t; e < S * H; e += blockDim.x) A[l * S * H + e] = silu(Z[l * S * H + e]);
-    __syncthreads();
+  for (int e = t; e < H * D; e += T) sm.w0[e % D][e / D] = __ldg(net.p + ly.w0 + e);
+  if (t < H) {
+    sm.b[0][t] = __ldg(net.p + ly.b0 + t);
+    for (int l = 1; l < L; ++l) sm.b[l][t] = __ldg(net.p + ly.bh[l - 1] + t);
+    sm.wo[t] = __ldg(net.p + ly.wo + t);
   }
-  const float *AL = A + (L - 1) * S * H;
-  for (int s = t; s < S; s += blockDim.x) {
-    float y = __ldg(net.p + ly.bo);
-    for (int k = 0; k < H; ++k) y = fmaf(AL[s * H + k], __ldg(net.p + ly.wo + k), y);
-    yv[s] = y;
-    const unsigned idx = base + s;
-    if (!kBackward) {
-      if (idx < n) yOut[idx] = y * net.outScale;
-    } else {
-      float dy = 0.0f;
-      if (idx < n) {
-        const float d = __ldg(samples + idx).w;
-        const float target = d / net.outScale;
-        const float w = fabsf(d) < band ? 10.0f : 1.0f;
-        const float r = y - target;
-        dy = 2.0f * w * r * invB;
-        atomicAdd(loss, w * r * r * invB);
+  const float bo = __ldg(net.p + ly.bo);
+  // gradient sums over the CTA's tiles
+  float gW[L - 1][kBlocks][4][4] = {}, gW0[4] = {}, gB[L] = {}, gWo = 0.0f, gBo = 0.0f;
+  for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const unsigned base = tile * S;
+    __syncthreads();  // the weights are in place; the last tile's readers are done
+    if (t < S * kSdfMaxInputs) sm.x[t / kSdfMaxInputs][t % kSdfMaxInputs] = x0;
+    __syncthreads();
+    x0 = input(tile + gridDim.x);
+    float act[4];  // this thread's activations of the layer
+    {  // first layer
+      float acc[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[u] = sm.b[0][col + Q * u];
+      for (int k = 0; k < D; ++k) {
+        const float x = sm.x[row][k];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) acc[u] = fmaf(x, sm.w0[k][col + Q * u], acc[u]);
       }
-      dyv[s] = dy;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        sm.z[0][row][col + Q * u] = acc[u];
+        act[u] = silu(acc[u]);
+        sm.a[0][row][col + Q * u] = act[u];
+      }
+    }
+#pragma unroll
+    for (int l = 1; l < L; ++l) {
+      __syncthreads();
+      float acc[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[u] = sm.b[l][col + Q * u];
+#pragma unroll 4
+      for (int k = 0; k < H; k += 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(&sm.a[l - 1][row][k]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float4 w = *reinterpret_cast<const float4 *>(&sm.w[l - 1][col + Q * u][k]);
+          acc[u] = fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, acc[u]))));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        sm.z[l][row][col + Q * u] = acc[u];
+        act[u] = silu(acc[u]);
+        sm.a[l][row][col + Q * u] = act[u];
+      }
+    }
+    // output layer, loss and its derivative: the Q lanes of a sample share it
+    float dy = 0.0f;
+    {
+      float y = 0.0f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) y = fmaf(act[u], sm.wo[col + Q * u], y);
+#pragma unroll
+      for (int o = Q / 2; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+      y += bo;
+      const unsigned idx = base + row;
+      if (!kBackward) {
+        if (col == 0 && idx < n) yOut[idx] = y * net.outScale;
+        continue;
+      }
+      if (idx < n) {
+        const float d = __ldg(&samples[idx].w);
+        const float w = fabsf(d) < band ? 10.0f : 1.0f;
+        const float r = y - d / net.outScale;
+        dy = 2.0f * w * r * invB;
+        if (col == 0) atomicAdd(lossSum, w * r * r * invB);
+      }
+      if (col == 0) sm.dy[row] = dy;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = col + Q * u;
+      sm.d[(L - 1) & 1][row][k] = dy * sm.wo[k] * dsilu(sm.z[L - 1][row][k]);
+    }
+    __syncthreads();
+    if (t < H) {
+#pragma unroll 4
+      for (int s = 0; s < S; ++s) gWo = fmaf(sm.dy[s], sm.a[L - 1][s][t], gWo);
+    }
+    if (t == T - 1) {
+#pragma unroll 4
+      for (int s = 0; s < S; ++s) gBo += sm.dy[s];
+    }
+#pragma unroll
+    for (int l = L - 1; l >= 1; --l) {
+      if (l < L - 1) __syncthreads();
+      const float(*cur)[TrainSmem<H, L>::kRow] = sm.d[l & 1];
+      float(*nxt)[TrainSmem<H, L>::kRow] = sm.d[(l - 1) & 1];
+      // weight gradient: block e of the layer is rows 4 (e / Q), columns 4 (e % Q)
+#pragma unroll
+      for (int e = 0; e < kBlocks; ++e) {
+        const int j0 = 4 * ((t + e * T) / Q), k0 = 4 * ((t + e * T) % Q);
+#pragma unroll 4
+        for (int s = 0; s < S; ++s) {
+          const float4 dj = *reinterpret_cast<const float4 *>(&cur[s][j0]);
+          const float4 ak = *reinterpret_cast<const float4 *>(&sm.a[l - 1][s][k0]);
+          const float dv[4] = {dj.x, dj.y, dj.z, dj.w}, av[4] = {ak.x, ak.y, ak.z, ak.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) gW[l - 1][e][u][v] = fmaf(dv[u], av[v], gW[l - 1][e][u][v]);
+        }
+      }
+      if (t < H) {
+        float acc = 0.0f;
+#pragma unroll 4
+        for (int s = 0; s < S; ++s) acc += cur[s][t];
+        gB[l] += acc;
+      }
+      // nxt[row][k] = dsilu * sum_j cur[row][j] W[j][k], four columns from 4 col
+      float acc[4] = {};
+#pragma unroll 4
+      for (int j = 0; j < H; j += 4) {
+        const float4 c = *reinterpret_cast<const float4 *>(&cur[row][j]);
+        const float cv[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float4 w = *reinterpret_cast<const float4 *>(&sm.w[l - 1][j + q][4 * col]);
+          acc[0] = fmaf(cv[q], w.x, acc[0]);
+          acc[1] = fmaf(cv[q], w.y, acc[1]);
+          acc[2] = fmaf(cv[q], w.z, acc[2]);
+          acc[3] = fmaf(cv[q], w.w, acc[3]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        nxt[row][4 * col + u] = acc[u] * dsilu(sm.z[l - 1][row][4 * col + u]);
+    }
+    __syncthreads();
+    // first layer: thread t has output t % H, inputs t / H, t / H + 4, ...
+    const float(*d0)[TrainSmem<H, L>::kRow] = sm.d[0];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = t / H + 4 * u;
+      if (k < D)
+#pragma unroll 4
+        for (int s = 0; s < S; ++s) gW0[u] = fmaf(d0[s][t % H], sm.x[s][k], gW0[u]);
+    }
+    if (t < H) {
+      float acc = 0.0f;
+#pragma unroll 4
+      for (int s = 0; s < S; ++s) acc += d0[s][t];
+      gB[0] += acc;
     }
   }
   if (!kBackward) return;
-  __syncthreads();
-  for (int k = t; k < H; k += blockDim.x) {
-    float acc = 0.0f;
-    for (int s = 0; s < S; ++s) acc = fmaf(dyv[s], AL[s * H + k], acc);
-    atomicAdd(grad + ly.wo + k, acc);
+  float *g = partial + (size_t)blockIdx.x * partialRow(ly.total);
+#pragma unroll
+  for (int l = 1; l < L; ++l)
+#pragma unroll
+    for (int e = 0; e < kBlocks; ++e)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        *reinterpret_cast<float4 *>(g + ly.wh[l - 1] + (4 * ((t + e * T) / Q) + u) * H +
+                                    4 * ((t + e * T) % Q)) =
+            make_float4(gW[l - 1][e][u][0], gW[l - 1][e][u][1], gW[l - 1][e][u][2],
+                        gW[l - 1][e][u][3]);
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (t / H + 4 * u < D) g[ly.w0 + (t % H) * D + t / H + 4 * u] = gW0[u];
+  if (t < H) {
+    g[ly.b0 + t] = gB[0];
+#pragma unroll
+    for (int l = 1; l < L; ++l) g[ly.bh[l - 1] + t] = gB[l];
+    g[ly.wo + t] = gWo;
   }
-  if (t == 0) {
-    float acc = 0.0f;
-    for (int s = 0; s < S; ++s) acc += dyv[s];
-    atomicAdd(grad + ly.bo, acc);
-  }
-  for (int e = t; e < S * H; e += blockDim.x) {
-    const int s = e / H, k = e % H;
-    D0[e] = dyv[s] * __ldg(net.p + ly.wo + k) * dsilu(Z[(L - 1) * S * H + e]);
-  }
-  __syncthreads();
-  float *cur = D0, *nxt = D1;
-  for (int l = L - 1; l >= 1; --l) {
-    weightGrad<H>(cur, A + (l - 1) * S * H, H, H, S, grad + ly.wh[l - 1], grad + ly.bh[l - 1]);
-    // nxt[s][k] = sum_j cur[s][j] W[j][k]: W row-major is the transposed operand
-    gemmTile<H>(cur, H, H, net.p + ly.wh[l - 1], nullptr, nxt);
-    __syncthreads();
-    for (int e = t; e < S * H; e += blockDim.x) nxt[e] *= dsilu(Z[(l - 1) * S * H + e]);
-    __syncthreads();
-    float *tmp = cur;
-    cur = nxt;
-    nxt = tmp;
-  }
-  weightGrad<H>(cur, X, kSdfMaxInputs, D, S, grad + ly.w0, grad + ly.b0);
+  if (t == T - 1) g[ly.bo] = gBo;
 }
 
-// Adam step over all parameters, then the transposed copy of every weight.
-__global__ void __launch_bounds__(256)
-kSdfAdam(SdfLayout ly, float *__restrict__ p, float *__restrict__ pT,
-         const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v, float lr,
-         float b1, float b2, float eps, float c1, float c2) {
-  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ly.total) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float pi = p[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-  p[i] = pi;
-  unsigned j = i;  // transposed position
-  if (i >= ly.w0 && i < ly.w0 + (unsigned)(ly.H * ly.D)) {
-    const unsigned r = i - ly.w0;
-    j = ly.w0 + (r % ly.D) * ly.H + r / ly.D;
+// Adds the `parts` rows of partial (32 parameters per CTA, the rows shared out
+// over its warps, added in a fixed order).  kAdam: one Adam step on the
+// parameters; otherwise the sums go to grad.
+constexpr int kReduceWarps = 8;
+template <bool kAdam>
+__global__ void __launch_bounds__(32 * kReduceWarps)
+kSdfReduce(const float *__restrict__ partial, unsigned parts, unsigned total, float *__restrict__ p,
+           float *__restrict__ grad, float *__restrict__ m, float *__restrict__ v,
+           float lr, float b1, float b2, float eps, float c1, float c2) {
+  __shared__ float sSum[kReduceWarps][32];
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const unsigned i = blockIdx.x * 32u + lane;
+  chainTrigger();
+  chainWait();
+  float acc = 0.0f, p0 = 0.0f, m0 = 0.0f, v0 = 0.0f;
+  if (kAdam && warp == 0 && i < total) {
+    p0 = p[i];
+    m0 = m[i];
+    v0 = v[i];
   }
-  for (int l = 1; l < ly.L; ++l) {
-    const unsigned w = ly.wh[l - 1];
-    if (i >= w && i < w + (unsigned)(ly.H * ly.H)) {
-      const unsigned r = i - w;
-      j = w + (r % ly.H) * ly.H + r / ly.H;
-    }
+  if (i < total) {
+#pragma unroll 8
+    for (unsigned r = warp; r < parts; r += kReduceWarps)
+      acc += __ldg(partial + (size_t)r * partialRow(total) + i);
   }
-  pT[j] = pi;
+  sSum[warp][lane] = acc;
+  __syncthreads();
+  if (warp != 0 || i >= total) return;
+#pragma unroll
+  for (int w = 1; w < kReduceWarps; ++w) acc += sSum[w][lane];
+  if (!kAdam) {
+    grad[i] = acc;
+  } else {
+    const float mi = b1 * m0 + (1.0f - b1) * acc;
+    const float vi = b2 * v0 + (1.0f - b2) * acc * acc;
+    m[i] = mi;
+    v[i] = vi;
+    p[i] = p0 - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -953,8 +1033,9 @@ struct fcdemSdfNet {
   int device = -1;
   SdfLayout lay{};
   float shift[3] = {0.0f, 0.0f, 0.0f}, scale[3] = {1.0f, 1.0f, 1.0f}, outScale = 1.0f;
-  float *params = nullptr, *paramsT = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
+  float *params = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
   float *loss = nullptr;  // one device float
+  float *partial = nullptr;  // kSdfTrain: numSms() rows of gradient sums (first training call)
   __nv_bfloat16 *w16 = nullptr;
   bool w16Fresh = false;
   unsigned adamStep = 0;
@@ -977,7 +1058,6 @@ SdfView sdfView(const fcdemSdfNet *net) {
   SdfView v;
   v.lay = net->lay;
   v.p = net->params;
-  v.pT = net->paramsT;
   v.w16 = net->w16;
   for (int k = 0; k < 3; ++k) {
     v.shift[k] = net->shift[k];
@@ -990,40 +1070,40 @@ SdfView sdfView(const fcdemSdfNet *net) {
 void freeNet(fcdemSdfNet *net) {
   if (!net) return;
   cudaFree(net->params);
-  cudaFree(net->paramsT);
   cudaFree(net->grad);
   cudaFree(net->m);
   cudaFree(net->v);
   cudaFree(net->loss);
+  cudaFree(net->partial);
   cudaFree(net->w16);
   cudaFree(net->hints);
   cudaFree(net->tileBuf);
   delete net;
 }
 
-std::vector<float> transposed(const SdfLayout &ly, const std::vector<float> &p) {
-  std::vector<float> t(p);
-  for (int j = 0; j < ly.H; ++j)
-    for (int d = 0; d < ly.D; ++d) t[ly.w0 + d * ly.H + j] = p[ly.w0 + j * ly.D + d];
-  for (int l = 1; l < ly.L; ++l)
-    for (int j = 0; j < ly.H; ++j)
-      for (int k = 0; k < ly.H; ++k)
-        t[ly.wh[l - 1] + k * ly.H + j] = p[ly.wh[l - 1] + j * ly.H + k];
-  return t;
-}
-
 bool uploadParams(fcdemSdfNet *net, const std::vector<float> &p) {
-  const std::vector<float> t = transposed(net->lay, p);
   const size_t bytes = sizeof(float) * p.size();
   net->w16Fresh = false;
   net->version++;
-  return cudaOk(cudaMemcpy(net->params, p.data(), bytes, cudaMemcpyHostToDevice)) &&
-         cudaOk(cudaMemcpy(net->paramsT, t.data(), bytes, cudaMemcpyHostToDevice));
+  return cudaOk(cudaMemcpy(net->params, p.data(), bytes, cudaMemcpyHostToDevice));
 }
 
 template <int H, int L>
 size_t tileSmemBytes() {
   return sizeof(SdfTileSmem<H, L>) + 1024;  // + alignment slack
+}
+
+// Opts a kernel into its dynamic shared memory, once per device (a bit each).
+template <class Kernel>
+bool smemReady(Kernel *kernel, int bytes, std::atomic<unsigned long long> &ready) {
+  int dev = 0;
+  if (!cudaOk(cudaGetDevice(&dev))) return false;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (ready.load(std::memory_order_relaxed) & bit) return true;
+  if (!cudaOk(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)))
+    return false;
+  ready.fetch_or(bit, std::memory_order_relaxed);
+  return true;
 }
 
 bool packWeights(fcdemSdfNet *net) {
@@ -1034,29 +1114,44 @@ bool packWeights(fcdemSdfNet *net) {
   return true;
 }
 
-// Runs the forward (+ backward) tile kernel over n samples.
+// Runs the forward (+ backward) tile kernel over n samples; parts receives
+// the rows of net->partial that the backward pass wrote.  chained: the kernel
+// before it on the stream is this call's own.
 bool runTrainKernel(fcdemSdfNet *net, bool backward, const float4 *samples, const int *shapes,
-                    unsigned n, float band, float invB, float *yOut) {
+                    unsigned n, float band, float invB, float *yOut, unsigned *parts = nullptr,
+                    bool chained = false) {
+  const unsigned sms = numSms();
+  if (backward && !net->partial &&
+      cudaMalloc(&net->partial, sizeof(float) * (size_t)sms * partialRow(net->lay.total)) !=
+          cudaSuccess) {
+    cudaGetLastError();
+    net->partial = nullptr;
+    setError(FCDEM_ERR_ALLOC);
+    return false;
+  }
   const SdfView v = sdfView(net);
   const int H = net->lay.H, L = net->lay.L;
-  const unsigned S = 4096u / (unsigned)H;
-  const unsigned blocks = (n + S - 1) / S;
-  cudaStream_t st = curStream();
-#define FCDEM_SDF_TRAIN(HH, LL)                                                              \
-  if (H == HH && L == LL) {                                                                  \
-    const size_t smem = trainSmemBytes<HH, LL>();                                            \
-    if (backward) {                                                                          \
-      cudaFuncSetAttribute(kSdfTrain<HH, LL, true>,                                          \
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
-      kSdfTrain<HH, LL, true><<<blocks, 256, smem, st>>>(v, samples, shapes, n, band, invB,  \
-                                                         net->grad, net->loss, nullptr);     \
-    } else {                                                                                 \
-      cudaFuncSetAttribute(kSdfTrain<HH, LL, false>,                                         \
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
-      kSdfTrain<HH, LL, false><<<blocks, 256, smem, st>>>(v, samples, shapes, n, band, invB, \
-                                                          nullptr, nullptr, yOut);           \
-    }                                                                                        \
-    return launchOk();                                                                       \
+  const unsigned tiles = (n + kTrainS - 1) / kTrainS;
+  // one CTA per SM (its row of partial sums); two of the narrow ones forward
+  const unsigned most = backward || H != 64 ? sms : 2u * sms;
+  const unsigned blocks = tiles < most ? tiles : most;
+  if (parts) *parts = blocks;
+#define FCDEM_SDF_TRAIN(HH, LL)                                                               \
+  if (H == HH && L == LL) {                                                                   \
+    constexpr int smem = (int)sizeof(TrainSmem<HH, LL>);                                      \
+    static_assert(smem <= 227 * 1024, "shared memory of a CTA");                              \
+    if (backward) {                                                                           \
+      static std::atomic<unsigned long long> ready{0};                                        \
+      if (!smemReady(kSdfTrain<HH, LL, true>, smem, ready)) return false;                     \
+      launchChained(chained, kSdfTrain<HH, LL, true>, blocks, 4 * HH, smem, v, samples,       \
+                    shapes, n, band, invB, net->partial, net->loss, nullptr);                 \
+    } else {                                                                                  \
+      static std::atomic<unsigned long long> ready{0};                                        \
+      if (!smemReady(kSdfTrain<HH, LL, false>, smem, ready)) return false;                    \
+      launchChained(false, kSdfTrain<HH, LL, false>, blocks, 4 * HH, smem, v, samples,        \
+                    shapes, n, band, invB, nullptr, nullptr, yOut);                           \
+    }                                                                                         \
+    return launchOk();                                                                        \
   }
   FCDEM_SDF_TRAIN(64, 3)
   FCDEM_SDF_TRAIN(64, 2)
@@ -1067,15 +1162,24 @@ bool runTrainKernel(fcdemSdfNet *net, bool backward, const float4 *samples, cons
   return false;
 }
 
-bool adamStep(fcdemSdfNet *net, float lr) {
+// The batch gradient (lr < 0) or one Adam step from the rows of net->partial.
+bool reducePartials(fcdemSdfNet *net, unsigned parts, float lr) {
+  const unsigned total = net->lay.total, blocks = (total + 31u) / 32u;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  if (lr < 0.0f) {
+    launchChained(
+        true, kSdfReduce<false>, blocks, 32 * kReduceWarps, 0, net->partial, parts, total, net->params, net->grad, net->m, net->v, 0.0f, b1,
+        b2, eps, 0.0f, 0.0f);
+    return launchOk();
+  }
   net->adamStep++;
   net->version++;
   const double t = (double)net->adamStep;
   const float c1 = (float)(1.0 / (1.0 - std::pow((double)b1, t)));
   const float c2 = (float)(1.0 / (1.0 - std::pow((double)b2, t)));
-  kSdfAdam<<<(net->lay.total + 255) / 256, 256, 0, curStream()>>>(
-      net->lay, net->params, net->paramsT, net->grad, net->m, net->v, lr, b1, b2, eps, c1, c2);
+  launchChained(
+      true, kSdfReduce<true>, blocks, 32 * kReduceWarps, 0, net->partial, parts, total, net->params, net->grad, net->m, net->v, lr, b1, b2,
+      eps, c1, c2);
   net->w16Fresh = false;
   return launchOk();
 }
@@ -1349,7 +1453,6 @@ fcdemSdfNet *fcdemSdfCreate(int inputs, int hidden, int hiddenLayers, unsigned l
   const size_t bytes = sizeof(float) * net->lay.total;
   const size_t w16 = sizeof(__nv_bfloat16) * (size_t)(hiddenLayers - 1) * hidden * hidden;
   bool ok = cudaMalloc(&net->params, bytes) == cudaSuccess &&
-            cudaMalloc(&net->paramsT, bytes) == cudaSuccess &&
             cudaMalloc(&net->grad, bytes) == cudaSuccess &&
             cudaMalloc(&net->m, bytes) == cudaSuccess && cudaMalloc(&net->v, bytes) == cudaSuccess &&
             cudaMalloc(&net->loss, sizeof(float)) == cudaSuccess &&
@@ -1452,11 +1555,11 @@ float fcdemSdfGradient(fcdemSdfNet *net, const float *samples4, const int *shape
                        float band, float *gradHost) {
   if (!net || !samples4 || n == 0) { setError(FCDEM_ERR_INVALID_VALUE); return 0.0f; }
   const size_t bytes = sizeof(float) * net->lay.total;
-  if (!cudaOk(cudaMemsetAsync(net->grad, 0, bytes, curStream())) ||
-      !cudaOk(cudaMemsetAsync(net->loss, 0, sizeof(float), curStream())))
-    return 0.0f;
+  if (!cudaOk(cudaMemsetAsync(net->loss, 0, sizeof(float), curStream()))) return 0.0f;
+  unsigned parts = 0;
   if (!runTrainKernel(net, true, (const float4 *)samples4, shapes, n, band, 1.0f / (float)n,
-                      nullptr))
+                      nullptr, &parts) ||
+      !reducePartials(net, parts, -1.0f))
     return 0.0f;
   float loss = 0.0f;
   cudaOk(cudaStreamSynchronize(curStream()));
@@ -1471,7 +1574,6 @@ float fcdemSdfTrainSamples(fcdemSdfNet *net, const float *samples4, const int *s
     setError(FCDEM_ERR_INVALID_VALUE);
     return 0.0f;
   }
-  const size_t bytes = sizeof(float) * net->lay.total;
   const unsigned batches = (n + batch - 1) / batch;
   const unsigned total = batches * epochs;
   float last = 0.0f;
@@ -1484,11 +1586,11 @@ float fcdemSdfTrainSamples(fcdemSdfNet *net, const float *samples4, const int *s
       const double prog = (double)(e * batches + b) / (double)total;
       const float lrNow =
           (float)(lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(3.14159265358979 * prog))));
-      if (!cudaOk(cudaMemsetAsync(net->grad, 0, bytes, curStream()))) return 0.0f;
+      unsigned parts = 0;
       if (!runTrainKernel(net, true, (const float4 *)samples4 + off, shapes ? shapes + off : nullptr,
-                          cnt, band, 1.0f / (float)cnt, nullptr))
+                          cnt, band, 1.0f / (float)cnt, nullptr, &parts, e + b > 0) ||
+          !reducePartials(net, parts, lrNow))
         return 0.0f;
-      if (!adamStep(net, lrNow)) return 0.0f;
     }
     if (e + 1 == epochs) {
       cudaOk(cudaStreamSynchronize(curStream()));

@@ -96,6 +96,35 @@ def test_training_gradient_matches_fp64_oracle(cfg):
     assert np.linalg.norm(err) <= 1e-5 * np.linalg.norm(gref) * 10
 
 
+@pytest.mark.parametrize("cfg", CONFIGS + [(16, 64, 3), (16, 128, 3)])
+@pytest.mark.parametrize("n", [1, 15, 17, 152 * 16 + 5, 304 * 16 + 3])
+def test_training_tiles_match_fp64_oracle(cfg, n):
+    """The 16-sample tiles at their edges: one sample, a partial tile, more
+    tiles than CTAs (each CTA sums several), every shape code.  Tolerances of
+    the test above; twice the same call gives the same gradient bits."""
+    from fullc0ntact_gb300 import sdf
+    dmap = _torus()
+    net = _net(*cfg, dmap, jitter=0.05)
+    s = sdf.samples(dmap, n, 0.5, 0.05, seed=n)
+    shapes = None
+    if cfg[0] > 3:
+        shapes = (torch.arange(n, device="cuda") % (cfg[0] - 3)).to(torch.int32)
+    loss, g = net.gradient(s, shapes, 0.02)
+    shift, scale, out_scale = net.normalization()
+    lref, gref = so.loss_and_grad(net.get_params().astype(np.float64), so.layout(*cfg),
+                                  s.cpu().numpy().astype(np.float64),
+                                  None if shapes is None else shapes.cpu().numpy(),
+                                  0.02, shift, scale, out_scale)
+    assert abs(loss - lref) <= 1e-5 * abs(lref) + 1e-7
+    err = np.abs(g.astype(np.float64) - gref)
+    assert np.max(err) <= 1e-4 * np.max(np.abs(gref))
+    assert np.linalg.norm(err) <= 1e-4 * np.linalg.norm(gref)
+    np.testing.assert_array_equal(net.gradient(s, shapes, 0.02)[1], g)
+    ref = _torch_forward(net, s, shapes)
+    tol = 1e-5 * float(ref.abs().max()) + 1e-6
+    assert float((net.eval_f32(s, shapes) - ref).abs().max()) <= tol
+
+
 @pytest.mark.parametrize("cfg", CONFIGS)
 def test_fp32_forward_matches_torch(cfg):
     from fullc0ntact_gb300 import sdf
