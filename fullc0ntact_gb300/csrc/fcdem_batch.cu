@@ -76,7 +76,7 @@ bool runBatchObstacles(fcdemBatch *b, const CountBuffers &cb, float4 *pos, float
     return false;
   for (unsigned s = 0; s < steps; ++s) {
     if (!countPipelineSort(c, cb, s == 0 ? nullptr : b->index, pos, vel, b->hash, b->index,
-                           b->sortedPos, b->sortedVel, b->n, b->numCells))
+                           b->sortedPos, b->sortedVel, b->n, b->numCells, nullptr))
       return false;
     const bool last = (s + 1 == steps);
     CollideOut out;
@@ -102,7 +102,7 @@ bool runBatch(fcdemBatch *b, float4 *pos, float4 *vel, float dt, unsigned steps)
     return false;
   for (unsigned s = 0; s < steps; ++s) {
     if (!countPipelineSort(c, cb, s == 0 ? nullptr : b->index, pos, vel, b->hash, b->index,
-                           b->sortedPos, b->sortedVel, b->n, b->numCells))
+                           b->sortedPos, b->sortedVel, b->n, b->numCells, nullptr))
       return false;
     const bool last = (s + 1 == steps);
     CollideOut out;

@@ -69,8 +69,8 @@ __device__ __forceinline__ void cellTerms(unsigned start, unsigned end, unsigned
 template <int kMode, bool kCollider, bool kForceOut>
 __device__ __forceinline__ void finishParticle(
     unsigned i, unsigned n, float3 pos, float3 vel, float4 p4, float ri,
-    float3 force, const unsigned *__restrict__ index, float4 *__restrict__ newVel,
-    const CollideOut &out, const SimParams &P) {
+    float3 force, const unsigned *index, float4 *newVel, const CollideOut &out,
+    const SimParams &P) {
   if (kCollider) {
     float3 rel = make_float3(P.colliderPos[0] - pos.x, P.colliderPos[1] - pos.y,
                              P.colliderPos[2] - pos.z);
@@ -97,7 +97,7 @@ __device__ __forceinline__ void finishParticle(
     countTile(out.tileCnt, h >> 12);  // per 4096-cell tile (the scan's)
     return;
   }
-  unsigned o = __ldg(index + i);
+  unsigned o = index[i];
   if (o >= n) return;  // not a permutation of 0..n-1: nothing to write to
   if (kForceOut) out.force[o] = force;
   if (kMode == 0 || kMode == 3) {
@@ -281,11 +281,6 @@ __device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b) {
 __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
   f32x2 r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
@@ -1037,11 +1032,11 @@ void applyCollideConfig(int k) {
 }
 
 // The group list for n particles (grown on demand; at most one group per
-// particle), its counters cleared on the current stream.  groups == nullptr
-// when the path is off or the list cannot be had.
+// particle).  groups == nullptr when the path is off, no neighbourhood can
+// reach the limit, or the list cannot be had.
 CrowdList crowdList(unsigned n) {
   CrowdList cl{nullptr, nullptr, 0u, g_crowdLimit};
-  if (!g_crowdPath) return cl;
+  if (!g_crowdPath || n <= g_crowdLimit) return cl;
   Context &c = ctx();
   if (c.crowdBuf == nullptr || c.crowdCap < n) {
     if (!cudaOk(cudaDeviceSynchronize())) return cl;
@@ -1055,7 +1050,6 @@ CrowdList crowdList(unsigned n) {
     }
     c.crowdCap = n;
   }
-  if (!cudaOk(cudaMemsetAsync(c.crowdBuf, 0, 8, curStream()))) return cl;
   cl.count = (unsigned *)c.crowdBuf;
   cl.groups = (uint2 *)((char *)c.crowdBuf + 16);
   cl.cap = n;
@@ -1072,14 +1066,21 @@ void launchT(bool tiled, bool cull, unsigned n, float4 *newVel, const float4 *sp
         <<<blocks, kTileThreads, 0, curStream()>>>(newVel, sp, sv, index, cells, n, kp, out,
                                                    ctx().dStatus);
   else {
-    const CrowdList crowd = crowdList(n);
+    CrowdList crowd = crowdList(n);
+    // (on the prefix table the scan has cleared the counters)
+    if (!kPrefix && crowd.groups && !cudaOk(cudaMemsetAsync(crowd.count, 0, 8, curStream())))
+      crowd.groups = nullptr;
     kCollideGlobal<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix>
-        <<<blocks, 128, 0, curStream()>>>(newVel, sp, sv, index, cells, n, kp, out, cull,
-                                          crowd, ctx().dStatus);
-    if (crowd.groups && launchOk())
+        <<<blocks, 128, 0, curStream()>>>(newVel, sp, sv, index, cells, n, kp, out, cull, crowd,
+                                          ctx().dStatus);
+    if (crowd.groups && launchOk()) {
+      // groups have up to 32 members: no more warps than that can be busy
+      const unsigned most = (n + 32 * kCrowdWarps - 1) / (32 * kCrowdWarps);
+      const unsigned all = numSms() * g_crowdCtasPerSm;
       kCollideCrowd<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix>
-          <<<numSms() * g_crowdCtasPerSm, kCrowdWarps * 32, 0, curStream()>>>(
+          <<<most < all ? most : all, kCrowdWarps * 32, 0, curStream()>>>(
               newVel, sp, sv, index, cells, n, kp, out, cull, crowd, ctx().dStatus);
+    }
   }
 }
 
@@ -1166,6 +1167,8 @@ int g_collidePath = -1;  // -1 auto, 0 global, 1 tiled (fcdemSetCollidePath)
 bool g_cullCells = true;  // fcdemSetCellCulling
 
 }  // namespace
+
+unsigned *collideCrowdCount(unsigned n) { return crowdList(n).count; }
 
 void launchCollide(int mode, bool collider, float4 *newVel, const float4 *sp,
                    const float4 *sv, const unsigned *index, const CellRanges &cells,

@@ -43,18 +43,27 @@ constexpr int kTileShift = 12;  // log2(kScanTile)
 constexpr unsigned kEmpty = 0xffffffffu;
 static_assert((1 << kTileShift) == kScanTile, "tile shift");
 
+// The fix-up lists this step's large cells afresh, and collide its crowded
+// groups (crowdCount: two counters, or none).
+__device__ __forceinline__ void resetLists(unsigned *largeCount, unsigned *crowdCount) {
+  *largeCount = 0u;
+  if (crowdCount) crowdCount[0] = crowdCount[1] = 0u;
+}
+
 // Exclusive prefix sums of the per-tile counts (one tile = kScanTile cells):
 // tileOff[t] = sum of tileCnt[0..t), tileOff[tiles] = the total; tileCnt is
 // cleared for the next step.  One CTA of 1024 threads, tiles in chunks.
 __global__ void __launch_bounds__(1024)
 kScanTiles(unsigned *__restrict__ tileCnt, unsigned *__restrict__ tileOff, unsigned tiles,
-           unsigned *__restrict__ largeCount) {
+           unsigned *__restrict__ largeCount, unsigned *__restrict__ crowdCount) {
+  chainTrigger();
+  chainWait();
   __shared__ unsigned sWarp[32];
   __shared__ unsigned sCarry;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) {
     sCarry = 0;
-    *largeCount = 0u;  // the fix-up lists this step's large cells afresh
+    resetLists(largeCount, crowdCount);
   }
   __syncthreads();
   for (unsigned base = 0; base < tiles; base += 1024) {
@@ -96,13 +105,17 @@ kScanTiles(unsigned *__restrict__ tileCnt, unsigned *__restrict__ tileOff, unsig
 // total, kAddTileBlocks adds the totals of the blocks before.
 constexpr unsigned kTileBlock = 1024;
 constexpr unsigned kTilesOneCta = 8192;  // up to this many tiles kScanTiles runs alone
+constexpr unsigned kTilesOwnPrefix = 4608;  // up to this many tiles kScanCells sums them itself
 
 __global__ void __launch_bounds__(kTileBlock)
 kScanTileBlocks(unsigned *__restrict__ tileCnt, unsigned *__restrict__ tileOff, unsigned tiles,
-                unsigned *__restrict__ blockSum, unsigned *__restrict__ largeCount) {
+                unsigned *__restrict__ blockSum, unsigned *__restrict__ largeCount,
+                unsigned *__restrict__ crowdCount) {
+  chainTrigger();
+  chainWait();
   __shared__ unsigned sWarp[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (blockIdx.x == 0 && tid == 0) *largeCount = 0u;
+  if (blockIdx.x == 0 && tid == 0) resetLists(largeCount, crowdCount);
   const unsigned t = blockIdx.x * kTileBlock + tid;
   const unsigned v = t < tiles ? tileCnt[t] : 0u;
   unsigned x = v;
@@ -132,11 +145,13 @@ kScanTileBlocks(unsigned *__restrict__ tileCnt, unsigned *__restrict__ tileOff, 
 
 __global__ void __launch_bounds__(kTileBlock)
 kAddTileBlocks(unsigned *__restrict__ tileOff, unsigned tiles,
-               const unsigned *__restrict__ blockSum) {
+               const unsigned *blockSum) {
+  chainTrigger();
+  chainWait();
   __shared__ unsigned sPart[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   unsigned part = 0;
-  for (unsigned b = tid; b < blockIdx.x; b += kTileBlock) part += __ldg(blockSum + b);
+  for (unsigned b = tid; b < blockIdx.x; b += kTileBlock) part += blockSum[b];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
   if (lane == 0) sPart[warp] = part;
@@ -146,7 +161,7 @@ kAddTileBlocks(unsigned *__restrict__ tileOff, unsigned tiles,
   const unsigned t = blockIdx.x * kTileBlock + tid;
   if (t < tiles) tileOff[t] += carry;
   if (blockIdx.x == gridDim.x - 1 && tid == 0)
-    tileOff[tiles] = carry + __ldg(blockSum + blockIdx.x);
+    tileOff[tiles] = carry + blockSum[blockIdx.x];
 }
 
 // off[c] = tileOff[tile] + exclusive prefix of cnt within the tile, cnt
@@ -158,15 +173,38 @@ kAddTileBlocks(unsigned *__restrict__ tileOff, unsigned tiles,
 // a pile -- is left as it is.
 // Round q of a tile covers cells q*1024 .. +1024, thread t the four at 4t
 // (16-byte accesses, coalesced).
+// kOwnPrefix: few tiles; each CTA sums the tile counts before its own itself
+// (tileOff is then tileCnt, cleared by the scatter), which saves the launch
+// of kScanTiles and its single CTA's latency (4 to 7 us per step).
+template <bool kOwnPrefix>
 __global__ void __launch_bounds__(kScanThreads)
 kScanCells(unsigned *__restrict__ cnt, unsigned *__restrict__ off, unsigned m,
-           const unsigned *__restrict__ tileOff, unsigned *__restrict__ tileOffPrev) {
+           const unsigned *tileOff, unsigned *__restrict__ tileOffPrev,
+           unsigned *__restrict__ largeCount, unsigned *__restrict__ crowdCount) {
   __shared__ unsigned sWarp[kScanThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned tile = blockIdx.x;
   constexpr int kRounds = kScanItems / 4;
   const size_t tbase = (size_t)tile * kScanTile;
-  const unsigned t0 = __ldg(tileOff + tile), t1 = __ldg(tileOff + tile + 1);
+  chainTrigger();
+  chainWait();
+  unsigned t0, t1;
+  if (kOwnPrefix) {
+    if (tile == 0 && tid == 0) resetLists(largeCount, crowdCount);
+    unsigned part = 0;
+    for (unsigned k = tid; k < tile; k += kScanThreads) part += tileOff[k];
+    part = __reduce_add_sync(0xffffffffu, part);
+    if (lane == 0) sWarp[warp] = part;
+    __syncthreads();
+    t0 = 0;
+#pragma unroll
+    for (int w = 0; w < kScanThreads / 32; ++w) t0 += sWarp[w];
+    t1 = t0 + tileOff[tile];
+    __syncthreads();  // sWarp is used again below
+  } else {
+    t0 = tileOff[tile];
+    t1 = tileOff[tile + 1];
+  }
   const unsigned prev = tileOffPrev[tile];  // read by every thread before thread 0 writes
   if (t0 == t1) {  // empty tile: every cell starts (and ends) at t0
     if (prev == t0) return;  // off already holds t0 in every cell of the tile
@@ -252,25 +290,29 @@ kScanCells(unsigned *__restrict__ cnt, unsigned *__restrict__ off, unsigned m,
 // step) holds the particle's new cell hash h and its count rank r; slot
 // off[h] + r receives the hash, the particle's index and the entry i.
 __global__ void __launch_bounds__(256)
-kScatterCells(const unsigned *__restrict__ hashN, const unsigned *__restrict__ rankN,
-              const unsigned *__restrict__ origOf, const unsigned *__restrict__ off,
+kScatterCells(const unsigned *hashN, const unsigned *rankN,
+              const unsigned *origOf, const unsigned *off,
               unsigned *__restrict__ slotKey, unsigned *__restrict__ slotOrig,
               unsigned *__restrict__ slotPrev, unsigned n, unsigned numCells,
-              unsigned *status) {
+              unsigned *__restrict__ tileCnt, unsigned tiles, unsigned *status) {
+  chainTrigger();
+  chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  // (tiles == 0 when kScanTiles has cleared the tile counts)
+  for (unsigned k = i; k < tiles; k += gridDim.x * blockDim.x) tileCnt[k] = 0u;
   if (i >= n) return;
-  unsigned h = __ldg(hashN + i);
+  unsigned h = hashN[i];
   if (h >= numCells) {
     atomicOr(status, (unsigned)kStatusKeyRange);
     return;
   }
-  unsigned s = __ldg(off + h) + __ldg(rankN + i);
+  unsigned s = off[h] + rankN[i];
   if (s >= n) {
     atomicOr(status, (unsigned)kStatusKeyRange);
     return;
   }
   slotKey[s] = h;
-  slotOrig[s] = origOf ? __ldg(origOf + i) : i;
+  slotOrig[s] = origOf ? origOf[i] : i;
   slotPrev[s] = i;
 }
 
@@ -288,20 +330,22 @@ inline unsigned largeCapacity(unsigned n) { return n / (kFixupMaxCell + 1) + 1; 
 // above kFixupMaxCell members is appended to large[1..] (large[0] counts) by
 // its first slot and left to kFixupLarge.
 __global__ void __launch_bounds__(256)
-kFixupGather(const unsigned *__restrict__ slotKey, const unsigned *__restrict__ slotOrig,
-             const unsigned *__restrict__ slotPrev, const unsigned *__restrict__ off,
+kFixupGather(const unsigned *slotKey, const unsigned *slotOrig,
+             const unsigned *slotPrev, const unsigned *off,
              unsigned *__restrict__ hashOut, unsigned *__restrict__ indexOut,
              float4 *__restrict__ sortedPos, float4 *__restrict__ sortedVel,
-             const float4 *__restrict__ prevPos, const float4 *__restrict__ prevVel,
+             const float4 *prevPos, const float4 *prevVel,
              unsigned n, unsigned numCells, unsigned *__restrict__ large, unsigned largeCap,
              unsigned *status) {
+  chainTrigger();
+  chainWait();
   unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
-  const unsigned h = __ldg(slotKey + s);
-  const unsigned me = __ldg(slotOrig + s);
-  const unsigned prev = __ldg(slotPrev + s);
+  const unsigned h = slotKey[s];
+  const unsigned me = slotOrig[s];
+  const unsigned prev = slotPrev[s];
   if (h >= numCells || me >= n || prev >= n) return;  // unfilled slot (reported)
-  const unsigned a = __ldg(off + h), b = __ldg(off + h + 1);
+  const unsigned a = off[h], b = off[h + 1];
   if (b - a > kFixupMaxCell) {
     if (s == a) {
       const unsigned k = atomicAdd(large, 1u);
@@ -313,13 +357,13 @@ kFixupGather(const unsigned *__restrict__ slotKey, const unsigned *__restrict__ 
     return;
   }
   unsigned r = 0;
-  for (unsigned t = a; t < b; ++t) r += __ldg(slotOrig + t) < me ? 1u : 0u;
+  for (unsigned t = a; t < b; ++t) r += slotOrig[t] < me ? 1u : 0u;
   const unsigned dst = a + r;
   if (dst >= n) return;
   hashOut[dst] = h;
   indexOut[dst] = me;
-  sortedPos[dst] = ldg4(prevPos + prev);
-  sortedVel[dst] = ldg4(prevVel + prev);
+  sortedPos[dst] = prevPos[prev];
+  sortedVel[dst] = prevVel[prev];
 }
 
 constexpr int kLargeThreads = 1024;
@@ -466,11 +510,13 @@ __device__ void largeRadixPass(const unsigned long long *src, unsigned long long
 // then the word prefix), or nullptr for the sort only.
 __global__ void __launch_bounds__(kLargeThreads)
 kFixupLarge(unsigned *__restrict__ slotOrig, unsigned *__restrict__ slotPrev,
-            const unsigned *__restrict__ off, const unsigned *__restrict__ large,
+            const unsigned *off, const unsigned *large,
             unsigned largeCap, unsigned *__restrict__ hashOut, unsigned *__restrict__ indexOut,
             float4 *__restrict__ sortedPos, float4 *__restrict__ sortedVel,
-            const float4 *__restrict__ prevPos, const float4 *__restrict__ prevVel, unsigned n,
+            const float4 *prevPos, const float4 *prevVel, unsigned n,
             int idBits, unsigned *__restrict__ bitmaps) {
+  chainTrigger();
+  chainWait();
   __shared__ LargeSmem sm;
   const unsigned count = min(large[0], largeCap);
   const int tid = threadIdx.x;
@@ -517,8 +563,8 @@ kFixupLarge(unsigned *__restrict__ slotOrig, unsigned *__restrict__ slotPrev,
           const unsigned dst = a + pre[wd] + __popc(bits[wd] & ((1u << (me & 31u)) - 1u));
           hashOut[dst] = h;
           indexOut[dst] = me;
-          sortedPos[dst] = ldg4(prevPos + prev);
-          sortedVel[dst] = ldg4(prevVel + prev);
+          sortedPos[dst] = prevPos[prev];
+          sortedVel[dst] = prevVel[prev];
         }
         __syncthreads();  // the bitmap is reused by the next cell
         continue;
@@ -546,8 +592,8 @@ kFixupLarge(unsigned *__restrict__ slotOrig, unsigned *__restrict__ slotPrev,
       if (me >= n || prev >= n) continue;  // unfilled slot (reported by the scatter)
       hashOut[a + t] = h;
       indexOut[a + t] = me;
-      sortedPos[a + t] = ldg4(prevPos + prev);
-      sortedVel[a + t] = ldg4(prevVel + prev);
+      sortedPos[a + t] = prevPos[prev];
+      sortedVel[a + t] = prevVel[prev];
     }
     __syncthreads();
   }
@@ -556,11 +602,13 @@ kFixupLarge(unsigned *__restrict__ slotOrig, unsigned *__restrict__ slotPrev,
 // cellStart/cellEnd from the prefix table (cellEnd of empty cells untouched,
 // as the reference leaves it).
 __global__ void __launch_bounds__(256)
-kCellTables(const unsigned *__restrict__ off, unsigned *__restrict__ cellStart,
+kCellTables(const unsigned *off, unsigned *__restrict__ cellStart,
             unsigned *__restrict__ cellEnd, unsigned numCells) {
+  chainTrigger();
+  chainWait();
   size_t stride = (size_t)gridDim.x * blockDim.x;
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < numCells; c += stride) {
-    unsigned a = __ldg(off + c), b = __ldg(off + c + 1);
+    unsigned a = off[c], b = off[c + 1];
     if (a < b) {
       cellStart[c] = a;
       cellEnd[c] = b;
@@ -570,12 +618,16 @@ kCellTables(const unsigned *__restrict__ off, unsigned *__restrict__ cellStart,
   }
 }
 
-// First step of fcdemUpdate: integrate + calcHash + count (the tile counts
-// follow in kTileReduce).
+// First step of fcdemUpdate: integrate + calcHash + count.  kTiles: the tile
+// counts too; otherwise they follow in kTileReduce.
+template <bool kTiles>
 __global__ void __launch_bounds__(256)
 kIntegrateHashCount(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt,
                     unsigned *__restrict__ hash, unsigned *__restrict__ rank,
-                    unsigned *__restrict__ cnt, unsigned n, KParams kp) {
+                    unsigned *__restrict__ cnt, unsigned *__restrict__ tileCnt, unsigned n,
+                    KParams kp) {
+  chainTrigger();
+  chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float4 p4 = pos[i], v4 = vel[i];
@@ -588,13 +640,16 @@ kIntegrateHashCount(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt
   unsigned h = gridHash(g.x, g.y, g.z, kp.p);
   hash[i] = h;
   rank[i] = atomicAdd(cnt + h, 1u);
+  if (kTiles) countTile(tileCnt, h >> kTileShift);
 }
 
 // tileCnt[t] = sum of cnt over tile t (after kIntegrateHashCount, whose
 // particle-order cells are scattered over the tiles: summing the counts once
 // is cheaper than one atomic per particle on the few tile counters).
 __global__ void __launch_bounds__(kScanThreads)
-kTileReduce(const unsigned *__restrict__ cnt, unsigned *__restrict__ tileCnt, unsigned m) {
+kTileReduce(const unsigned *cnt, unsigned *__restrict__ tileCnt, unsigned m) {
+  chainTrigger();
+  chainWait();
   __shared__ unsigned sWarp[kScanThreads / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const size_t tbase = (size_t)blockIdx.x * kScanTile;
@@ -631,6 +686,8 @@ kBatchIntegrateHashCount(const BatchScene *__restrict__ scenes,
                          const unsigned *__restrict__ sceneOf, float4 *__restrict__ pos,
                          float4 *__restrict__ vel, float dt, unsigned *__restrict__ hash,
                          unsigned *__restrict__ rank, unsigned *__restrict__ cnt, unsigned n) {
+  chainTrigger();
+  chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const BatchScene &S = scenes[__ldg(sceneOf + i)];
@@ -714,68 +771,80 @@ bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsi
   return true;
 }
 
+// Up to this many particles the first step counts its tiles with atomics
+// (one per distinct tile of a warp) instead of a pass over all cells: the
+// pass is a launch (3 us), the atomics cost more only once many particles in
+// random order queue on the tile counters.
+constexpr unsigned kTileAtomicsMax = 1u << 17;
+
 bool countPipelineBegin(Context &c, float4 *pos, float4 *vel, float dt, unsigned *hash,
                         unsigned n, unsigned numCells, const KParams &kp, CountBuffers &b) {
   if (!countBuffers(c, n, numCells, b)) return false;
-  kIntegrateHashCount<<<(n + 255) / 256, 256, 0, curStream()>>>(pos, vel, dt, hash, b.rank,
-                                                                b.cnt, n, kp);
+  const bool tiles = n <= kTileAtomicsMax;
+  launchChained(false, tiles ? kIntegrateHashCount<true> : kIntegrateHashCount<false>,
+                (n + 255) / 256, 256, 0, pos, vel, dt, hash, b.rank, b.cnt, b.tileCnt, n, kp);
   if (!launchOk()) return false;
-  kTileReduce<<<b.scanTiles, kScanThreads, 0, curStream()>>>(b.cnt, b.tileCnt, numCells + 1);
+  if (tiles) return true;
+  launchChained(true, kTileReduce, b.scanTiles, kScanThreads, 0, b.cnt, b.tileCnt, numCells + 1);
   return launchOk();
 }
 
 bool countPipelineBeginBatch(const BatchScene *scenes, const unsigned *sceneOf, bool radiusFromW,
                              float4 *pos, float4 *vel, float dt, unsigned *hash, unsigned n,
                              unsigned numCells, const CountBuffers &b) {
-  if (radiusFromW)
-    kBatchIntegrateHashCount<true><<<(n + 255) / 256, 256, 0, curStream()>>>(
-        scenes, sceneOf, pos, vel, dt, hash, b.rank, b.cnt, n);
-  else
-    kBatchIntegrateHashCount<false><<<(n + 255) / 256, 256, 0, curStream()>>>(
-        scenes, sceneOf, pos, vel, dt, hash, b.rank, b.cnt, n);
+  launchChained(false, radiusFromW ? kBatchIntegrateHashCount<true> : kBatchIntegrateHashCount<false>,
+                (n + 255) / 256, 256, 0, scenes, sceneOf, pos, vel, dt, hash, b.rank, b.cnt, n);
   if (!launchOk()) return false;
-  kTileReduce<<<b.scanTiles, kScanThreads, 0, curStream()>>>(b.cnt, b.tileCnt, numCells + 1);
+  launchChained(true, kTileReduce, b.scanTiles, kScanThreads, 0, b.cnt, b.tileCnt, numCells + 1);
   return launchOk();
 }
 
 // scan + scatter + fix-up/gather for one step (the counts are in place).
 // hashN/rankN/origOf/prevPos/prevVel are indexed by the previous order's
 // entries (origOf == nullptr: entry i is particle i, the first step).
+// crowdCount (optional): collide's two group counters, cleared on the way.
 bool countPipelineSort(Context &c, const CountBuffers &b, const unsigned *origOf,
                        const float4 *prevPos, const float4 *prevVel, unsigned *hash,
                        unsigned *index, float4 *sortedPos, float4 *sortedVel, unsigned n,
-                       unsigned numCells) {
-  cudaStream_t st = curStream();
+                       unsigned numCells, unsigned *crowdCount) {
   const unsigned m = numCells + 1;
-  if (b.scanTiles <= kTilesOneCta) {
-    kScanTiles<<<1, 1024, 0, st>>>(b.tileCnt, b.tileOff, b.scanTiles, b.large);
+  const bool own = b.scanTiles <= kTilesOwnPrefix;
+  if (own) {
+    launchChained(true, kScanCells<true>, b.scanTiles, kScanThreads, 0, b.cnt, b.off, m, b.tileCnt,
+                  b.tileOffPrev, b.large, crowdCount);
     if (!launchOk()) return false;
   } else {
-    const unsigned blocks = (b.scanTiles + kTileBlock - 1) / kTileBlock;
-    kScanTileBlocks<<<blocks, kTileBlock, 0, st>>>(b.tileCnt, b.tileOff, b.scanTiles,
-                                                   b.tileBlockSum, b.large);
-    if (!launchOk()) return false;
-    kAddTileBlocks<<<blocks, kTileBlock, 0, st>>>(b.tileOff, b.scanTiles, b.tileBlockSum);
+    if (b.scanTiles <= kTilesOneCta) {
+      launchChained(true, kScanTiles, 1, 1024, 0, b.tileCnt, b.tileOff, b.scanTiles, b.large,
+                    crowdCount);
+      if (!launchOk()) return false;
+    } else {
+      const unsigned blocks = (b.scanTiles + kTileBlock - 1) / kTileBlock;
+      launchChained(true, kScanTileBlocks, blocks, kTileBlock, 0, b.tileCnt, b.tileOff, b.scanTiles,
+                    b.tileBlockSum, b.large, crowdCount);
+      if (!launchOk()) return false;
+      launchChained(true, kAddTileBlocks, blocks, kTileBlock, 0, b.tileOff, b.scanTiles,
+                    b.tileBlockSum);
+      if (!launchOk()) return false;
+    }
+    launchChained(true, kScanCells<false>, b.scanTiles, kScanThreads, 0, b.cnt, b.off, m, b.tileOff,
+                  b.tileOffPrev, b.large, crowdCount);
     if (!launchOk()) return false;
   }
-  kScanCells<<<b.scanTiles, kScanThreads, 0, st>>>(b.cnt, b.off, m, b.tileOff,
-                                                    b.tileOffPrev);
-  if (!launchOk()) return false;
   // hash holds the new hashes in entry order until the fix-up overwrites it
-  kScatterCells<<<(n + 255) / 256, 256, 0, st>>>(hash, b.rank, origOf, b.off, b.slotKey,
-                                                  b.slotIdx, b.slotPrev, n, numCells,
-                                                  c.dStatus);
+  launchChained(true, kScatterCells, (n + 255) / 256, 256, 0, hash, b.rank, origOf, b.off, b.slotKey,
+                b.slotIdx, b.slotPrev, n, numCells, b.tileCnt, own ? b.scanTiles : 0u, c.dStatus);
   if (!launchOk()) return false;
-  kFixupGather<<<(n + 255) / 256, 256, 0, st>>>(b.slotKey, b.slotIdx, b.slotPrev, b.off, hash,
-                                                 index, sortedPos, sortedVel, prevPos, prevVel,
-                                                 n, numCells, b.large, b.largeCap, c.dStatus);
+  launchChained(true, kFixupGather, (n + 255) / 256, 256, 0, b.slotKey, b.slotIdx, b.slotPrev, b.off,
+                hash, index, sortedPos, sortedVel, prevPos, prevVel, n, numCells, b.large,
+                b.largeCap, c.dStatus);
   if (!launchOk()) return false;
+  if (n <= kFixupMaxCell) return true;  // no cell can be large
   // Returns at once when the fix-up listed no cell (the common case).
   const unsigned largeCtas = b.largeCap < numSms() ? b.largeCap : numSms();  // one per SM at most
-  kFixupLarge<<<largeCtas, kLargeThreads, 0, st>>>(b.slotIdx, b.slotPrev, b.off, b.large,
-                                                   b.largeCap, hash, index, sortedPos,
-                                                   sortedVel, prevPos, prevVel, n, keyBits(n),
-                                                   b.bitmaps);
+  launchChained(true, kFixupLarge, largeCtas, kLargeThreads, 0, b.slotIdx, b.slotPrev, b.off,
+                b.large, b.largeCap, hash, index, sortedPos, sortedVel, prevPos, prevVel, n,
+                keyBits(n), b.bitmaps);
   return launchOk();
 }
 
@@ -783,7 +852,7 @@ bool countPipelineTables(const CountBuffers &b, unsigned *cellStart, unsigned *c
                          unsigned numCells) {
   unsigned blocks = (numCells + 255) / 256;
   if (blocks > numSms() * 16u) blocks = numSms() * 16u;
-  kCellTables<<<blocks, 256, 0, curStream()>>>(b.off, cellStart, cellEnd, numCells);
+  launchChained(true, kCellTables, blocks, 256, 0, b.off, cellStart, cellEnd, numCells);
   return launchOk();
 }
 

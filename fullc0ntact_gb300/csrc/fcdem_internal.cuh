@@ -93,7 +93,10 @@ bool launchOk();
 // when the kernels before it are complete and their writes visible, and only
 // then reads or writes what others touch: a kernel's completion thus still
 // implies that of all before it.  Before chainWait() it may read what was
-// complete before the last launch that was not chained.  The first launch of
+// complete before the last launch that was not chained.  What earlier kernels
+// wrote is read with plain loads: a __ldg or a const __restrict__ parameter
+// tells the compiler that the value never changes, and it may then load it
+// before chainWait().  The first launch of
 // a call is not chained (its inputs come from the caller's work); launched
 // that way the two calls do nothing.
 __device__ __forceinline__ void chainTrigger() {
@@ -192,6 +195,11 @@ void launchCollide(int mode, bool collider, float4 *newVel, const float4 *sp,
                    const float4 *sv, const unsigned *index, const CellRanges &cells,
                    unsigned n, const KParams &kp, const CollideOut &out);
 
+// collide's counters of crowded groups for n particles, for whoever clears
+// them before launchCollide on the prefix table (countPipelineSort does);
+// nullptr when the crowded path is off.
+unsigned *collideCrowdCount(unsigned n);
+
 // One scene of a batch (fcdem_batch.cu), on the device.
 struct BatchScene {
   SimParams p;
@@ -233,7 +241,7 @@ bool countPipelineBeginBatch(const BatchScene *scenes, const unsigned *sceneOf, 
 bool countPipelineSort(Context &c, const CountBuffers &b, const unsigned *origOf,
                        const float4 *prevPos, const float4 *prevVel, unsigned *hash,
                        unsigned *index, float4 *sortedPos, float4 *sortedVel, unsigned n,
-                       unsigned numCells);
+                       unsigned numCells, unsigned *crowdCount);
 bool countPipelineTables(const CountBuffers &b, unsigned *cellStart, unsigned *cellEnd,
                          unsigned numCells);
 

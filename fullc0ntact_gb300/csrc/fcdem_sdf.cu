@@ -70,7 +70,7 @@ SdfLayout makeLayout(int D, int H, int L) {
 // What the kernels read of a network.
 struct SdfView {
   SdfLayout lay;
-  const float *__restrict__ p;   // parameters
+  const float *p;                // parameters
   const __nv_bfloat16 *__restrict__ w16;  // hidden layers 1..L-1, tensor-core tiles
   float shift[3], scale[3], outScale;
 };
@@ -209,15 +209,15 @@ kSdfTrain(SdfView net, const float4 *__restrict__ samples, const int *__restrict
     const float4 *src = reinterpret_cast<const float4 *>(net.p + ly.wh[l - 1]);
 #pragma unroll 4
     for (int e = t; e < H * Q; e += T)
-      *reinterpret_cast<float4 *>(&sm.w[l - 1][e / Q][4 * (e % Q)]) = __ldg(src + e);
+      *reinterpret_cast<float4 *>(&sm.w[l - 1][e / Q][4 * (e % Q)]) = src[e];
   }
-  for (int e = t; e < H * D; e += T) sm.w0[e % D][e / D] = __ldg(net.p + ly.w0 + e);
+  for (int e = t; e < H * D; e += T) sm.w0[e % D][e / D] = net.p[ly.w0 + e];
   if (t < H) {
-    sm.b[0][t] = __ldg(net.p + ly.b0 + t);
-    for (int l = 1; l < L; ++l) sm.b[l][t] = __ldg(net.p + ly.bh[l - 1] + t);
-    sm.wo[t] = __ldg(net.p + ly.wo + t);
+    sm.b[0][t] = net.p[ly.b0 + t];
+    for (int l = 1; l < L; ++l) sm.b[l][t] = net.p[ly.bh[l - 1] + t];
+    sm.wo[t] = net.p[ly.wo + t];
   }
-  const float bo = __ldg(net.p + ly.bo);
+  const float bo = net.p[ly.bo];
   // gradient sums over the CTA's tiles
   float gW[L - 1][kBlocks][4][4] = {}, gW0[4] = {}, gB[L] = {}, gWo = 0.0f, gBo = 0.0f;
   for (unsigned tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -394,7 +394,7 @@ kSdfTrain(SdfView net, const float4 *__restrict__ samples, const int *__restrict
 constexpr int kReduceWarps = 8;
 template <bool kAdam>
 __global__ void __launch_bounds__(32 * kReduceWarps)
-kSdfReduce(const float *__restrict__ partial, unsigned parts, unsigned total, float *__restrict__ p,
+kSdfReduce(const float *partial, unsigned parts, unsigned total, float *__restrict__ p,
            float *__restrict__ grad, float *__restrict__ m, float *__restrict__ v,
            float lr, float b1, float b2, float eps, float c1, float c2) {
   __shared__ float sSum[kReduceWarps][32];
@@ -411,7 +411,7 @@ kSdfReduce(const float *__restrict__ partial, unsigned parts, unsigned total, fl
   if (i < total) {
 #pragma unroll 8
     for (unsigned r = warp; r < parts; r += kReduceWarps)
-      acc += __ldg(partial + (size_t)r * partialRow(total) + i);
+      acc += partial[(size_t)r * partialRow(total) + i];
   }
   sSum[warp][lane] = acc;
   __syncthreads();

@@ -284,6 +284,7 @@ void fcdemUpdate(float *pos, float *vel, float *sortedPos, float *sortedVel,
     // starts from particle order; the last collide writes vel and pos back in
     // particle order, and the cell tables are written once at the end.
     CountBuffers b;
+    unsigned *crowd = collideCrowdCount(n);
     stageBegin(0);
     bool ok = countPipelineBegin(c, (float4 *)pos, (float4 *)vel, deltaTime, hash, n,
                                  numCells, kp, b);
@@ -292,7 +293,7 @@ void fcdemUpdate(float *pos, float *vel, float *sortedPos, float *sortedVel,
       stageBegin(1);
       ok = countPipelineSort(c, b, s == 0 ? nullptr : index, (const float4 *)pos,
                              (const float4 *)vel, hash, index, (float4 *)sortedPos,
-                             (float4 *)sortedVel, n, numCells);
+                             (float4 *)sortedVel, n, numCells, crowd);
       stageEnd(1);
       if (!ok) break;
       const bool last = (s + 1 == steps);
@@ -376,13 +377,14 @@ void fcdemUM_update(float *pos, float *vel, float *force, float *sortedPos, floa
   CountBuffers b;
   if (!countBuffersIn(c.countBuf, c.countBytes, c.countCells, n, numCells, b)) return;
   const UmCount count{hash, b.rank, b.cnt, b.tileCnt};
+  unsigned *crowd = collideCrowdCount(n);
   stageBegin(0);
   bool ok = umHashCount((const float4 *)pos, n, kp, count);
   stageEnd(0);
   for (uint s = 0; ok && s < steps; ++s) {
     stageBegin(1);
     ok = countPipelineSort(c, b, nullptr, (const float4 *)pos, (const float4 *)vel, hash, index,
-                           (float4 *)sortedPos, (float4 *)sortedVel, n, numCells);
+                           (float4 *)sortedPos, (float4 *)sortedVel, n, numCells, crowd);
     stageEnd(1);
     if (!ok) break;
     CellRanges cells;
