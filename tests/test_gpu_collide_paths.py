@@ -264,23 +264,26 @@ def test_collide_autotuner_keeps_the_state_and_the_results():
         np.testing.assert_array_equal(x.view(np.uint32), y.view(np.uint32))
 
 
-def _rows_scene(grid, n, poly, kind, seed):
+def _rows_scene(grid, n, poly, kind, many, seed):
     """Scenes at the edges of the row scan: `rows` puts n particles into one
     column of cells (rows of n candidates), `full` spreads them over the whole
-    grid and past it, so that the first and last columns wrap."""
+    grid and past it, so that the first and last columns wrap.  many: 25,000
+    more over the whole grid, above the size up to which nine lanes share a
+    particle."""
     from fullc0ntact_gb300 import scenes
     radius = 1.0 / 64.0
-    sc = scenes.random_box(n, grid=grid, radius=radius, seed=seed, cell=1.0 / 32.0, poly=poly)
+    total = n + 25000 if many else n
+    sc = scenes.random_box(total, grid=grid, radius=radius, seed=seed, cell=1.0 / 32.0, poly=poly)
     rng = np.random.default_rng(seed + 1)
+    ext = np.array(grid) / 32.0
+    sc["pos"][:, :3] = np.clip(-1.0 + rng.uniform(-0.02, 1.02, (total, 3)) * ext, -0.98, 0.98)
     if kind == "rows":
-        sc["pos"][:, 0] = rng.uniform(-0.5, -0.5 + 3.0 / 32.0, n)
-        sc["pos"][:, 1:3] = rng.uniform(-0.5, -0.5 + 1.0 / 32.0, (n, 2))
-    else:
-        ext = np.array(grid) / 32.0
-        sc["pos"][:, :3] = np.clip(-1.0 + rng.uniform(-0.02, 1.02, (n, 3)) * ext, -0.98, 0.98)
+        sc["pos"][:n, 0] = rng.uniform(-0.5, -0.5 + 3.0 / 32.0, n)
+        sc["pos"][:n, 1:3] = rng.uniform(-0.5, -0.5 + 1.0 / 32.0, (n, 2))
     return sc
 
 
+@pytest.mark.parametrize("many", [False, True])
 @pytest.mark.parametrize("poly", [False, True])
 @pytest.mark.parametrize("grid,n,kind", [
     ((64, 64, 64), 1, "rows"), ((64, 64, 64), 3, "rows"), ((64, 64, 64), 4, "rows"),
@@ -288,13 +291,14 @@ def _rows_scene(grid, n, poly, kind, seed):
     ((64, 64, 64), 129, "rows"), ((64, 64, 64), 255, "rows"), ((64, 64, 64), 256, "rows"),
     ((64, 64, 64), 700, "rows"), ((4, 4, 4), 300, "full"), ((4, 8, 16), 700, "full"),
     ((8, 2, 4), 200, "full"), ((2, 8, 8), 300, "full"), ((16, 16, 16), 4001, "full")])
-def test_row_scan_edges_match_oracle(grid, n, kind, poly):
-    """The hit-mask scan and the general loop on rows of 0 to 700 candidates,
-    wrapped columns and aliased axes: bit-exact against the oracle, staged
-    (cellStart/cellEnd) and fused (prefix table)."""
+def test_row_scan_edges_match_oracle(grid, n, kind, poly, many):
+    """One thread per particle (the hit-mask scan and the general loop) and nine
+    lanes per particle, on rows of 0 to 700 candidates, wrapped columns and
+    aliased axes: bit-exact against the oracle, staged (cellStart/cellEnd) and
+    fused (prefix table), with and without the crowded path."""
     from fullc0ntact_gb300 import dem
     from oracle import oracle as O
-    sc = _rows_scene(grid, n, poly, kind, 100 + n)
+    sc = _rows_scene(grid, n, poly, kind, many, 100 + n)
     P = O.SimParams.from_buffer_copy(bytes(sc["params"]))
     with O.gpu_arithmetic():
         pos, vel = sc["pos"].copy(), sc["vel"].copy()
