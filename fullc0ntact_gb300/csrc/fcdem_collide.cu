@@ -268,27 +268,6 @@ __device__ __forceinline__ float3 neighbourForceGlobal(
 // ---------------------------------------------------------------------------
 // The per-particle scan with hit masks.
 
-// Packed pairs of floats (one instruction for two lanes' worth of FP32).
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 // The near test of one particle against candidates, conservative: a pair that
 // passes `sqrtf(d2) < cd` is always near.  With e = 2^-24 and s = 1 + 16 e,
 //   c = w s + r_i s >= cd (1 + 13 e)   (three roundings off 16 e),

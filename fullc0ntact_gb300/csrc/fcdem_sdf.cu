@@ -81,15 +81,19 @@ __device__ __forceinline__ float silu(float z) { return z * sigm(z); }
 // tanh approximation (one special-function op; relative error about 2^-11,
 // near the bf16 rounding of the activations it feeds).  The culling
 // threshold is calibrated on this arithmetic (the prediction the kernels
-// make), so its error is part of what the exact map judges.
+// make), so its error is part of what the exact map judges.  The kernels hold
+// every weight and bias of a SiLU layer halved -- an exact scaling, all sums
+// round as before -- so their layers give h itself.
 __device__ __forceinline__ float tanhApprox(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float siluFast(float z) {
-  const float h = 0.5f * z;
-  return fmaf(h, tanhApprox(h), h);
+// silu of two halved arguments
+__device__ __forceinline__ f32x2 siluHalf2(f32x2 h) {
+  float a, b;
+  unpack2(h, a, b);
+  return fma2(h, pack2(tanhApprox(a), tanhApprox(b)), h);
 }
 __device__ __forceinline__ float dsilu(float z) {
   const float s = sigm(z);
@@ -545,13 +549,13 @@ struct SdfTileSmem {
   static_assert(L >= 2 && L <= 3, "hidden layers");
   static_assert(T == 1 || T == 2, "tiles per CTA");
   __nv_bfloat16 a[T * 128 * H];        // activation tiles (A operands), 128 points each
-  __nv_bfloat16 w[(L - 1) * H * H];    // hidden-layer weights (B operands)
-  float w0[H * kSdfMaxInputs];         // first layer, [H][D]
-  float b[L * H];                      // biases of the hidden layers
+  __nv_bfloat16 w[(L - 1) * H * H];    // hidden-layer weights (B operands), halved
+  float w0[kSdfMaxInputs][H];          // first layer, [D][H], halved
+  float b[L * H];                      // biases of the hidden layers, halved
   float wo[H];
   float bo;
   unsigned tmem;
-  unsigned long long bar;
+  unsigned long long bar[T];           // one per tile
 };
 
 // Per-CTA set-up of the tile forward: TMEM columns (H per tile), the
@@ -564,17 +568,18 @@ __device__ __forceinline__ void sdfTileSetup(SdfTileSmem<H, L, T> &sm, const Sdf
     tmemRelinquish();
   }
   if (t == 0) {
-    mbarInit1(smemU32(&sm.bar));
+    for (int k = 0; k < T; ++k) mbarInit1(smemU32(&sm.bar[k]));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   const uint4 *src = reinterpret_cast<const uint4 *>(net.w16);
   uint4 *dst = reinterpret_cast<uint4 *>(sm.w);
   for (int e = t; e < (L - 1) * H * H / 8; e += blockDim.x) dst[e] = __ldg(src + e);
   const SdfLayout &ly = net.lay;
-  for (int e = t; e < H * ly.D; e += blockDim.x) sm.w0[e] = __ldg(net.p + ly.w0 + e);
+  for (int e = t; e < H * ly.D; e += blockDim.x)
+    sm.w0[e % ly.D][e / ly.D] = 0.5f * __ldg(net.p + ly.w0 + e);
   for (int e = t; e < H; e += blockDim.x) {
-    sm.b[e] = __ldg(net.p + ly.b0 + e);
-    for (int l = 1; l < L; ++l) sm.b[l * H + e] = __ldg(net.p + ly.bh[l - 1] + e);
+    sm.b[e] = 0.5f * __ldg(net.p + ly.b0 + e);
+    for (int l = 1; l < L; ++l) sm.b[l * H + e] = 0.5f * __ldg(net.p + ly.bh[l - 1] + e);
     sm.wo[e] = __ldg(net.p + ly.wo + e);
   }
   if (t == 0) sm.bo = __ldg(net.p + ly.bo);
@@ -594,14 +599,53 @@ __device__ __forceinline__ void sdfTileTeardown(SdfTileSmem<H, L, T> &sm) {
   }
 }
 
+// Barrier of one tile's 128 threads, and the same with an OR over them.  (The
+// barrier's number is an immediate: a register would reserve all 16.)
+template <int T>
+__device__ __forceinline__ void tileSync(int tile) {
+  if (T == 1)
+    __syncthreads();
+  else if (tile == 0)
+    asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+  else
+    asm volatile("barrier.cta.sync 2, 128;" ::: "memory");
+}
+template <int kId>
+__device__ __forceinline__ bool barrierOr(bool v) {
+  unsigned r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.or.pred q, %2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((unsigned)v), "n"(kId)
+      : "memory");
+  return r != 0u;
+}
+template <int T>
+__device__ __forceinline__ bool tileSyncOr(int tile, bool v) {
+  if (T == 1) return __syncthreads_or(v);
+  return tile == 0 ? barrierOr<1>(v) : barrierOr<2>(v);
+}
+
 // The distance prediction for this thread's point (x normalised, shape code
-// `shape` or -1); 128 * T threads, one point each, all threads of the CTA.
+// `shape` or -1); 128 * T threads, one point each, all threads of a tile.
 // Thread t works on tile t / 128, row t % 128: the tile's A operand is its
 // own 128-row block of sm.a and its accumulator TMEM columns tile * H ..,
-// read by the warp's lane quarter (warp % 4).  Every tile's chain uses the
-// same B operands and one commit.  `phase` is the barrier parity, flipped
-// per layer.  Returns false (for every thread) when an MMA chain did not
-// complete in time.
+// read by the warp's lane quarter (warp % 4).  The tiles of a CTA share the
+// weights only; each has its barrier, MMA chain and commit, so that one's
+// products overlap with another's activations.  `phase` is the tile's mbarrier
+// parity, flipped per layer.  Returns false (for every thread of the tile)
+// when an MMA chain did not complete in time.
+//
+// Bound by the special-function unit: a tanh.approx keeps it for 15 cycles per
+// warp (measured: 192 of them per point of 3-64-64-64-1, 77% active over the
+// kernel's 91 us per 1M points, so 70 us at best).  Everything else is kept out
+// of its way: biases, the SiLU's multiply-add and the output product work on
+// packed pairs, weights are halved once instead of every argument, the first
+// layer's weights lie [input][output] for 16-byte loads: 112 us per call
+// against 120 (43% issue active).
 template <int H, int L, int kLdBatch = 1, int T = 1>
 __device__ __forceinline__ bool sdfTileForward(SdfTileSmem<H, L, T> &sm, const SdfView &net,
                                                float x0, float x1, float x2, int shape,
@@ -609,53 +653,60 @@ __device__ __forceinline__ bool sdfTileForward(SdfTileSmem<H, L, T> &sm, const S
   const int t = threadIdx.x, warp = t >> 5;
   const int tile = t >> 7, row = t & 127, quarter = warp & 3;
   __nv_bfloat16 *aTile = sm.a + tile * 128 * H;
-  const int D = net.lay.D;
+  const unsigned bar = smemU32(&sm.bar[tile]);
+  const bool coded = shape >= 0 && 3 + shape < net.lay.D;
+  // four consecutive floats of shared memory as two pairs
+  auto four = [](const float *p) { return *reinterpret_cast<const ulonglong2 *>(p); };
+  auto packed = [](f32x2 v) {
+    float a, b;
+    unpack2(v, a, b);
+    return packBf16(a, b);
+  };
   // first layer on the CUDA cores, 8 outputs per 16-byte chunk of the A row
+  const f32x2 xx0 = pack2(x0, x0), xx1 = pack2(x1, x1), xx2 = pack2(x2, x2);
 #pragma unroll 1
   for (int c = 0; c < H / 8; ++c) {
-    float h[8];
+    unsigned v[4];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int j = c * 8 + u;
-      const float *w = sm.w0 + j * D;
-      float z = sm.b[j];
-      z = fmaf(w[0], x0, z);
-      z = fmaf(w[1], x1, z);
-      z = fmaf(w[2], x2, z);
-      if (shape >= 0 && 3 + shape < D) z += w[3 + shape];
-      h[u] = siluFast(z);
+    for (int u = 0; u < 2; ++u) {
+      const int j = c * 8 + u * 4;
+      ulonglong2 z = four(sm.b + j);
+      const ulonglong2 w0 = four(&sm.w0[0][j]), w1 = four(&sm.w0[1][j]), w2 = four(&sm.w0[2][j]);
+      z.x = fma2(w2.x, xx2, fma2(w1.x, xx1, fma2(w0.x, xx0, z.x)));
+      z.y = fma2(w2.y, xx2, fma2(w1.y, xx1, fma2(w0.y, xx0, z.y)));
+      if (coded) {
+        const ulonglong2 ws = four(&sm.w0[3 + shape][j]);
+        z.x = add2(z.x, ws.x);
+        z.y = add2(z.y, ws.y);
+      }
+      v[2 * u] = packed(siluHalf2(z.x));
+      v[2 * u + 1] = packed(siluHalf2(z.y));
     }
-    uint4 v = make_uint4(packBf16(h[0], h[1]), packBf16(h[2], h[3]), packBf16(h[4], h[5]),
-                         packBf16(h[6], h[7]));
-    *reinterpret_cast<uint4 *>(aTile + tileOffset(row, c * 8, 128)) = v;
+    *reinterpret_cast<uint4 *>(aTile + tileOffset(row, c * 8, 128)) =
+        make_uint4(v[0], v[1], v[2], v[3]);
   }
   proxyFence();
   tcFenceBefore();
-  __syncthreads();
+  tileSync<T>(tile);
   const unsigned idesc = umIdesc(128, H);
-  const unsigned aBase = smemU32(sm.a);
-  float y = sm.bo;
+  f32x2 y = pack2(sm.bo, 0.0f);
   bool ok = true;
 #pragma unroll 1
   for (int l = 1; l < L; ++l) {
-    if (t == 0) {
+    if (row == 0) {
       tcFenceAfter();
-      const unsigned bBase = smemU32(sm.w + (l - 1) * H * H);
+      const unsigned aBase = smemU32(aTile), bBase = smemU32(sm.w + (l - 1) * H * H);
 #pragma unroll
-      for (int tt = 0; tt < T; ++tt) {
-        const unsigned aTileBase = aBase + (unsigned)(tt * 128 * H * 2);
-#pragma unroll
-        for (int s = 0; s < H / 16; ++s)
-          umma(sm.tmem + (unsigned)(tt * H), umDesc(aTileBase + s * 2 * 128 * 16, 128 * 16, 128),
-               umDesc(bBase + s * 2 * H * 16, H * 16, 128), idesc, s > 0 ? 1u : 0u);
-      }
-      ummaCommit(smemU32(&sm.bar));
+      for (int s = 0; s < H / 16; ++s)
+        umma(sm.tmem + (unsigned)(tile * H), umDesc(aBase + s * 2 * 128 * 16, 128 * 16, 128),
+             umDesc(bBase + s * 2 * H * 16, H * 16, 128), idesc, s > 0 ? 1u : 0u);
+      ummaCommit(bar);
     }
-    const bool done = mbarWaitParity(smemU32(&sm.bar), phase);
+    const bool done = mbarWaitParity(bar, phase);
     phase ^= 1u;
-    if (__syncthreads_or(!done)) {
+    if (tileSyncOr<T>(tile, !done)) {
       // let the chain finish (bounded) before the tile buffers are reused
-      mbarWaitParity(smemU32(&sm.bar), phase ^ 1u);
+      mbarWaitParity(bar, phase ^ 1u);
       ok = false;
       break;
     }
@@ -676,35 +727,43 @@ __device__ __forceinline__ bool sdfTileForward(SdfTileSmem<H, L, T> &sm, const S
       tmemWaitLoad();
 #pragma unroll
       for (int q = 0; q < kLdBatch; ++q) {
-        const int c = c0 + q;
+        const int c = (c0 + q) * 16;
 #pragma unroll
-        for (int u = 0; u < 16; ++u) r[q][u] = siluFast(r[q][u] + sm.b[l * H + c * 16 + u]);
-        if (last) {
+        for (int h = 0; h < 2; ++h) {  // eight columns at a time
+          unsigned v[4];
 #pragma unroll
-          for (int u = 0; u < 16; ++u) y = fmaf(r[q][u], sm.wo[c * 16 + u], y);
-        } else {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            uint4 v = make_uint4(packBf16(r[q][8 * h], r[q][8 * h + 1]),
-                                 packBf16(r[q][8 * h + 2], r[q][8 * h + 3]),
-                                 packBf16(r[q][8 * h + 4], r[q][8 * h + 5]),
-                                 packBf16(r[q][8 * h + 6], r[q][8 * h + 7]));
-            *reinterpret_cast<uint4 *>(aTile + tileOffset(row, c * 16 + 8 * h, 128)) = v;
+          for (int u = 0; u < 2; ++u) {
+            const int k = 8 * h + 4 * u;
+            const ulonglong2 b = four(sm.b + l * H + c + k);
+            const f32x2 s0 = siluHalf2(add2(pack2(r[q][k], r[q][k + 1]), b.x));
+            const f32x2 s1 = siluHalf2(add2(pack2(r[q][k + 2], r[q][k + 3]), b.y));
+            if (last) {
+              const ulonglong2 w = four(sm.wo + c + k);
+              y = fma2(s1, w.y, fma2(s0, w.x, y));
+            } else {
+              v[2 * u] = packed(s0);
+              v[2 * u + 1] = packed(s1);
+            }
           }
+          if (!last)
+            *reinterpret_cast<uint4 *>(aTile + tileOffset(row, c + 8 * h, 128)) =
+                make_uint4(v[0], v[1], v[2], v[3]);
         }
       }
     }
     tcFenceBefore();
     if (!last) proxyFence();
-    __syncthreads();
+    tileSync<T>(tile);
   }
-  dOut = y * net.outScale;
+  float ya, yb;
+  unpack2(y, ya, yb);
+  dOut = (ya + yb) * net.outScale;
   return ok;
 }
 
 // d[i] for point i (float4, w ignored) with shape code shapes[i] (or none).
-// kInferTiles 128-point tiles per CTA share the weights and one barrier
-// round per layer; inferLd<H>() TMEM column loads are in flight per wait.
+// kInferTiles 128-point tiles per CTA share the weights; inferLd<H>() TMEM
+// column loads are in flight per wait.
 constexpr int kInferTiles = 2;
 template <int H> constexpr int inferLd() { return H == 64 ? 2 : 4; }
 template <int H, int L>
@@ -726,7 +785,7 @@ kSdfInfer(SdfView net, const float4 *__restrict__ pts, const int *__restrict__ s
     if (!sdfTileForward<H, L, inferLd<H>(), kInferTiles>(
             sm, net, (q.x - net.shift[0]) * net.scale[0], (q.y - net.shift[1]) * net.scale[1],
             (q.z - net.shift[2]) * net.scale[2], shape, phase, d)) {
-      if (threadIdx.x == 0) atomicOr(status, (unsigned)kStatusTimeout);
+      if ((threadIdx.x & 127u) == 0) atomicOr(status, (unsigned)kStatusTimeout);
       break;
     }
     if (valid) dOut[i] = d;
@@ -1010,7 +1069,8 @@ kBatchObstacle(const BatchScene *__restrict__ scenes, const unsigned *__restrict
   if (kNet) sdfTileTeardown<H, L>(sm);
 }
 
-// Hidden-layer weights, FP32 [out][in], to the BF16 B-operand tiles.
+// Hidden-layer weights, FP32 [out][in], halved (siluHalf2), to the BF16
+// B-operand tiles.
 __global__ void __launch_bounds__(256)
 kSdfPackBf16(const float *__restrict__ p, SdfLayout ly, __nv_bfloat16 *__restrict__ w16) {
   const int H = ly.H;
@@ -1020,7 +1080,7 @@ kSdfPackBf16(const float *__restrict__ p, SdfLayout ly, __nv_bfloat16 *__restric
        e += gridDim.x * blockDim.x) {
     const unsigned l = e / per, r = e % per;
     const int o = (int)(r / H), k = (int)(r % H);
-    w16[l * per + tileOffset(o, k, H)] = __float2bfloat16_rn(p[ly.wh[l] + r]);
+    w16[l * per + tileOffset(o, k, H)] = __float2bfloat16_rn(0.5f * p[ly.wh[l] + r]);
   }
 }
 
