@@ -577,13 +577,13 @@ __device__ __forceinline__ unsigned neighbourhoodCount(int3 g, const CellRanges 
 // sign -- with no branch and no store per hit, and all table loads go out
 // before it.  Measured against the kernel it replaced (rows copied to shared
 // memory one after the other, a branch and two stores per near partner), per
-// collide: 4.2M spheres 507 against 748 us, 1M in piles 250 against 395, 1M
-// falling monodisperse 72 against 121.  All lanes scan the same row at a time:
-// skipping a lane's empty rows costs L1 hits (+13%).  64 registers (8 CTAs
-// per SM) against 72: -3%.  Shared memory is kept small because L1 gets the
+// collide: 4.2M spheres 490 against 748 us, 1M in piles 245 against 395, 1M
+// falling monodisperse 67 against 121.  All lanes scan the same row at a time:
+// skipping a lane's empty rows costs L1 hits (+13%).  56 registers (9 CTAs
+// per SM) against 72: -4%; 48 are slower again.  Shared memory is kept small because L1 gets the
 // rest of the 256 KB (31 KB per CTA instead of 17: +6%).
 template <int kMode, bool kRadiusFromW, bool kCollider, bool kForceOut, bool kPrefix>
-__global__ void __launch_bounds__(128, 8)
+__global__ void __launch_bounds__(128, 9)
 kCollideGlobal(float4 *__restrict__ newVel, const float4 *__restrict__ sortedPos,
                const float4 *__restrict__ sortedVel, const unsigned *__restrict__ index,
                CellRanges cells, unsigned n, KParams kp, CollideOut out, bool cull,
@@ -1253,7 +1253,7 @@ kCollideBatch(const BatchScene *__restrict__ scenes, const unsigned *__restrict_
   float4 v4 = ldg4(sortedVel + i);
   float3 pos = make_float3(p4.x, p4.y, p4.z), vel = make_float3(v4.x, v4.y, v4.z);
   float ri = kRadiusFromW ? p4.w : P.particleRadius;
-  int3 g = gridPos(pos.x, pos.y, pos.z, P);
+  int3 g = gridPosDivide(pos.x, pos.y, pos.z, P);
   bool cull = S.cull != 0;
   if (kRadiusFromW && !(ri <= P.particleRadius)) {
     atomicOr(status, (unsigned)kStatusRadiusBound);
@@ -1295,7 +1295,7 @@ kCollideBatch(const BatchScene *__restrict__ scenes, const unsigned *__restrict_
     integrateOneBox(pos, nv, out.dt, ri, P, S.lo, S.hi);
     out.posOut[i] = make_float4(pos.x, pos.y, pos.z, p4.w);
     newVel[i] = make_float4(nv.x, nv.y, nv.z, 0.0f);
-    int3 gn = gridPos(pos.x, pos.y, pos.z, P);
+    int3 gn = gridPosDivide(pos.x, pos.y, pos.z, P);
     const unsigned h = S.cellBase + gridHash(gn.x, gn.y, gn.z, P);
     out.hashOut[i] = h;
     out.rankOut[i] = atomicAdd(out.cnt + h, 1u);
@@ -1328,7 +1328,7 @@ void launchCollide(int mode, bool collider, float4 *newVel, const float4 *sp,
   // opt-in (fcdemSetCollidePath(1)): the culled global kernel is faster.
   // (its row windows assume the linear cell order)
   bool tiled = !prefix && g_collidePath == 1 && ((uintptr_t)sp & 15u) == 0 &&
-               kp.p.maxParticlesPerCell != kMortonTag;
+               !(kp.p.maxParticlesPerCell & kMortonOrder);
   // Culling is exact when every grid dimension is >= 3 and the largest
   // contact distance 2 * particleRadius fits in the smallest cell.
   const SimParams &P = kp.p;

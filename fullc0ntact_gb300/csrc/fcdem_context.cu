@@ -154,10 +154,20 @@ bool mortonUsable(const SimParams &p) {
          p.gridSize[0] >= 1u && p.gridSize[0] <= 1024u;
 }
 
+unsigned paramFlags(const SimParams &p, bool morton) {
+  bool exact = true;  // positive normal powers of two whose reciprocal is normal too
+  for (int k = 0; k < 3; ++k) {
+    unsigned bits;
+    std::memcpy(&bits, &p.cellSize[k], sizeof(bits));
+    exact = exact && (bits & 0x007fffffu) == 0u && bits >= 0x00800000u && bits <= 0x7e800000u;
+  }
+  return (morton && mortonUsable(p) ? kMortonOrder : 0u) | (exact ? kExactInverse : 0u);
+}
+
 KParams kparams(const Context &c) {
   KParams k;
   k.p = c.params;
-  k.p.maxParticlesPerCell = (c.morton && mortonUsable(c.params)) ? kMortonTag : 0u;
+  k.p.maxParticlesPerCell = paramFlags(c.params, c.morton != 0);
   k.radiusFromW = c.radiusFromW;
   return k;
 }

@@ -47,7 +47,7 @@ bool paramsFor(const i3d::HashGrid<float, i3d::cpu> &hg, KParams &kp) {
   kp.p.cellSize[0] = hg.cellSize_.x;
   kp.p.cellSize[1] = hg.cellSize_.y;
   kp.p.cellSize[2] = hg.cellSize_.z;
-  kp.p.maxParticlesPerCell = 0u;
+  kp.p.maxParticlesPerCell = paramFlags(kp.p, false);
   kp.radiusFromW = 0;
   for (int k = 0; k < 3; ++k) {
     const unsigned g = kp.p.gridSize[k];

@@ -129,10 +129,12 @@ void stageEnd(int stage);
 void *scratch(Context &c, size_t bytes);
 
 KParams kparams(const Context &c);
+// Flags of the library's parameter copies, in maxParticlesPerCell (unused by
+// the reference): Morton cell keys (gridHash), cell sizes that are powers of
+// two (gridPos).  Every copy that a kernel gets sets the field.
+constexpr unsigned kMortonOrder = 1u, kExactInverse = 2u;
+unsigned paramFlags(const SimParams &p, bool morton);
 // Morton cell keys need a cubic power-of-two grid of at most 1024 cells a side.
-// The library's parameter copy marks Morton order with this value in
-// maxParticlesPerCell (unused by the reference); see gridHash.
-constexpr unsigned kMortonTag = 0x4d4f5254u;
 bool mortonUsable(const SimParams &p);
 
 // Number of key bits a sort must cover for keys below numCells.

@@ -172,3 +172,31 @@ def test_tuning_and_culling_arguments_are_checked():
     assert lib.fcdemGetLastError() == 1
     net.set_tile_culling(0.0)
     assert lib.fcdemGetLastError() == 0
+
+
+@pytest.mark.parametrize("cell", [(2.0 ** -7,) * 3, (8.0, 0.5, 2.0 ** -30), (0.1,) * 3,
+                                  (2.0 ** -7, 2.0 ** -7, 0.03), (2.0 ** 126, 1.0, 2.0 ** -126)])
+def test_hash_of_power_of_two_cells_matches_oracle(cell):
+    """calcHash by multiplication (every cell size a power of two) and by
+    division: the oracle's hashes, bit for bit, cell faces, subnormal and
+    infinite quotients included."""
+    from fullc0ntact_gb300 import dem, scenes
+    from oracle import oracle as O
+    sc = scenes.random_box(5000, grid=(16, 8, 32), seed=5)
+    sc["params"].cellSize[:] = list(cell)
+    rng = np.random.default_rng(6)
+    pos = sc["pos"]
+    pos[:2000, :3] = -1.0 + rng.integers(-3, 70, (2000, 3)) * np.float32(cell)  # on faces
+    pos[2000:2010, :3] = np.float32(1e-38)
+    pos[2010, :3] = 3e38
+    pos[2011, :3] = -3e38
+    sc["params"].worldOrigin[:] = [0.0, 0.0, -1.0]
+    ds = dem.DeviceScene(sc)
+    ds.activate()
+    dem.calc_hash(ds.hash, ds.index, ds.pos, ds.n)
+    dem.check("calcHash")
+    q = (pos[:, :3].astype(np.float32) - np.float32([0.0, 0.0, -1.0])) / np.float32(cell)
+    sure = (np.abs(q) < 2.0 ** 31).all(axis=1)  # the int conversion of larger ones is undefined in C
+    h, _ = O.calc_hash(O.SimParams.from_buffer_copy(bytes(sc["params"])), pos)
+    np.testing.assert_array_equal(dem.u32(ds.hash)[sure], h[sure])
+    assert sure.any()
