@@ -288,13 +288,14 @@ kScanCells(unsigned *__restrict__ cnt, unsigned *__restrict__ off, unsigned m,
 
 // Entry i (a slot of the previous order, or the particle itself on the first
 // step) holds the particle's new cell hash h and its count rank r; slot
-// off[h] + r receives the hash, the particle's index and the entry i.
+// off[h] + r receives (h, the particle's index, the entry i, off[h]) as one
+// 16-byte word: the scatter is bound by the sectors it touches, and three
+// 4-byte arrays touched three (4.2M spheres, four steps, the first from random
+// order: 40 us a step against 50; 2M in box scenes 16.7 against 19.1).
 __global__ void __launch_bounds__(256)
-kScatterCells(const unsigned *hashN, const unsigned *rankN,
-              const unsigned *origOf, const unsigned *off,
-              unsigned *__restrict__ slotKey, unsigned *__restrict__ slotOrig,
-              unsigned *__restrict__ slotPrev, unsigned n, unsigned numCells,
-              unsigned *__restrict__ tileCnt, unsigned tiles, unsigned *status) {
+kScatterCells(const unsigned *hashN, const unsigned *rankN, const unsigned *origOf,
+              const unsigned *off, uint4 *slots, unsigned n, unsigned numCells, unsigned *tileCnt,
+              unsigned tiles, unsigned *status) {
   chainTrigger();
   chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -306,14 +307,12 @@ kScatterCells(const unsigned *hashN, const unsigned *rankN,
     atomicOr(status, (unsigned)kStatusKeyRange);
     return;
   }
-  unsigned s = off[h] + rankN[i];
+  const unsigned a = off[h], s = a + rankN[i];
   if (s >= n) {
     atomicOr(status, (unsigned)kStatusKeyRange);
     return;
   }
-  slotKey[s] = h;
-  slotOrig[s] = origOf ? origOf[i] : i;
-  slotPrev[s] = i;
+  slots[s] = make_uint4(h, origOf ? origOf[i] : i, i, a);
 }
 
 // Largest cell that the per-slot re-rank handles (each slot reads every
@@ -326,26 +325,22 @@ inline unsigned largeCapacity(unsigned n) { return n / (kFixupMaxCell + 1) + 1; 
 
 // Stable order inside each cell + the reorder gather.  The particle of slot
 // s is re-ranked among its cell's members by particle index; its position and
-// velocity are gathered from entry slotPrev[s] of the previous order.  A cell
-// above kFixupMaxCell members is appended to large[1..] (large[0] counts) by
-// its first slot and left to kFixupLarge.
+// velocity are gathered from its entry of the previous order.  A cell above
+// kFixupMaxCell members is appended to large[1..] (large[0] counts) by its
+// first slot and left to kFixupLarge.
 __global__ void __launch_bounds__(256)
-kFixupGather(const unsigned *slotKey, const unsigned *slotOrig,
-             const unsigned *slotPrev, const unsigned *off,
-             unsigned *__restrict__ hashOut, unsigned *__restrict__ indexOut,
-             float4 *__restrict__ sortedPos, float4 *__restrict__ sortedVel,
-             const float4 *prevPos, const float4 *prevVel,
-             unsigned n, unsigned numCells, unsigned *__restrict__ large, unsigned largeCap,
-             unsigned *status) {
+kFixupGather(const uint4 *slots, const unsigned *off, unsigned *hashOut, unsigned *indexOut,
+             float4 *sortedPos, float4 *sortedVel, const float4 *prevPos, const float4 *prevVel,
+             unsigned n, unsigned numCells, unsigned *large, unsigned largeCap, unsigned *status) {
   chainTrigger();
   chainWait();
   unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= n) return;
-  const unsigned h = slotKey[s];
-  const unsigned me = slotOrig[s];
-  const unsigned prev = slotPrev[s];
-  if (h >= numCells || me >= n || prev >= n) return;  // unfilled slot (reported)
-  const unsigned a = off[h], b = off[h + 1];
+  const uint4 w = slots[s];
+  const unsigned h = w.x, me = w.y, prev = w.z, a = w.w;
+  if (h >= numCells || me >= n || prev >= n || a > s) return;  // unfilled slot (reported)
+  const float4 p4 = prevPos[prev], v4 = prevVel[prev];
+  const unsigned b = min(off[h + 1], n);
   if (b - a > kFixupMaxCell) {
     if (s == a) {
       const unsigned k = atomicAdd(large, 1u);
@@ -357,13 +352,13 @@ kFixupGather(const unsigned *slotKey, const unsigned *slotOrig,
     return;
   }
   unsigned r = 0;
-  for (unsigned t = a; t < b; ++t) r += slotOrig[t] < me ? 1u : 0u;
+  for (unsigned t = a; t < b; ++t) r += slots[t].y < me ? 1u : 0u;
   const unsigned dst = a + r;
   if (dst >= n) return;
   hashOut[dst] = h;
   indexOut[dst] = me;
-  sortedPos[dst] = prevPos[prev];
-  sortedVel[dst] = prevVel[prev];
+  sortedPos[dst] = p4;
+  sortedVel[dst] = v4;
 }
 
 constexpr int kLargeThreads = 1024;
@@ -391,14 +386,14 @@ struct LargeSmem {
 // this path when the span is at most kBitmapSpan words per member.
 constexpr unsigned kBitmapSpan = 16;
 
-__device__ void bitmapRanks(const unsigned *slotOrig, unsigned a, unsigned c, unsigned n,
+__device__ void bitmapRanks(const uint4 *slots, unsigned a, unsigned c, unsigned n,
                             unsigned w0, unsigned w1, unsigned *bits, unsigned *pre,
                             LargeSmem &sm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   for (unsigned w = w0 + tid; w <= w1; w += kLargeThreads) bits[w] = 0u;
   __syncthreads();
   for (unsigned t = tid; t < c; t += kLargeThreads) {
-    const unsigned me = slotOrig[a + t];
+    const unsigned me = slots[a + t].y;
     if (me < n) atomicOr(bits + (me >> 5), 1u << (me & 31u));
   }
   __syncthreads();
@@ -504,13 +499,12 @@ __device__ void largeRadixPass(const unsigned long long *src, unsigned long long
 // bitmapRanks and gathers each member straight to its ranked place.
 // Otherwise the members (particle index, previous entry) are sorted by
 // particle index in the cell's own range of sortedPos (16 bytes per member:
-// two 8-byte arrays of the cell's size), written back to slotOrig/slotPrev,
+// two 8-byte arrays of the cell's size), written back to their slots,
 // then gathered as in kFixupGather.  idBits = bits of the largest particle
 // index; bitmaps = kBitmapSlots slots of 2 * bitmapWords(n) words (the bits,
 // then the word prefix), or nullptr for the sort only.
 __global__ void __launch_bounds__(kLargeThreads)
-kFixupLarge(unsigned *__restrict__ slotOrig, unsigned *__restrict__ slotPrev,
-            const unsigned *off, const unsigned *large,
+kFixupLarge(uint4 *slots, const unsigned *off, const unsigned *large,
             unsigned largeCap, unsigned *__restrict__ hashOut, unsigned *__restrict__ indexOut,
             float4 *__restrict__ sortedPos, float4 *__restrict__ sortedVel,
             const float4 *prevPos, const float4 *prevVel, unsigned n,
@@ -538,7 +532,7 @@ kFixupLarge(unsigned *__restrict__ slotOrig, unsigned *__restrict__ slotPrev,
       __syncthreads();
       unsigned lo = 0xffffffffu, hi = 0u;
       for (unsigned t = tid; t < c; t += kLargeThreads) {
-        const unsigned me = slotOrig[a + t];
+        const unsigned me = slots[a + t].y;
         if (me < n) {
           lo = min(lo, me);
           hi = max(hi, me);
@@ -555,9 +549,9 @@ kFixupLarge(unsigned *__restrict__ slotOrig, unsigned *__restrict__ slotPrev,
       const unsigned w0 = mlo >> 5, w1 = mhi >> 5;
       if (mlo <= mhi && w1 - w0 + 1u <= kBitmapSpan * c) {
         unsigned *pre = bits + words;
-        bitmapRanks(slotOrig, a, c, n, w0, w1, bits, pre, sm);
+        bitmapRanks(slots, a, c, n, w0, w1, bits, pre, sm);
         for (unsigned t = tid; t < c; t += kLargeThreads) {
-          const unsigned me = slotOrig[a + t], prev = slotPrev[a + t];
+          const unsigned me = slots[a + t].y, prev = slots[a + t].z;
           if (me >= n || prev >= n) continue;  // unfilled slot (reported by the scatter)
           const unsigned wd = me >> 5;
           const unsigned dst = a + pre[wd] + __popc(bits[wd] & ((1u << (me & 31u)) - 1u));
@@ -573,7 +567,7 @@ kFixupLarge(unsigned *__restrict__ slotOrig, unsigned *__restrict__ slotPrev,
     unsigned long long *A = reinterpret_cast<unsigned long long *>(sortedPos + a);
     unsigned long long *B = A + c;
     for (unsigned t = tid; t < c; t += kLargeThreads)
-      A[t] = ((unsigned long long)slotOrig[a + t] << 32) | slotPrev[a + t];
+      A[t] = ((unsigned long long)slots[a + t].y << 32) | slots[a + t].z;
     __syncthreads();
     for (int shift = 0; shift < idBits; shift += 8) {
       largeRadixPass(A, B, c, 32 + shift, sm);
@@ -583,12 +577,12 @@ kFixupLarge(unsigned *__restrict__ slotOrig, unsigned *__restrict__ slotPrev,
     }
     for (unsigned t = tid; t < c; t += kLargeThreads) {
       const unsigned long long e = A[t];
-      slotOrig[a + t] = (unsigned)(e >> 32);
-      slotPrev[a + t] = (unsigned)e;
+      slots[a + t].y = (unsigned)(e >> 32);
+      slots[a + t].z = (unsigned)e;
     }
     __syncthreads();
     for (unsigned t = tid; t < c; t += kLargeThreads) {
-      const unsigned me = slotOrig[a + t], prev = slotPrev[a + t];
+      const unsigned me = slots[a + t].y, prev = slots[a + t].z;
       if (me >= n || prev >= n) continue;  // unfilled slot (reported by the scatter)
       hashOut[a + t] = h;
       indexOut[a + t] = me;
@@ -600,20 +594,38 @@ kFixupLarge(unsigned *__restrict__ slotOrig, unsigned *__restrict__ slotPrev,
 }
 
 // cellStart/cellEnd from the prefix table (cellEnd of empty cells untouched,
-// as the reference leaves it).
+// as the reference leaves it).  Bound by HBM (8 bytes per cell): four cells per
+// thread, 16-byte accesses where the caller's cellStart allows (kVec); 16.7M
+// cells in 19 us, one cell per thread 34 (23 with read-only loads).
+template <bool kVec>
 __global__ void __launch_bounds__(256)
-kCellTables(const unsigned *off, unsigned *__restrict__ cellStart,
-            unsigned *__restrict__ cellEnd, unsigned numCells) {
+kCellTables(const unsigned *off, unsigned *cellStart, unsigned *cellEnd, unsigned numCells) {
   chainTrigger();
   chainWait();
-  size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < numCells; c += stride) {
-    unsigned a = off[c], b = off[c + 1];
-    if (a < b) {
-      cellStart[c] = a;
-      cellEnd[c] = b;
+  const size_t stride = (size_t)gridDim.x * blockDim.x * 4;
+  for (size_t c = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; c < numCells; c += stride) {
+    if (c + 4 <= numCells) {
+      const uint4 o = *reinterpret_cast<const uint4 *>(off + c);
+      const unsigned v[5] = {o.x, o.y, o.z, o.w, off[c + 4]};
+      unsigned st[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool some = v[k] < v[k + 1];
+        st[k] = some ? v[k] : kEmpty;
+        if (some) cellEnd[c + k] = v[k + 1];
+      }
+      if (kVec) {
+        *reinterpret_cast<uint4 *>(cellStart + c) = make_uint4(st[0], st[1], st[2], st[3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) cellStart[c + k] = st[k];
+      }
     } else {
-      cellStart[c] = kEmpty;
+      for (size_t k = c; k < numCells; ++k) {
+        const unsigned a = off[k], b = off[k + 1];
+        cellStart[k] = a < b ? a : kEmpty;
+        if (a < b) cellEnd[k] = b;
+      }
     }
   }
 }
@@ -705,8 +717,8 @@ kBatchIntegrateHashCount(const BatchScene *__restrict__ scenes,
 }
 
 // Buffers of the pipeline, kept in the context between calls: cnt (all zero
-// between calls) and off over numCells + 1 cells, rank/slotKey/slotIdx over
-// the particles, and the scan's look-back words.
+// between calls) and off over numCells + 1 cells, ranks and slots over the
+// particles, and the scan's look-back words.
 static bool countBuffers(Context &c, unsigned n, unsigned numCells, CountBuffers &b) {
   return countBuffersIn(c.countBuf, c.countBytes, c.countCells, n, numCells, b);
 }
@@ -718,7 +730,7 @@ bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsi
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const unsigned largeCap = largeCapacity(n);
   const unsigned tileBlocks = (tiles + kTileBlock - 1) / kTileBlock;
-  const size_t need = 2 * al(m * 4) + 4 * al((size_t)n * 4) + 3 * al((size_t)(tiles + 1) * 4) +
+  const size_t need = 2 * al(m * 4) + al((size_t)n * 4) + al((size_t)n * 16) + 3 * al((size_t)(tiles + 1) * 4) +
                       al(((size_t)largeCap + 1) * 4) + al((size_t)tileBlocks * 4) +
                       al((size_t)kBitmapSlots * 2 * bitmapWords(n) * 4);
   if (buf == nullptr || bytes < need || cells != numCells) {
@@ -755,12 +767,8 @@ bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsi
   p += al((size_t)(tiles + 1) * 4);
   b.rank = (unsigned *)p;
   p += al((size_t)n * 4);
-  b.slotKey = (unsigned *)p;
-  p += al((size_t)n * 4);
-  b.slotIdx = (unsigned *)p;
-  p += al((size_t)n * 4);
-  b.slotPrev = (unsigned *)p;
-  p += al((size_t)n * 4);
+  b.slots = (uint4 *)p;
+  p += al((size_t)n * 16);
   b.large = (unsigned *)p;
   b.largeCap = largeCap;
   p += al(((size_t)largeCap + 1) * 4);
@@ -832,27 +840,28 @@ bool countPipelineSort(Context &c, const CountBuffers &b, const unsigned *origOf
     if (!launchOk()) return false;
   }
   // hash holds the new hashes in entry order until the fix-up overwrites it
-  launchChained(true, kScatterCells, (n + 255) / 256, 256, 0, hash, b.rank, origOf, b.off, b.slotKey,
-                b.slotIdx, b.slotPrev, n, numCells, b.tileCnt, own ? b.scanTiles : 0u, c.dStatus);
+  launchChained(true, kScatterCells, (n + 255) / 256, 256, 0, hash, b.rank, origOf, b.off, b.slots, n,
+                numCells, b.tileCnt, own ? b.scanTiles : 0u, c.dStatus);
   if (!launchOk()) return false;
-  launchChained(true, kFixupGather, (n + 255) / 256, 256, 0, b.slotKey, b.slotIdx, b.slotPrev, b.off,
-                hash, index, sortedPos, sortedVel, prevPos, prevVel, n, numCells, b.large,
+  launchChained(true, kFixupGather, (n + 255) / 256, 256, 0, b.slots, b.off, hash, index,
+                 sortedPos, sortedVel, prevPos, prevVel, n, numCells, b.large,
                 b.largeCap, c.dStatus);
   if (!launchOk()) return false;
   if (n <= kFixupMaxCell) return true;  // no cell can be large
   // Returns at once when the fix-up listed no cell (the common case).
   const unsigned largeCtas = b.largeCap < numSms() ? b.largeCap : numSms();  // one per SM at most
-  launchChained(true, kFixupLarge, largeCtas, kLargeThreads, 0, b.slotIdx, b.slotPrev, b.off,
-                b.large, b.largeCap, hash, index, sortedPos, sortedVel, prevPos, prevVel, n,
+  launchChained(true, kFixupLarge, largeCtas, kLargeThreads, 0, b.slots, b.off, b.large,
+                b.largeCap, hash, index, sortedPos, sortedVel, prevPos, prevVel, n,
                 keyBits(n), b.bitmaps);
   return launchOk();
 }
 
 bool countPipelineTables(const CountBuffers &b, unsigned *cellStart, unsigned *cellEnd,
                          unsigned numCells) {
-  unsigned blocks = (numCells + 255) / 256;
+  unsigned blocks = numCells / 1024 + 1;
   if (blocks > numSms() * 16u) blocks = numSms() * 16u;
-  launchChained(true, kCellTables, blocks, 256, 0, b.off, cellStart, cellEnd, numCells);
+  const bool vec = ((uintptr_t)cellStart & 15u) == 0;
+  launchChained(true, vec ? kCellTables<true> : kCellTables<false>, blocks, 256, 0, b.off, cellStart, cellEnd, numCells);
   return launchOk();
 }
 

@@ -222,7 +222,8 @@ void launchCollideBatch(int mode, bool radiusFromW, const BatchScene *scenes,
 
 // The counting-sort pipeline of fcdemUpdate (fcdem_count.cu).
 struct CountBuffers {
-  unsigned *cnt, *off, *rank, *slotKey, *slotIdx, *slotPrev;
+  unsigned *cnt, *off, *rank;
+  uint4 *slots;                 // per slot: cell, particle, previous entry, cell's first slot
   unsigned *tileCnt, *tileOff;  // per 4096-cell tile: counts and their prefix
   unsigned *tileOffPrev;        // per tile: the constant its offsets hold, or 0xffffffff
   unsigned *large;              // [0] = count, [1..largeCap] = cells too full for the re-rank
