@@ -56,6 +56,9 @@ struct Context {
   void *countBuf = nullptr;     // counting-sort pipeline of fcdemUpdate
   size_t countBytes = 0;
   unsigned countCells = 0;
+  void *sortBuf = nullptr;      // counting sort of sortParticles
+  size_t sortBytes = 0;
+  unsigned sortCells = 0;
   void *crowdBuf = nullptr;     // collide: groups of crowded particles
   unsigned crowdCap = 0;        // particles the group list covers
 };
@@ -71,6 +74,9 @@ unsigned numSms();
 // Look-back rounds a sort tile may make before it gives up
 // (fcdemSetSortWaitLimit; default kSortWaitRounds).
 unsigned sortWaitLimit();
+// Whether a set look-back limit or a configuration chosen for n's size class
+// asks for the radix sort.
+bool radixSortAsked(unsigned n);
 // The status word of the allocation-free sort on the current device, or
 // nullptr when that sort has not been set up there (fcdem_sort.cu).
 unsigned *noAllocStatusWord();
@@ -228,6 +234,7 @@ struct CountBuffers {
   unsigned *tileOffPrev;        // per tile: the constant its offsets hold, or 0xffffffff
   unsigned *large;              // [0] = count, [1..largeCap] = cells too full for the re-rank
   unsigned *tileBlockSum;       // per 1024 tiles: their total (many-tile scans)
+  void *work;                   // countBuffersIn's extra work space
   unsigned *bitmaps;            // kFixupLarge: per-CTA bitmap + word prefix of particle indices
   unsigned scanTiles, largeCap;
 };
@@ -235,8 +242,12 @@ bool countPipelineBegin(Context &c, float4 *pos, float4 *vel, float dt, unsigned
                         unsigned n, unsigned numCells, const KParams &kp, CountBuffers &b);
 // Buffers over explicit storage (a batch owns its own); cnt/tileCnt must be
 // zero on first use.
+// workBytes: extra work space (CountBuffers::work).  mayAllocate false: only
+// buffers that are there already.
 bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsigned numCells,
-                    CountBuffers &b);
+                    CountBuffers &b, size_t workBytes = 0, bool mayAllocate = true);
+// sortParticles' counting sort; false: not taken (fcdem_count.cu).
+bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int bits);
 // First step of a batch: integrate in each scene's box + hash + count.
 bool countPipelineBeginBatch(const BatchScene *scenes, const unsigned *sceneOf, bool radiusFromW,
                              float4 *pos, float4 *vel, float dt, unsigned *hash, unsigned n,

@@ -508,6 +508,13 @@ unsigned *noAllocStatusWord() {
 
 unsigned sortWaitLimit() { return g_sortWaitRounds.load(std::memory_order_relaxed); }
 
+bool radixSortAsked(unsigned n) {
+  if (sortWaitLimit() != kSortWaitRounds) return true;
+  chooseConfig(n);  // initialises the table
+  std::lock_guard<std::mutex> lock(g_sortChoiceMutex);
+  return g_sortChoice[sizeClass(n)] >= 0;
+}
+
 }  // namespace fcdem
 
 extern "C" void fcdemSetSortWaitLimit(int rounds) {
@@ -650,6 +657,23 @@ extern "C" int fcdemAutotuneSort(unsigned numParticles, unsigned numCells, float
     if (tot < bestT) { bestT = tot; best = k; }
   }
   fcdemSetSortConfig(n, best);
+  // the counting sort that sortParticles takes by default, timed alike
+  float count = 0.0f;
+  bool counted = true;
+  for (int rep = 0; rep < 4 && counted; ++rep) {
+    cudaMemcpyAsync(k1, k0, (size_t)n * 8, cudaMemcpyDeviceToDevice, st);
+    cudaEventRecord(e0, st);
+    counted = countSortPairs(c, k1, v1, n, bits);
+    cudaEventRecord(e1, st);
+    cudaEventSynchronize(e1);
+    float t = 0.0f;
+    cudaEventElapsedTime(&t, e0, e1);
+    if (rep > 0) count += t;
+  }
+  if (counted && count < bestT) {
+    bestT = count;
+    fcdemSetSortConfig(n, -1);
+  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaFree(k0);

@@ -13,6 +13,8 @@ constexpr unsigned kEmpty = 0xffffffffu;
 __global__ void __launch_bounds__(256)
 kIntegrate(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt,
            unsigned n, KParams kp) {
+  chainTrigger();
+  chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float4 p4 = pos[i], v4 = vel[i];
@@ -27,10 +29,12 @@ kIntegrate(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt,
 // calcHash (particles_kernel.cu:97-115).
 __global__ void __launch_bounds__(256)
 kCalcHash(unsigned *__restrict__ hash, unsigned *__restrict__ index,
-          const float4 *__restrict__ pos, unsigned n, KParams kp) {
+          const float4 *pos, unsigned n, KParams kp) {
+  chainTrigger();
+  chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float4 p = ldg4(pos + i);
+  float4 p = pos[i];
   int3 g = gridPos(p.x, p.y, p.z, kp.p);
   hash[i] = gridHash(g.x, g.y, g.z, kp.p);
   index[i] = i;
@@ -60,6 +64,8 @@ kIntegrateHash(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt,
 // pointer allows, grid-stride.
 __global__ void __launch_bounds__(256)
 kFill(unsigned *__restrict__ p, size_t count, unsigned value) {
+  chainTrigger();
+  chainWait();
   size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   size_t stride = (size_t)gridDim.x * blockDim.x;
   size_t head = (16u - ((uintptr_t)p & 15u)) / 4u & 3u;
@@ -79,7 +85,7 @@ void fillU32(Context &, unsigned *p, size_t count, unsigned value) {
   unsigned blocks = (unsigned)((work + 255) / 256);
   if (blocks > numSms() * 16u) blocks = numSms() * 16u;
   if (blocks == 0) blocks = 1;
-  kFill<<<blocks, 256, 0, curStream()>>>(p, count, value);
+  launchChained(true, kFill, blocks, 256, 0, p, count, value);
   launchOk();
 }
 
@@ -90,13 +96,15 @@ void fillU32(Context &, unsigned *p, size_t count, unsigned value) {
 __global__ void __launch_bounds__(256)
 kReorder(unsigned *__restrict__ cellStart, unsigned *__restrict__ cellEnd,
          float4 *__restrict__ sortedPos, float4 *__restrict__ sortedVel,
-         const unsigned *__restrict__ hash, const unsigned *__restrict__ index,
-         const float4 *__restrict__ oldPos, const float4 *__restrict__ oldVel,
+         const unsigned *hash, const unsigned *index,
+         const float4 *oldPos, const float4 *oldVel,
          unsigned n, unsigned numCells, unsigned *status) {
+  chainTrigger();
+  chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  unsigned h = __ldg(hash + i);
-  unsigned s = __ldg(index + i);
+  unsigned h = hash[i];
+  unsigned s = index[i];
   // Hashes come from calcHash and are below numCells, indices below n; a
   // caller's array that breaks this is reported instead of written through.
   if (h >= numCells || s >= n) {
@@ -106,15 +114,15 @@ kReorder(unsigned *__restrict__ cellStart, unsigned *__restrict__ cellEnd,
   if (i == 0) {
     cellStart[h] = 0;
   } else {
-    unsigned hp = __ldg(hash + i - 1);
+    unsigned hp = hash[i - 1];
     if (h != hp) {
       cellStart[h] = i;
       if (hp < numCells) cellEnd[hp] = i;
     }
   }
   if (i == n - 1) cellEnd[h] = n;
-  sortedPos[i] = ldg4(oldPos + s);
-  sortedVel[i] = ldg4(oldVel + s);
+  sortedPos[i] = oldPos[s];
+  sortedVel[i] = oldVel[s];
 }
 
 // collide lives in fcdem_collide.cu (launchCollide).
@@ -129,14 +137,14 @@ void launchIntegrateHash(float4 *pos, float4 *vel, float dt, unsigned *hash,
 
 void launchIntegrate(float4 *pos, float4 *vel, float dt, unsigned n, const KParams &kp) {
   if (n == 0) return;
-  kIntegrate<<<(n + 255) / 256, 256, 0, curStream()>>>(pos, vel, dt, n, kp);
+  launchChained(true, kIntegrate, (n + 255) / 256, 256, 0, pos, vel, dt, n, kp);
   launchOk();
 }
 
 void launchCalcHash(unsigned *hash, unsigned *index, const float4 *pos, unsigned n,
                     const KParams &kp) {
   if (n == 0) return;
-  kCalcHash<<<(n + 255) / 256, 256, 0, curStream()>>>(hash, index, pos, n, kp);
+  launchChained(true, kCalcHash, (n + 255) / 256, 256, 0, hash, index, pos, n, kp);
   launchOk();
 }
 
@@ -145,9 +153,8 @@ void launchReorder(unsigned *cellStart, unsigned *cellEnd, float4 *sortedPos,
                    const unsigned *index, const float4 *oldPos,
                    const float4 *oldVel, unsigned n, unsigned numCells) {
   if (n == 0) return;
-  kReorder<<<(n + 255) / 256, 256, 0, curStream()>>>(
-      cellStart, cellEnd, sortedPos, sortedVel, hash, index, oldPos, oldVel, n,
-      numCells, ctx().dStatus);
+  launchChained(true, kReorder, (n + 255) / 256, 256, 0, cellStart, cellEnd, sortedPos, sortedVel,
+                hash, index, oldPos, oldVel, n, numCells, ctx().dStatus);
   launchOk();
 }
 
@@ -189,9 +196,7 @@ void integrateSystem(float *pos, float *vel, float deltaTime, uint numParticles)
   if (!c.haveParams) { setError(FCDEM_ERR_NO_PARAMS); return; }
   if (numParticles == 0) return;
   if (!pos || !vel) { setError(FCDEM_ERR_INVALID_VALUE); return; }
-  kIntegrate<<<(numParticles + 255) / 256, 256, 0, curStream()>>>(
-      (float4 *)pos, (float4 *)vel, deltaTime, numParticles, kparams(c));
-  launchOk();
+  launchIntegrate((float4 *)pos, (float4 *)vel, deltaTime, numParticles, kparams(c));
 }
 
 void calcHash(uint *gridParticleHash, uint *gridParticleIndex, float *pos,
@@ -206,10 +211,8 @@ void calcHash(uint *gridParticleHash, uint *gridParticleIndex, float *pos,
     setError(FCDEM_ERR_INVALID_VALUE);
     return;
   }
-  unsigned n = (unsigned)numParticles;
-  kCalcHash<<<(n + 255) / 256, 256, 0, curStream()>>>(
-      gridParticleHash, gridParticleIndex, (const float4 *)pos, n, kparams(c));
-  launchOk();
+  launchCalcHash(gridParticleHash, gridParticleIndex, (const float4 *)pos,
+                 (unsigned)numParticles, kparams(c));
 }
 
 void reorderDataAndFindCellStart(uint *cellStart, uint *cellEnd,
@@ -258,6 +261,9 @@ void sortParticles(uint *dGridParticleHash, uint *dGridParticleIndex,
     return;
   }
   int bits = c.haveParams ? keyBits(c.params.numCells) : 32;
+  if (!radixSortAsked(numParticles) &&
+      countSortPairs(c, dGridParticleHash, dGridParticleIndex, numParticles, bits))
+    return;
   radixSortPairs(c, dGridParticleHash, dGridParticleIndex, numParticles, bits);
 }
 

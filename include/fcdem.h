@@ -109,7 +109,9 @@ void calcHash(uint *gridParticleHash, uint *gridParticleIndex, float *pos,
 
 /* particleSystem.cu:265-270: stable ascending sort of (hash, index) in place.
  * Keys are expected below 2^ceil(log2(numCells)) of the current parameters;
- * a larger key records FCDEM_ERR_KEY_RANGE. */
+ * a larger key records FCDEM_ERR_KEY_RANGE.  Up to 2,097,152 pairs with keys
+ * of at most 24 bits are counted (a counting sort over the cells), others
+ * take the radix sort. */
 void sortParticles(uint *dGridParticleHash, uint *dGridParticleIndex,
                    uint numParticles);
 
@@ -228,19 +230,22 @@ void fcdemUpdate(float *pos, float *vel, float *sortedPos, float *sortedVel,
 void fcdemSetCollidePath(int path);
 
 /* Test hook: the number of look-back rounds a tile of the radix sort
- * (sortParticles, fcdemSortParticlesNoAlloc) may wait for its predecessors
+ * (fcdemSortParticlesNoAlloc, and sortParticles, which takes the radix sort
+ * while a limit is set) may wait for its predecessors
  * before it gives up, records FCDEM_ERR_DEVICE_TIMEOUT and finishes with the
  * prefix it has (a wrong order, every write still inside the arrays).
  * 0: no waiting at all; negative: the default, 2^22 rounds. */
 void fcdemSetSortWaitLimit(int rounds);
 
-/* Sort tuning.  The counting passes of the sort come in several block
- * shapes (threads x keys per thread); results are identical.
- * fcdemAutotuneSort times each on numParticles uniform keys below numCells
- * (allocating temporary device memory), keeps the fastest for that size
- * class (power-of-two bucket of numParticles) and returns its index (-1 on
- * error); *bestMs receives its time.  fcdemSetSortConfig forces one
- * (-1 = default) and returns the number of configurations. */
+/* Sort tuning.  The passes of the radix sort come in several block shapes
+ * (threads x keys per thread); results are identical.  fcdemAutotuneSort
+ * times each on numParticles uniform keys below numCells (allocating
+ * temporary device memory), keeps the fastest for that size class
+ * (power-of-two bucket of numParticles) and returns its index (-1 on error);
+ * where sortParticles' default, the counting sort, is faster than all of
+ * them, that stays the choice.  *bestMs receives the kept one's time.
+ * fcdemSetSortConfig forces a shape, and with it the radix sort in
+ * sortParticles (-1 = default), and returns the number of shapes. */
 int fcdemAutotuneSort(unsigned numParticles, unsigned numCells, float *bestMs);
 int fcdemSetSortConfig(unsigned numParticles, int config);
 

@@ -151,3 +151,33 @@ def test_lookback_wait_that_runs_out_is_reported_and_recovers():
     rk, rv = _sort_cpu(keys, vals)
     np.testing.assert_array_equal(k, rk)
     np.testing.assert_array_equal(v, rv)
+
+
+@pytest.mark.parametrize("cells", [1, 2, 4096, 2 ** 18, 3 * 2 ** 17, 2 ** 24, 2 ** 25])
+@pytest.mark.parametrize("n", [2, 255, 257, 1024, 1025, 4096, 262_144, 262_145, 2 ** 21, 2 ** 21 + 1])
+def test_counting_and_radix_sort_agree(n, cells):
+    """sortParticles by default (the counting sort up to its bounds) against the
+    CPU's stable sort: sizes around its blocks, its large cells and its
+    bounds; uniform keys, one cell for all, and a few crowded cells; values
+    that are no permutation.  A forced configuration (the radix sort) gives
+    the same arrays."""
+    from fullc0ntact_gb300 import dem
+    rng = np.random.default_rng(n + cells)
+    vals = rng.integers(0, 2 ** 32, n, dtype=np.uint64).astype(np.uint32)
+    kinds = [rng.integers(0, cells, n), np.full(n, cells - 1)]
+    if n <= 300_000:
+        kinds.append(np.where(rng.random(n) < 0.7, rng.integers(0, min(cells, 3), n),
+                              rng.integers(0, cells, n)))
+    for keys in kinds:
+        keys = keys.astype(np.uint32)
+        rk, rv = _sort_cpu(keys, vals)
+        k, v = _sort_gpu(keys, vals, cells)
+        np.testing.assert_array_equal(k, rk)
+        np.testing.assert_array_equal(v, rv)
+    try:
+        dem.lib.fcdemSetSortConfig(n, 0)
+        k, v = _sort_gpu(keys, vals, cells)
+    finally:
+        dem.lib.fcdemSetSortConfig(n, -1)
+    np.testing.assert_array_equal(k, rk)
+    np.testing.assert_array_equal(v, rv)
