@@ -86,10 +86,14 @@ Context &ctx() {
   if (c.device < 0) {
     std::lock_guard<std::mutex> lock(g_mutex);
     if (c.device < 0) {
+      // mapped host memory: kernels touch it on an error only, and
+      // fcdemGetLastError reads it without a copy
       unsigned *status = nullptr;
-      if (cudaOk(cudaMalloc(&status, sizeof(unsigned))) &&
-          cudaOk(cudaMemset(status, 0, sizeof(unsigned)))) {
-        c.dStatus = status;
+      if (cudaOk(cudaHostAlloc(&status, sizeof(unsigned),
+                               cudaHostAllocMapped | cudaHostAllocPortable))) {
+        *status = 0u;
+        c.hStatus = status;
+        if (!cudaOk(cudaHostGetDevicePointer(&c.dStatus, status, 0))) c.dStatus = nullptr;
       }
       c.device = dev;
     }
@@ -257,9 +261,17 @@ void setParameters(SimParams *hostParams) {
 }  // extern "C"
 
 namespace {
-// Reads and clears a device status word (synchronising the library stream)
-// and records the first error its bits stand for.
-void drainStatus(unsigned *word) {
+// Records the first error that the bits of a status word stand for.
+void recordStatus(unsigned status) {
+  if (status & kStatusTimeout) setError(FCDEM_ERR_DEVICE_TIMEOUT);
+  else if (status & kStatusKeyRange) setError(FCDEM_ERR_KEY_RANGE);
+  else if (status & kStatusRadiusBound) setError(FCDEM_ERR_RADIUS_BOUND);
+  else if (status & kStatusCellOverflow) setError(FCDEM_ERR_CELL_OVERFLOW);
+}
+
+// Reads and clears a status word in device memory (synchronising the library
+// stream).
+void drainDeviceStatus(unsigned *word) {
   unsigned status = 0;
   cudaStream_t s = curStream();
   if (cudaMemcpyAsync(&status, word, sizeof(unsigned), cudaMemcpyDeviceToHost, s) ==
@@ -267,14 +279,22 @@ void drainStatus(unsigned *word) {
       cudaStreamSynchronize(s) == cudaSuccess) {
     if (status) {
       cudaMemsetAsync(word, 0, sizeof(unsigned), s);
-      if (status & kStatusTimeout) setError(FCDEM_ERR_DEVICE_TIMEOUT);
-      else if (status & kStatusKeyRange) setError(FCDEM_ERR_KEY_RANGE);
-      else if (status & kStatusRadiusBound) setError(FCDEM_ERR_RADIUS_BOUND);
-      else if (status & kStatusCellOverflow) setError(FCDEM_ERR_CELL_OVERFLOW);
+      recordStatus(status);
     }
   } else {
     cudaGetLastError();
     setError(FCDEM_ERR_CUDA);
+  }
+}
+
+// The same for the context's word, in mapped host memory.
+void drainStatus(Context &c) {
+  if (!cudaOk(cudaStreamSynchronize(curStream()))) return;
+  volatile unsigned *word = c.hStatus;
+  const unsigned status = *word;
+  if (status) {
+    *word = 0u;
+    recordStatus(status);
   }
 }
 }  // namespace
@@ -283,9 +303,9 @@ extern "C" {
 
 int fcdemGetLastError(void) {
   Context &c = ctx();
-  if (c.dStatus) drainStatus(c.dStatus);
+  if (c.dStatus) drainStatus(c);
   // the allocation-free sort keeps its own status word in its static scratch
-  if (unsigned *w = noAllocStatusWord()) drainStatus(w);
+  if (unsigned *w = noAllocStatusWord()) drainDeviceStatus(w);
   return g_error.exchange(FCDEM_SUCCESS);
 }
 

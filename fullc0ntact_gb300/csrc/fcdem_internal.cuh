@@ -50,7 +50,8 @@ struct Context {
   SimParams params{};
   int radiusFromW = 0;
   int morton = 0;               // fcdemSetCellOrder
-  unsigned *dStatus = nullptr;  // one device word of kStatus* bits
+  unsigned *dStatus = nullptr;  // one word of kStatus* bits (mapped host memory) ...
+  unsigned *hStatus = nullptr;  // ... as the host sees it
   void *scratch = nullptr;      // grown on demand, never shrunk
   size_t scratchBytes = 0;
   void *countBuf = nullptr;     // counting-sort pipeline of fcdemUpdate

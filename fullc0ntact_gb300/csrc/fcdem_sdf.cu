@@ -215,7 +215,7 @@ kSdfTrain(SdfView net, const float4 *__restrict__ samples, const int *__restrict
     for (int e = t; e < H * Q; e += T)
       *reinterpret_cast<float4 *>(&sm.w[l - 1][e / Q][4 * (e % Q)]) = src[e];
   }
-  for (int e = t; e < H * D; e += T) sm.w0[e % D][e / D] = net.p[ly.w0 + e];
+  for (int e = t; e < H * D; e += T) sm.w0[e / H][e % H] = net.p[ly.w0 + (e % H) * D + e / H];
   if (t < H) {
     sm.b[0][t] = net.p[ly.b0 + t];
     for (int l = 1; l < L; ++l) sm.b[l][t] = net.p[ly.bh[l - 1] + t];
@@ -576,7 +576,7 @@ __device__ __forceinline__ void sdfTileSetup(SdfTileSmem<H, L, T> &sm, const Sdf
   for (int e = t; e < (L - 1) * H * H / 8; e += blockDim.x) dst[e] = __ldg(src + e);
   const SdfLayout &ly = net.lay;
   for (int e = t; e < H * ly.D; e += blockDim.x)
-    sm.w0[e % ly.D][e / ly.D] = 0.5f * __ldg(net.p + ly.w0 + e);
+    sm.w0[e / H][e % H] = 0.5f * __ldg(net.p + ly.w0 + (e % H) * ly.D + e / H);
   for (int e = t; e < H; e += blockDim.x) {
     sm.b[e] = 0.5f * __ldg(net.p + ly.b0 + e);
     for (int l = 1; l < L; ++l) sm.b[l * H + e] = 0.5f * __ldg(net.p + ly.bh[l - 1] + e);

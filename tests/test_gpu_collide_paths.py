@@ -314,3 +314,4 @@ def test_row_scan_edges_match_oracle(grid, n, kind, poly, many):
                     np.testing.assert_array_equal(a.cpu().numpy(), b)
         finally:
             dem.lib.fcdemSetCrowdPath(1)
+            dem.set_radius_mode(False)
