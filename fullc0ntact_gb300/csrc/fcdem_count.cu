@@ -866,7 +866,7 @@ bool countPipelineBegin(Context &c, float4 *pos, float4 *vel, float dt, unsigned
                         unsigned n, unsigned numCells, const KParams &kp, CountBuffers &b) {
   if (!countBuffers(c, n, numCells, b)) return false;
   const bool tiles = n <= kTileAtomicsMax;
-  launchChained(false, tiles ? kIntegrateHashCount<true> : kIntegrateHashCount<false>,
+  launchChained(true, tiles ? kIntegrateHashCount<true> : kIntegrateHashCount<false>,
                 (n + 255) / 256, 256, 0, pos, vel, dt, hash, b.rank, b.cnt, b.tileCnt, n, kp);
   if (!launchOk()) return false;
   if (tiles) return true;
@@ -877,7 +877,7 @@ bool countPipelineBegin(Context &c, float4 *pos, float4 *vel, float dt, unsigned
 bool countPipelineBeginBatch(const BatchScene *scenes, const unsigned *sceneOf, bool radiusFromW,
                              float4 *pos, float4 *vel, float dt, unsigned *hash, unsigned n,
                              unsigned numCells, const CountBuffers &b) {
-  launchChained(false, radiusFromW ? kBatchIntegrateHashCount<true> : kBatchIntegrateHashCount<false>,
+  launchChained(true, radiusFromW ? kBatchIntegrateHashCount<true> : kBatchIntegrateHashCount<false>,
                 (n + 255) / 256, 256, 0, scenes, sceneOf, pos, vel, dt, hash, b.rank, b.cnt, n);
   if (!launchOk()) return false;
   launchChained(true, kTileReduce, b.scanTiles, kScanThreads, 0, b.cnt, b.tileCnt, numCells + 1);

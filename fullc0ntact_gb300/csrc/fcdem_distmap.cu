@@ -20,6 +20,8 @@ template <bool kCount>
 __global__ void __launch_bounds__(256)
 kIntegrateDistMap(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt, unsigned n,
                   KParams kp, MapView M, int useMap, UmCount count) {
+  chainTrigger();
+  chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const SimParams &P = kp.p;
@@ -40,10 +42,12 @@ kIntegrateDistMap(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt, 
 }
 
 __global__ void __launch_bounds__(256)
-kHashCount(const float4 *__restrict__ pos, unsigned n, KParams kp, UmCount count) {
+kHashCount(const float4 *pos, unsigned n, KParams kp, UmCount count) {
+  chainTrigger();
+  chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const float4 p4 = __ldg(pos + i);
+  const float4 p4 = pos[i];
   const int3 gp = gridPos(p4.x, p4.y, p4.z, kp.p);
   const unsigned h = gridHash(gp.x, gp.y, gp.z, kp.p);
   count.hash[i] = h;
@@ -169,7 +173,7 @@ kIntegrateRigidBodies(fcdemRigidBody *__restrict__ bodies, unsigned nb,
 namespace fcdem {
 
 bool umHashCount(const float4 *pos, unsigned n, const KParams &kp, const UmCount &count) {
-  kHashCount<<<(n + 255) / 256, 256, 0, curStream()>>>(pos, n, kp, count);
+  launchChained(true, kHashCount, (n + 255) / 256, 256, 0, pos, n, kp, count);
   return launchOk();
 }
 
@@ -178,12 +182,8 @@ bool mapIntegrate(float4 *pos, float4 *vel, float dt, unsigned n, const KParams 
   MapView M{};
   if (map) M = view(map);
   const unsigned blocks = (n + 255) / 256;
-  if (count)
-    kIntegrateDistMap<true><<<blocks, 256, 0, curStream()>>>(pos, vel, dt, n, kp, M,
-                                                             map ? 1 : 0, *count);
-  else
-    kIntegrateDistMap<false><<<blocks, 256, 0, curStream()>>>(pos, vel, dt, n, kp, M,
-                                                              map ? 1 : 0, UmCount{});
+  launchChained(true, count ? kIntegrateDistMap<true> : kIntegrateDistMap<false>, blocks, 256, 0, pos,
+                vel, dt, n, kp, M, map ? 1 : 0, count ? *count : UmCount{});
   return launchOk();
 }
 

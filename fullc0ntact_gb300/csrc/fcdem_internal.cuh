@@ -99,13 +99,12 @@ bool launchOk();
 // chainTrigger() (the next one may start), then chainWait(), which returns
 // when the kernels before it are complete and their writes visible, and only
 // then reads or writes what others touch: a kernel's completion thus still
-// implies that of all before it.  Before chainWait() it may read what was
-// complete before the last launch that was not chained.  What earlier kernels
+// implies that of all before it, the caller's included.  What earlier kernels
 // wrote is read with plain loads: a __ldg or a const __restrict__ parameter
 // tells the compiler that the value never changes, and it may then load it
-// before chainWait().  The first launch of
-// a call is not chained (its inputs come from the caller's work); launched
-// that way the two calls do nothing.
+// before chainWait().  (kSdfTrain reads its samples before chainWait(); its
+// first launch of a call is not chained.)  Launched without the attribute the
+// two calls do nothing.
 __device__ __forceinline__ void chainTrigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
