@@ -9,14 +9,15 @@
 //           collide+integrate of the previous step, or kIntegrateHashCount)
 //           also takes r = atomicAdd(&cnt[h], 1) and counts h's 4096-cell
 //           tile in tileCnt;
-//   scan    kScanTiles (one CTA; above 8192 tiles kScanTileBlocks and
-//           kAddTileBlocks) scans the tile counts, kScanCells scans
-//           each tile's cells from its tile offset -- no inter-CTA waits; a
+//   scan    up to 4,608 tiles kScanCellsOwn, whose CTAs sum the tile counts
+//           before their own; above that kScanTiles (one CTA) or
+//           kScanTileBlocks and kAddTileBlocks scan the tile counts and
+//           kScanCellsMany the tiles' cells -- no inter-CTA waits; a
 //           tile without particles writes its constant offsets and skips
 //           reading cnt.  off = exclusive prefix sum of cnt over C + 1 cells,
 //           cnt and tileCnt are cleared for the next step; off[c] .. off[c+1]
 //           is cell c's range, empty or not;
-//   scatter kScatterCells: slot off[h] + r receives (h, particle);
+//   scatter kScatterCells: slot off[h] + r receives (h, particle, ...);
 //   fix-up  kFixupGather: the atomic ranks order a cell's members
 //           arbitrarily, so each slot re-ranks its particle among the
 //           members of its cell by particle index (the order of the
@@ -31,6 +32,8 @@
 // listed cell one CTA that ranks its members by particle index, whatever the
 // cell's size: with a bitmap of their indices when the indices are dense
 // enough, else with a stable block radix sort.
+#include <algorithm>
+
 #include "fcdem_dem.cuh"
 
 namespace fcdem {
@@ -105,7 +108,7 @@ kScanTiles(unsigned *__restrict__ tileCnt, unsigned *__restrict__ tileOff, unsig
 // total, kAddTileBlocks adds the totals of the blocks before.
 constexpr unsigned kTileBlock = 1024;
 constexpr unsigned kTilesOneCta = 8192;  // up to this many tiles kScanTiles runs alone
-constexpr unsigned kTilesOwnPrefix = 4608;  // up to this many tiles kScanCells sums them itself
+constexpr unsigned kTilesOwnPrefix = 4608;  // up to this many tiles kScanCellsOwn
 
 __global__ void __launch_bounds__(kTileBlock)
 kScanTileBlocks(unsigned *__restrict__ tileCnt, unsigned *__restrict__ tileOff, unsigned tiles,
@@ -164,52 +167,24 @@ kAddTileBlocks(unsigned *__restrict__ tileOff, unsigned tiles,
     tileOff[tiles] = carry + blockSum[blockIdx.x];
 }
 
-// off[c] = tileOff[tile] + exclusive prefix of cnt within the tile, cnt
-// cleared.  A tile without particles only writes its constant offsets, and
-// not even those when off already holds them: tileOffPrev[tile] records the
-// constant a tile's offsets were last written with (0xffffffff after a tile
-// with particles, whose offsets vary), so a tile that stays empty with the
-// same prefix -- the common case in sparse grids: the cells above and below
-// a pile -- is left as it is.
+// One tile of the cell scan: off[c] = t0 + exclusive prefix of cnt within the
+// tile, cnt cleared.  A tile without particles (t0 == t1) only writes its
+// constant offsets; tileOffPrev[tile] records the constant a tile's offsets
+// were last written with (0xffffffff after a tile with particles, whose
+// offsets vary), and a tile that stays empty with the same prefix -- the
+// common case in sparse grids: the cells above and below a pile -- is left as
+// it is by the callers.
 // Round q of a tile covers cells q*1024 .. +1024, thread t the four at 4t
-// (16-byte accesses, coalesced).
-// kOwnPrefix: few tiles; each CTA sums the tile counts before its own itself
-// (tileOff is then tileCnt, cleared by the scatter), which saves the launch
-// of kScanTiles and its single CTA's latency (4 to 7 us per step).
-template <bool kOwnPrefix>
-__global__ void __launch_bounds__(kScanThreads)
-kScanCells(unsigned *__restrict__ cnt, unsigned *__restrict__ off, unsigned m,
-           const unsigned *tileOff, unsigned *__restrict__ tileOffPrev,
-           unsigned *__restrict__ largeCount, unsigned *__restrict__ crowdCount) {
-  __shared__ unsigned sWarp[kScanThreads / 32];
+// (16-byte accesses, coalesced).  All threads of the CTA, which have met at a
+// barrier since tileOffPrev was read and sWarp was used.
+__device__ __forceinline__ void scanTile(unsigned tile, unsigned t0, unsigned t1, unsigned *cnt,
+                                         unsigned *off, unsigned m, unsigned *tileOffPrev,
+                                         unsigned *sWarp) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const unsigned tile = blockIdx.x;
   constexpr int kRounds = kScanItems / 4;
   const size_t tbase = (size_t)tile * kScanTile;
-  chainTrigger();
-  chainWait();
-  unsigned t0, t1;
-  if (kOwnPrefix) {
-    if (tile == 0 && tid == 0) resetLists(largeCount, crowdCount);
-    unsigned part = 0;
-    for (unsigned k = tid; k < tile; k += kScanThreads) part += tileOff[k];
-    part = __reduce_add_sync(0xffffffffu, part);
-    if (lane == 0) sWarp[warp] = part;
-    __syncthreads();
-    t0 = 0;
-#pragma unroll
-    for (int w = 0; w < kScanThreads / 32; ++w) t0 += sWarp[w];
-    t1 = t0 + tileOff[tile];
-    __syncthreads();  // sWarp is used again below
-  } else {
-    t0 = tileOff[tile];
-    t1 = tileOff[tile + 1];
-  }
-  const unsigned prev = tileOffPrev[tile];  // read by every thread before thread 0 writes
-  if (t0 == t1) {  // empty tile: every cell starts (and ends) at t0
-    if (prev == t0) return;  // off already holds t0 in every cell of the tile
-    __syncthreads();
-    if (tid == 0) tileOffPrev[tile] = t0;
+  if (tid == 0) tileOffPrev[tile] = t0 == t1 ? t0 : 0xffffffffu;
+  if (t0 == t1) {  // every cell starts (and ends) at t0
 #pragma unroll
     for (int q = 0; q < kRounds; ++q) {
       const size_t c0 = tbase + (size_t)q * (kScanThreads * 4) + (size_t)tid * 4;
@@ -222,8 +197,6 @@ kScanCells(unsigned *__restrict__ cnt, unsigned *__restrict__ off, unsigned m,
     }
     return;
   }
-  __syncthreads();
-  if (tid == 0 && prev != 0xffffffffu) tileOffPrev[tile] = 0xffffffffu;  // offsets vary
   uint4 v[kRounds];
   unsigned excl[kRounds];
 #pragma unroll
@@ -283,6 +256,60 @@ kScanCells(unsigned *__restrict__ cnt, unsigned *__restrict__ off, unsigned m,
           cnt[c0 + k] = 0u;
         }
     }
+  }
+}
+
+// Few tiles (kTilesOwnPrefix): one CTA per tile, which sums the tile counts
+// before its own itself; the scatter clears them.  Saves the launch of
+// kScanTiles and its single CTA's latency (4 to 7 us per step).
+__global__ void __launch_bounds__(kScanThreads)
+kScanCellsOwn(unsigned *cnt, unsigned *off, unsigned m, const unsigned *tileCnt,
+              unsigned *tileOffPrev, unsigned *largeCount, unsigned *crowdCount) {
+  __shared__ unsigned sWarp[kScanThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned tile = blockIdx.x;
+  chainTrigger();
+  chainWait();
+  if (tile == 0 && tid == 0) resetLists(largeCount, crowdCount);
+  const unsigned held = tileOffPrev[tile], mine = tileCnt[tile];
+  unsigned part = 0;
+  for (unsigned k = tid; k < tile; k += kScanThreads) part += tileCnt[k];
+  part = __reduce_add_sync(0xffffffffu, part);
+  if (lane == 0) sWarp[warp] = part;
+  __syncthreads();
+  unsigned t0 = 0;
+#pragma unroll
+  for (int w = 0; w < kScanThreads / 32; ++w) t0 += sWarp[w];
+  if (mine == 0u && held == t0) return;
+  __syncthreads();  // sWarp is used again
+  scanTile(tile, t0, t0 + mine, cnt, off, m, tileOffPrev, sWarp);
+}
+
+// Many tiles: a CTA takes tiles blockIdx, blockIdx + grid, ... (at most 32).
+// Neighbouring tiles, which are full or empty together, go to different CTAs,
+// and an empty one that stays as it is costs a lane's three loads instead of
+// a CTA (20,481 tiles of 40 obstacle scenes: 25 -> 11 us; with 4,097 tiles a
+// CTA each is as fast).
+constexpr unsigned kScanCtas = 8 * 152;
+__global__ void __launch_bounds__(kScanThreads)
+kScanCellsMany(unsigned *cnt, unsigned *off, unsigned m, unsigned tiles, const unsigned *tileOff,
+               unsigned *tileOffPrev) {
+  __shared__ unsigned sWarp[kScanThreads / 32];
+  const unsigned lane = threadIdx.x & 31u;
+  chainTrigger();
+  chainWait();
+  // lane k: the CTA's tile k, its first slot, its end and what off holds there
+  const unsigned mine = blockIdx.x + lane * gridDim.x;
+  const unsigned first = mine < tiles ? tileOff[mine] : 0u;
+  const unsigned end = mine < tiles ? tileOff[mine + 1] : 0u;
+  const unsigned held = mine < tiles ? tileOffPrev[mine] : 0u;
+  unsigned todo = __ballot_sync(0xffffffffu, mine < tiles && (first != end || held != first));
+  __syncthreads();  // every warp has read tileOffPrev
+  while (todo) {
+    const int k = __ffs((int)todo) - 1;
+    todo &= todo - 1u;
+    scanTile(blockIdx.x + (unsigned)k * gridDim.x, __shfl_sync(0xffffffffu, first, k),
+             __shfl_sync(0xffffffffu, end, k), cnt, off, m, tileOffPrev, sWarp);
   }
 }
 
@@ -821,7 +848,7 @@ bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsi
     bytes = need;
     cells = numCells;
     if (!cudaOk(cudaMemset(buf, 0, need))) return false;  // cnt starts at zero
-    // no tile's offsets are known yet (see kScanCells)
+    // no tile's offsets are known yet (see scanTile)
     const size_t prevAt = 2 * al(m * 4) + 2 * al((size_t)(tiles + 1) * 4);
     if (!cudaOk(cudaMemset((char *)buf + prevAt, 0xff, (size_t)(tiles + 1) * 4))) return false;
   }
@@ -895,7 +922,7 @@ bool countPipelineSort(Context &c, const CountBuffers &b, const unsigned *origOf
   const unsigned m = numCells + 1;
   const bool own = b.scanTiles <= kTilesOwnPrefix;
   if (own) {
-    launchChained(true, kScanCells<true>, b.scanTiles, kScanThreads, 0, b.cnt, b.off, m, b.tileCnt,
+    launchChained(true, kScanCellsOwn, b.scanTiles, kScanThreads, 0, b.cnt, b.off, m, b.tileCnt,
                   b.tileOffPrev, b.large, crowdCount);
     if (!launchOk()) return false;
   } else {
@@ -912,8 +939,9 @@ bool countPipelineSort(Context &c, const CountBuffers &b, const unsigned *origOf
                     b.tileBlockSum);
       if (!launchOk()) return false;
     }
-    launchChained(true, kScanCells<false>, b.scanTiles, kScanThreads, 0, b.cnt, b.off, m, b.tileOff,
-                  b.tileOffPrev, b.large, crowdCount);
+    const unsigned ctas = std::min(b.scanTiles, std::max(kScanCtas, (b.scanTiles + 31u) / 32u));
+    launchChained(true, kScanCellsMany, ctas, kScanThreads, 0, b.cnt, b.off, m, b.scanTiles, b.tileOff,
+                  b.tileOffPrev);
     if (!launchOk()) return false;
   }
   // hash holds the new hashes in entry order until the fix-up overwrites it
@@ -934,7 +962,7 @@ bool countPipelineSort(Context &c, const CountBuffers &b, const unsigned *origOf
 }
 
 // Keys of at most this many bits are counted: 4096 tiles, whose counts
-// kScanCells sums itself.
+// kScanCellsOwn sums itself.
 constexpr int kCountSortBits = 24;
 constexpr unsigned kCountSortMax = 1u << 21;  // pairs
 
@@ -970,8 +998,8 @@ bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int 
     launchChained(true, kTileReduce, b.scanTiles, kScanThreads, 0, b.cnt, b.tileCnt, cells + 1);
     if (!launchOk()) return true;
   }
-  launchChained(true, kScanCells<true>, b.scanTiles, kScanThreads, 0, b.cnt, b.off, cells + 1,
-                b.tileCnt, b.tileOffPrev, b.large, nullptr);
+  launchChained(true, kScanCellsOwn, b.scanTiles, kScanThreads, 0, b.cnt, b.off, cells + 1, b.tileCnt,
+                b.tileOffPrev, b.large, nullptr);
   if (!launchOk()) return true;
   launchChained(true, kScatterPairs, blocks, 256, 0, keys, vals, b.rank, b.off, b.slots, n, mask,
                 b.tileCnt, b.scanTiles);
