@@ -824,7 +824,7 @@ static bool countBuffers(Context &c, unsigned n, unsigned numCells, CountBuffers
 }
 
 bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsigned numCells,
-                    CountBuffers &b, size_t workBytes, bool mayAllocate) {
+                    CountBuffers &b, size_t workBytes, bool mayAllocate, bool optional) {
   const size_t m = (size_t)numCells + 1;
   const unsigned tiles = (unsigned)((m + kScanTile - 1) / kScanTile);
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
@@ -842,7 +842,7 @@ bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsi
     if (cudaMalloc(&buf, need) != cudaSuccess) {
       cudaGetLastError();
       buf = nullptr;
-      setError(FCDEM_ERR_ALLOC);
+      if (!optional) setError(FCDEM_ERR_ALLOC);
       return false;
     }
     bytes = need;
@@ -987,7 +987,7 @@ bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int 
   const unsigned cells = 1u << bits, mask = cells - 1u;
   CountBuffers b;
   if (!countBuffersIn(c.sortBuf, c.sortBytes, c.sortCells, n, cells, b, 16 * (size_t)n,
-                      cap == cudaStreamCaptureStatusNone))
+                      cap == cudaStreamCaptureStatusNone, true))
     return false;
   const unsigned blocks = (n + 255) / 256;
   const bool tiles = n <= kTileAtomicsMax;

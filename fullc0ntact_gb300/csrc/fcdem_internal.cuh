@@ -243,9 +243,10 @@ bool countPipelineBegin(Context &c, float4 *pos, float4 *vel, float dt, unsigned
 // Buffers over explicit storage (a batch owns its own); cnt/tileCnt must be
 // zero on first use.
 // workBytes: extra work space (CountBuffers::work).  mayAllocate false: only
-// buffers that are there already.
+// buffers that are there already.  optional: no error when they cannot be had.
 bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsigned numCells,
-                    CountBuffers &b, size_t workBytes = 0, bool mayAllocate = true);
+                    CountBuffers &b, size_t workBytes = 0, bool mayAllocate = true,
+                    bool optional = false);
 // sortParticles' counting sort; false: not taken (fcdem_count.cu).
 bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int bits);
 // First step of a batch: integrate in each scene's box + hash + count.

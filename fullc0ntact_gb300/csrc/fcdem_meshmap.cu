@@ -23,8 +23,10 @@
 //
 // Both kernels are bound by instruction issue.  The 128-cell map of a torus
 // mesh of 32,768 triangles, host work and the vertices' copy to the host
-// included: 7.7 ms against 128 ms with every pair evaluated (closest points
-// 3.4 ms, solid angles 2.8 ms, signs 0.35 ms); the same bits.
+// included: 6.9 ms against 128 ms with every pair evaluated (closest points
+// 3.3 ms, solid angles 2.8 ms, signs 0.35 ms); the same bits.  Replacing the
+// solid angles of far clusters by those of their area vectors, with a rigorous
+// bound of the error, gained nothing: the clusters are too wide for the bound.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -191,15 +193,25 @@ kMeshNearest(float4 *__restrict__ vert, float *__restrict__ dist, Lattice L, con
   // the first bound: the nearest of the clusters' first vertices, seen from
   // the brick's middle
   float near2 = 3.4e38f;
+  unsigned nearest = 0u;
   for (unsigned c = lane; c < clusters; c += 32) {
     const float4 a = __ldg(tri + 3 * (size_t)c * kCluster);
     if (isinf(__ldg(&box[2 * c].x))) continue;  // a triangle that is not finite
     const float dx = a.x - mid.x, dy = a.y - mid.y, dz = a.z - mid.z;
-    near2 = fminf(near2, dx * dx + dy * dy + dz * dz);
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    if (d2 < near2) {
+      near2 = d2;
+      nearest = c;
+    }
   }
+  {
+    const float own = near2;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    near2 = fminf(near2, __shfl_xor_sync(0xffffffffu, near2, o));
+    for (int o = 16; o > 0; o >>= 1)
+      near2 = fminf(near2, __shfl_xor_sync(0xffffffffu, near2, o));
+    const unsigned who = __ballot_sync(0xffffffffu, own == near2);
+    nearest = __shfl_sync(0xffffffffu, nearest, who ? __ffs((int)who) - 1 : 0);
+  }
   float bound;  // the closest point is no farther than this (plus slack)
   {
     const float dx = p.x - mid.x, dy = p.y - mid.y, dz = p.z - mid.z;
@@ -209,6 +221,29 @@ kMeshNearest(float4 *__restrict__ vert, float *__restrict__ dist, Lattice L, con
   unsigned bestTri = 0xffffffffu;
   float3 bestCp = p;
   float4 *s = sTri[warp];
+  // the closest points of one cluster's triangles
+  auto evaluate = [&](unsigned c) {
+    const unsigned t0 = c * kCluster, cnt = min(kCluster, nt - t0);
+    __syncwarp();
+    for (unsigned e = lane; e < 3 * cnt; e += 32) s[e] = __ldg(tri + 3 * (size_t)t0 + e);
+    __syncwarp();
+    for (unsigned q = 0; q < cnt; ++q) {
+      const float4 a4 = s[3 * q], b4 = s[3 * q + 1], c4 = s[3 * q + 2];
+      const float3 cp = closestOnTriangle(p, make_float3(a4.x, a4.y, a4.z),
+                                          make_float3(b4.x, b4.y, b4.z),
+                                          make_float3(c4.x, c4.y, c4.z));
+      const float dx = p.x - cp.x, dy = p.y - cp.y, dz = p.z - cp.z;
+      const float d2 = dx * dx + dy * dy + dz * dz;
+      const unsigned id = __float_as_uint(a4.w);
+      if (d2 < best || (d2 == best && id < bestTri)) {
+        best = d2;
+        bestTri = id;
+        bestCp = cp;
+      }
+    }
+    bound = fminf(bound, sqrtf(best));
+  };
+  evaluate(nearest);  // most of the bound's slack goes here
   for (unsigned c0 = 0; c0 < clusters; c0 += 32) {
     // 32 clusters against the brick, one a lane
     float far = bound;
@@ -219,7 +254,7 @@ kMeshNearest(float4 *__restrict__ vert, float *__restrict__ dist, Lattice L, con
       const float4 a = __ldg(box + 2 * (c0 + lane)), b = __ldg(box + 2 * (c0 + lane) + 1);
       const float gx = gap(lo.x, hi.x, a.x, b.x), gy = gap(lo.y, hi.y, a.y, b.y),
                   gz = gap(lo.z, hi.z, a.z, b.z);
-      take = !(sqrtf(gx * gx + gy * gy + gz * gz) > far + slack);
+      take = c0 + lane != nearest && !(sqrtf(gx * gx + gy * gy + gz * gz) > far + slack);
     }
     unsigned todo = __ballot_sync(0xffffffffu, take);
     while (todo) {
@@ -229,26 +264,7 @@ kMeshNearest(float4 *__restrict__ vert, float *__restrict__ dist, Lattice L, con
       const float gx = gap(p.x, p.x, a.x, b.x), gy = gap(p.y, p.y, a.y, b.y),
                   gz = gap(p.z, p.z, a.z, b.z);
       const bool need = !(sqrtf(gx * gx + gy * gy + gz * gz) > bound + slack);
-      if (!__any_sync(0xffffffffu, need)) continue;
-      const unsigned t0 = c * kCluster, cnt = min(kCluster, nt - t0);
-      __syncwarp();
-      for (unsigned e = lane; e < 3 * cnt; e += 32) s[e] = __ldg(tri + 3 * (size_t)t0 + e);
-      __syncwarp();
-      for (unsigned q = 0; q < cnt; ++q) {
-        const float4 a4 = s[3 * q], b4 = s[3 * q + 1], c4 = s[3 * q + 2];
-        const float3 cp = closestOnTriangle(p, make_float3(a4.x, a4.y, a4.z),
-                                            make_float3(b4.x, b4.y, b4.z),
-                                            make_float3(c4.x, c4.y, c4.z));
-        const float dx = p.x - cp.x, dy = p.y - cp.y, dz = p.z - cp.z;
-        const float d2 = dx * dx + dy * dy + dz * dz;
-        const unsigned id = __float_as_uint(a4.w);
-        if (d2 < best || (d2 == best && id < bestTri)) {
-          best = d2;
-          bestTri = id;
-          bestCp = cp;
-        }
-      }
-      bound = fminf(bound, sqrtf(best));
+      if (__any_sync(0xffffffffu, need)) evaluate(c);
     }
   }
   if (valid) {
@@ -344,13 +360,14 @@ kMeshSign(float4 *__restrict__ vert, const float *__restrict__ dist, Lattice L, 
 // constant off the surface.  Each directed edge adds a 64-bit hash of its
 // ends with its direction's sign; a mesh with a boundary sums to zero with a
 // probability of 2^-64.
-bool meshClosed(const float *v3, const uint *t3, uint nt) {
+bool meshClosed(const float *v3, uint nv, const uint *t3, uint nt) {
   auto mix = [](unsigned long long z) {
     z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
     z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
     return z ^ (z >> 31);
   };
-  auto vertexHash = [&](uint v) {
+  std::vector<unsigned long long> hash(nv);
+  for (uint v = 0; v < nv; ++v) {
     unsigned long long h = 0x9e3779b97f4a7c15ull;
     for (int a = 0; a < 3; ++a) {
       const float x = v3[3 * (size_t)v + a] + 0.0f;  // -0 and 0 are one place
@@ -358,24 +375,21 @@ bool meshClosed(const float *v3, const uint *t3, uint nt) {
       std::memcpy(&b, &x, 4);
       h = mix(h + b + 0x9e3779b97f4a7c15ull);
     }
-    return h;
-  };
+    hash[v] = h;
+  }
   unsigned long long sum = 0;
-  for (uint t = 0; t < nt; ++t) {
-    unsigned long long h[3];
-    for (int c = 0; c < 3; ++c) h[c] = vertexHash(t3[3 * (size_t)t + c]);
+  for (size_t t = 0; t < nt; ++t)
     for (int c = 0; c < 3; ++c) {
-      const unsigned long long a = h[c], b = h[(c + 1) % 3];
+      const unsigned long long a = hash[t3[3 * t + c]], b = hash[t3[3 * t + (c + 1) % 3]];
       if (a < b) sum += mix(a + 3 * mix(b));
       if (b < a) sum -= mix(b + 3 * mix(a));
     }
-  }
   return sum == 0;
 }
 
 // The map's vertices from the triangles (device, three float4 each).
-bool meshMap(fcdemDistanceMap *m, const float4 *tri, unsigned nt, bool closed, const float lo[3],
-             const float hi[3]) {
+bool meshMap(fcdemDistanceMap *m, const float4 *tri, unsigned nt, const float *vertices3,
+             unsigned nv, const uint *triangles3, const float lo[3], const float hi[3]) {
   const Lattice L{m->cells[0] + 1, m->cells[1] + 1, m->cells[2] + 1,
                   make_float3(m->vmin[0], m->vmin[1], m->vmin[2]), m->cellSize};
   const long long total = (long long)L.vx * L.vy * L.vz;
@@ -414,6 +428,7 @@ bool meshMap(fcdemDistanceMap *m, const float4 *tri, unsigned nt, bool closed, c
   kMeshNearest<<<(unsigned)((bricks + kNearWarps - 1) / kNearWarps), 32 * kNearWarps, 0, st>>>(
       m->vert, dist, L, sorted, nt, box, 1e-5f * extent);
   ok = ok && launchOk();
+  const bool closed = meshClosed(vertices3, nv, triangles3, nt);  // meanwhile
   kMeshRoots<<<vBlocks, 256, 0, st>>>(dist, L, closed, list, count);
   ok = ok && launchOk();
   kMeshWinding<<<numSms() * 4, 32 * kWindWarps, 0, st>>>(L, sorted, nt, list, count, inside);
@@ -479,7 +494,7 @@ extern "C" fcdemDistanceMap *fcdemDistMapFromMesh(const float *vertices3, uint n
   }
   const bool ok =
       cudaOk(cudaMemcpy(dTri, tri.data(), tri.size() * sizeof(float4), cudaMemcpyHostToDevice)) &&
-      meshMap(m, dTri, numTriangles, meshClosed(vertices3, triangles3, numTriangles), lo, hi);
+      meshMap(m, dTri, numTriangles, vertices3, numVertices, triangles3, lo, hi);
   cudaFree(dTri);
   if (!ok) {
     fcdemDistMapDestroy(m);
