@@ -5,12 +5,14 @@
 // Arithmetic order.  The reference sums each neighbour cell's pair terms into
 // a cell subtotal (collideCell) and adds the subtotals in z, y, x order
 // (collideD); within a cell the partners come in ascending sorted index.
-// Both kernels below keep exactly that order, so the float sums are the
+// The kernels below keep exactly that order, so the float sums are the
 // reference's.
 //
-// Two kernels:
+// The kernels:
 //  * kCollideGlobal -- one thread per sorted particle, neighbours read
 //    through the read-only cache (kCollideBatch is the same over many scenes).
+//  * kCollideRows -- nine lanes per particle, for few particles.
+//  * kCollideCrowd -- a warp per group of a crowded cell's members.
 //  * kCollideTiled  -- a CTA takes 128 consecutive sorted particles, splits
 //    them into row groups (same (y, z) grid row), and for each group stages
 //    in shared memory the 9 neighbour-row windows of the cell tables and the
@@ -571,10 +573,9 @@ __device__ __forceinline__ unsigned neighbourhoodCount(int3 g, const CellRanges 
   return total;
 }
 
-// One thread per sorted particle.  Bound by instruction issue and the ALU
-// pipe, then by L1 latency (4.2M spheres at 30% volume fraction, an earlier
-// form of this scan: 67% issue active, ALU 56%, L1 data 55%, DRAM 6%, 17 of
-// 32 lanes).  So the scan spends 8 instructions on a candidate -- one 16-byte
+// One thread per sorted particle.  Bound by instruction issue, then by the L1
+// data path and its latency (4.2M spheres at 30% volume fraction: 76% issue
+// active, 17 of 32 lanes, L1 data 67%, ALU 44%, DRAM 7%).  So the scan spends 8 instructions on a candidate -- one 16-byte
 // load, packed differences, three multiply-adds, one shift that collects the
 // sign -- with no branch and no store per hit, and all table loads go out
 // before it.  Measured against the kernel it replaced (rows copied to shared
@@ -1202,7 +1203,8 @@ void launchT(bool tiled, bool cull, unsigned n, float4 *newVel, const float4 *sp
                                                    ctx().dStatus);
   else {
     CrowdList crowd = crowdList(n);
-    // (on the prefix table the scan has cleared the counters)
+    // on the prefix table the scan has cleared the counters it was given
+    if (kPrefix && crowd.count != out.crowdCount) crowd.groups = nullptr;
     if (!kPrefix && crowd.groups && !cudaOk(cudaMemsetAsync(crowd.count, 0, 8, curStream())))
       crowd.groups = nullptr;
     if (n <= kRowsMax)

@@ -190,6 +190,8 @@ struct CollideOut {
   unsigned *rankOut = nullptr; // mode 2: rank of the particle in its cell count
   unsigned *cnt = nullptr;     // mode 2: per-cell counters (atomic)
   unsigned *tileCnt = nullptr; // mode 2: per-4096-cell-tile counters (atomic)
+  unsigned *crowdCount = nullptr;  // prefix table: the crowded groups' counters, cleared (else
+                                   // none are listed)
   float dt = 0.0f;
 };
 

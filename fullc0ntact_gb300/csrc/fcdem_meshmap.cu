@@ -292,16 +292,16 @@ __device__ __forceinline__ long long signParent(const float *__restrict__ dist, 
 
 // Lists the roots.
 __global__ void __launch_bounds__(256)
-kMeshRoots(const float *__restrict__ dist, Lattice L, bool closed, unsigned *__restrict__ list,
-           unsigned *__restrict__ count) {
+kMeshRoots(const float *__restrict__ dist, Lattice L, bool closed, long long *__restrict__ list,
+           unsigned long long *__restrict__ count) {
   const long long total = (long long)L.vx * L.vy * L.vz;
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool root = v < total && signParent(dist, L, v, closed) < 0;
   const unsigned lane = threadIdx.x & 31u, m = __ballot_sync(0xffffffffu, root);
-  unsigned at = 0;
-  if (lane == 0 && m) at = atomicAdd(count, (unsigned)__popc(m));
+  unsigned long long at = 0;
+  if (lane == 0 && m) at = atomicAdd(count, (unsigned long long)__popc(m));
   at = __shfl_sync(0xffffffffu, at, 0);
-  if (root) list[at + __popc(m & ((1u << lane) - 1u))] = (unsigned)v;
+  if (root) list[at + __popc(m & ((1u << lane) - 1u))] = v;
 }
 
 // inside[v] of the listed roots: 32 roots per CTA at a time, one a lane, the
@@ -309,17 +309,18 @@ kMeshRoots(const float *__restrict__ dist, Lattice L, bool closed, unsigned *__r
 constexpr int kWindWarps = 8;
 __global__ void __launch_bounds__(32 * kWindWarps)
 kMeshWinding(Lattice L, const float4 *__restrict__ tri, unsigned nt,
-             const unsigned *__restrict__ list, const unsigned *__restrict__ count,
+             const long long *__restrict__ list, const unsigned long long *__restrict__ count,
              unsigned char *__restrict__ inside) {
   __shared__ float4 sTri[kWindWarps][3 * kCluster];
   __shared__ float sOmega[kWindWarps][32];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const unsigned n = *count, clusters = (nt + kCluster - 1) / kCluster;
+  const unsigned long long n = *count;
+  const unsigned clusters = (nt + kCluster - 1) / kCluster;
   float4 *s = sTri[warp];
-  for (unsigned base = blockIdx.x * 32u; base < n; base += gridDim.x * 32u) {
-    const unsigned v = __ldg(list + min(base + lane, n - 1u));
-    const float3 p = latticePoint(L, (int)(v % (unsigned)L.vx), (int)(v / (unsigned)L.vx % (unsigned)L.vy),
-                                  (int)(v / ((unsigned)L.vx * (unsigned)L.vy)));
+  for (unsigned long long base = blockIdx.x * 32u; base < n; base += gridDim.x * 32u) {
+    const long long v = __ldg(list + min(base + lane, n - 1ull));
+    const float3 p = latticePoint(L, (int)(v % L.vx), (int)(v / L.vx % L.vy),
+                                  (int)(v / ((long long)L.vx * L.vy)));
     float omega = 0.0f;
     for (unsigned c = warp; c < clusters; c += kWindWarps) {
       const unsigned t0 = c * kCluster, cnt = min(kCluster, nt - t0);
@@ -397,7 +398,7 @@ bool meshMap(fcdemDistanceMap *m, const float4 *tri, unsigned nt, const float *v
   cudaStream_t st = curStream();
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const size_t sortedAt = al((size_t)nt * 8), boxAt = sortedAt + al((size_t)nt * 48),
-               listAt = boxAt + al((size_t)clusters * 32), distAt = listAt + al((size_t)total * 4),
+               listAt = boxAt + al((size_t)clusters * 32), distAt = listAt + al((size_t)total * 8),
                insideAt = distAt + al((size_t)total * 4), countAt = insideAt + al((size_t)total);
   char *buf = nullptr;
   if (cudaMalloc(&buf, countAt + 256) != cudaSuccess) {
@@ -405,8 +406,9 @@ bool meshMap(fcdemDistanceMap *m, const float4 *tri, unsigned nt, const float *v
     setError(FCDEM_ERR_ALLOC);
     return false;
   }
-  unsigned *key = (unsigned *)buf, *order = key + nt, *list = (unsigned *)(buf + listAt);
-  unsigned *count = (unsigned *)(buf + countAt);
+  unsigned *key = (unsigned *)buf, *order = key + nt;
+  long long *list = (long long *)(buf + listAt);
+  unsigned long long *count = (unsigned long long *)(buf + countAt);
   float4 *sorted = (float4 *)(buf + sortedAt), *box = (float4 *)(buf + boxAt);
   float *dist = (float *)(buf + distAt);
   unsigned char *inside = (unsigned char *)(buf + insideAt);
@@ -418,7 +420,7 @@ bool meshMap(fcdemDistanceMap *m, const float4 *tri, unsigned nt, const float *v
     extent = std::fmax(extent, std::fmax(std::fabs(m->vmin[a]), std::fabs(m->vmax[a])));
   const unsigned vBlocks = (unsigned)((total + 255) / 256);
   const long long bricks = (long long)((L.vx + 3) / 4) * ((L.vy + 3) / 4) * ((L.vz + 1) / 2);
-  bool ok = cudaOk(cudaMemsetAsync(count, 0, 4, st));
+  bool ok = cudaOk(cudaMemsetAsync(count, 0, 8, st));
   kMeshKeys<<<(nt + 255) / 256, 256, 0, st>>>(tri, nt, make_float3(lo[0], lo[1], lo[2]), scale, key,
                                              order);
   ok = ok && launchOk();

@@ -307,6 +307,7 @@ void fcdemUpdate(float *pos, float *vel, float *sortedPos, float *sortedVel,
       cells.off = b.off;
       CollideOut out;
       out.posOut = (float4 *)pos;
+      out.crowdCount = crowd;
       if (!last) {
         out.hashOut = hash;
         out.rankOut = b.rank;
@@ -397,6 +398,7 @@ void fcdemUM_update(float *pos, float *vel, float *force, float *sortedPos, floa
     cells.off = b.off;
     CollideOut out;
     out.force = (float3 *)force;
+    out.crowdCount = crowd;
     stageBegin(4);
     launchCollide(0, false, (float4 *)vel, (const float4 *)sortedPos, (const float4 *)sortedVel,
                   index, cells, n, kp, out);
