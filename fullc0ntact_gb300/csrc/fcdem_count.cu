@@ -345,6 +345,11 @@ kScatterCells(const unsigned *hashN, const unsigned *rankN, const unsigned *orig
 // Largest cell that the per-slot re-rank handles (each slot reads every
 // member of its cell).
 constexpr unsigned kFixupMaxCell = 1024;
+// Up to this many particles it handles any cell, and kFixupLarge is not
+// launched: one launch of nine of a small scene's update (2,000 spheres: 28 ->
+// 25.7 us); a cell of all 4,096 costs some 50 us then.
+constexpr unsigned kFixupAllCells = 4096;
+inline unsigned fixupMaxCell(unsigned n) { return n <= kFixupAllCells ? n : kFixupMaxCell; }
 
 // Capacity of the large-cell list: a listed cell has more than kFixupMaxCell
 // of the n particles, so at most n / (kFixupMaxCell + 1) cells are listed.
@@ -353,12 +358,13 @@ inline unsigned largeCapacity(unsigned n) { return n / (kFixupMaxCell + 1) + 1; 
 // Stable order inside each cell + the reorder gather.  The particle of slot
 // s is re-ranked among its cell's members by particle index; its position and
 // velocity are gathered from its entry of the previous order.  A cell above
-// kFixupMaxCell members is appended to large[1..] (large[0] counts) by its
+// maxCell members is appended to large[1..] (large[0] counts) by its
 // first slot and left to kFixupLarge.
 __global__ void __launch_bounds__(256)
 kFixupGather(const uint4 *slots, const unsigned *off, unsigned *hashOut, unsigned *indexOut,
              float4 *sortedPos, float4 *sortedVel, const float4 *prevPos, const float4 *prevVel,
-             unsigned n, unsigned numCells, unsigned *large, unsigned largeCap, unsigned *status) {
+             unsigned n, unsigned numCells, unsigned maxCell, unsigned *large, unsigned largeCap,
+             unsigned *status) {
   chainTrigger();
   chainWait();
   unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -368,7 +374,7 @@ kFixupGather(const uint4 *slots, const unsigned *off, unsigned *hashOut, unsigne
   if (h >= numCells || me >= n || prev >= n || a > s) return;  // unfilled slot (reported)
   const float4 p4 = prevPos[prev], v4 = prevVel[prev];
   const unsigned b = min(off[h + 1], n);
-  if (b - a > kFixupMaxCell) {
+  if (b - a > maxCell) {
     if (s == a) {
       const unsigned k = atomicAdd(large, 1u);
       if (k < largeCap)
@@ -422,7 +428,7 @@ kScatterPairs(const unsigned *keys, const unsigned *vals, const unsigned *rankN,
 
 __global__ void __launch_bounds__(256)
 kFixupPairs(const uint4 *slots, const unsigned *off, unsigned *keys, unsigned *vals, unsigned n,
-            unsigned mask, unsigned *large, unsigned largeCap, unsigned *status) {
+            unsigned mask, unsigned maxCell, unsigned *large, unsigned largeCap, unsigned *status) {
   chainTrigger();
   chainWait();
   const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -430,7 +436,7 @@ kFixupPairs(const uint4 *slots, const unsigned *off, unsigned *keys, unsigned *v
   const uint4 w = slots[s];
   const unsigned h = w.x & mask, a = w.w, b = min(off[h + 1], n);
   if (a > s) return;
-  if (b - a > kFixupMaxCell) {
+  if (b - a > maxCell) {
     if (s == a) {
       const unsigned k = atomicAdd(large, 1u);
       if (k < largeCap)
@@ -949,10 +955,11 @@ bool countPipelineSort(Context &c, const CountBuffers &b, const unsigned *origOf
                 numCells, b.tileCnt, own ? b.scanTiles : 0u, c.dStatus);
   if (!launchOk()) return false;
   launchChained(true, kFixupGather, (n + 255) / 256, 256, 0, b.slots, b.off, hash, index,
-                 sortedPos, sortedVel, prevPos, prevVel, n, numCells, b.large,
+                 sortedPos, sortedVel, prevPos, prevVel, n, numCells,
+                fixupMaxCell(n), b.large,
                 b.largeCap, c.dStatus);
   if (!launchOk()) return false;
-  if (n <= kFixupMaxCell) return true;  // no cell can be large
+  if (n <= kFixupAllCells) return true;  // no cell is left
   // Returns at once when the fix-up listed no cell (the common case).
   const unsigned largeCtas = b.largeCap < numSms() ? b.largeCap : numSms();  // one per SM at most
   launchChained(true, kFixupLarge<false>, largeCtas, kLargeThreads, 0, b.slots, b.off, b.large,
@@ -1004,9 +1011,10 @@ bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int 
   launchChained(true, kScatterPairs, blocks, 256, 0, keys, vals, b.rank, b.off, b.slots, n, mask,
                 b.tileCnt, b.scanTiles);
   if (!launchOk()) return true;
-  launchChained(true, kFixupPairs, blocks, 256, 0, b.slots, b.off, keys, vals, n, mask, b.large,
+  launchChained(true, kFixupPairs, blocks, 256, 0, b.slots, b.off, keys, vals, n, mask,
+                fixupMaxCell(n), b.large,
                 b.largeCap, c.dStatus);
-  if (!launchOk() || n <= kFixupMaxCell) return true;
+  if (!launchOk() || n <= kFixupAllCells) return true;
   const unsigned largeCtas = b.largeCap < numSms() ? b.largeCap : numSms();
   launchChained(true, kFixupLarge<true>, largeCtas, kLargeThreads, 0, b.slots, b.off, b.large,
                 b.largeCap, keys, vals, (float4 *)b.work, nullptr, nullptr, nullptr, n, keyBits(n),
