@@ -187,11 +187,9 @@ fcdemBatch *fcdemBatchCreate(const fcdemBatchScene *scenes, uint numScenes, int 
     freeBatch(b);
     return nullptr;
   }
-  cudaOk(cudaMemcpy(b->scenes, hs.data(), sizeof(BatchScene) * numScenes,
-                    cudaMemcpyHostToDevice));
+  uploadNow(b->scenes, hs.data(), sizeof(BatchScene) * numScenes);
   b->hostScenes = hs;
-  if (b->n)
-    cudaOk(cudaMemcpy(b->sceneOf, sceneOf.data(), 4 * (size_t)b->n, cudaMemcpyHostToDevice));
+  if (b->n) uploadNow(b->sceneOf, sceneOf.data(), 4 * (size_t)b->n);
   CountBuffers cb;  // allocate now: recording a graph must not allocate
   if (!countBuffersIn(b->countBuf, b->countBytes, b->countCells, b->n, b->numCells, cb)) {
     freeBatch(b);
@@ -226,9 +224,7 @@ void fcdemBatchSetObstacles(fcdemBatch *b, const fcdemDistanceMap *const *maps, 
   }
   for (uint s = 0; s < b->numScenes; ++s)
     b->hostScenes[s].shape = numMaps ? sceneShape[s] : -1;
-  if (!cudaOk(cudaMemcpy(b->scenes, b->hostScenes.data(), sizeof(BatchScene) * b->numScenes,
-                         cudaMemcpyHostToDevice)))
-    return;
+  if (!uploadNow(b->scenes, b->hostScenes.data(), sizeof(BatchScene) * b->numScenes)) return;
   b->net = numMaps ? net : nullptr;
   b->skin = skin;
   if (numMaps == 0) return;
@@ -246,8 +242,8 @@ void fcdemBatchSetObstacles(fcdemBatch *b, const fcdemDistanceMap *const *maps, 
     setError(FCDEM_ERR_ALLOC);
     return;
   }
-  cudaOk(cudaMemcpy(b->maps, hv.data(), sizeof(MapView) * numMaps, cudaMemcpyHostToDevice));
-  cudaOk(cudaMemset(b->exact, 0, sizeof(unsigned)));
+  uploadNow(b->maps, hv.data(), sizeof(MapView) * numMaps);
+  clearNow(b->exact, 0, sizeof(unsigned));
 }
 
 unsigned long long fcdemBatchExactQueries(fcdemBatch *b, int reset) {
@@ -255,9 +251,9 @@ unsigned long long fcdemBatchExactQueries(fcdemBatch *b, int reset) {
   if (!b->exact) return 0;
   unsigned v = 0;
   if (!cudaOk(cudaDeviceSynchronize()) ||
-      !cudaOk(cudaMemcpy(&v, b->exact, sizeof(unsigned), cudaMemcpyDeviceToHost)))
+      !downloadNow(&v, b->exact, sizeof(unsigned)))
     return 0;
-  if (reset) cudaOk(cudaMemset(b->exact, 0, sizeof(unsigned)));
+  if (reset) clearNow(b->exact, 0, sizeof(unsigned));
   return v;
 }
 

@@ -75,6 +75,19 @@ bool launchOk() {
   return cudaOk(cudaGetLastError());
 }
 
+bool uploadNow(void *device, const void *host, size_t bytes) {
+  return cudaOk(cudaMemcpyAsync(device, host, bytes, cudaMemcpyHostToDevice, t_stream)) &&
+         cudaOk(cudaStreamSynchronize(t_stream));
+}
+bool downloadNow(void *host, const void *device, size_t bytes) {
+  return cudaOk(cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, t_stream)) &&
+         cudaOk(cudaStreamSynchronize(t_stream));
+}
+bool clearNow(void *device, int byte, size_t bytes) {
+  return cudaOk(cudaMemsetAsync(device, byte, bytes, t_stream)) &&
+         cudaOk(cudaStreamSynchronize(t_stream));
+}
+
 Context &ctx() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
@@ -223,17 +236,12 @@ void copyArrayFromDevice(void *host, const void *device,
     return;
   }
   if (size < 0) { setError(FCDEM_ERR_INVALID_VALUE); return; }
-  cudaStream_t s = curStream();
-  if (cudaOk(cudaMemcpyAsync(host, device, (size_t)size, cudaMemcpyDeviceToHost, s)))
-    cudaOk(cudaStreamSynchronize(s));
+  downloadNow(host, device, (size_t)size);
 }
 
 void copyArrayToDevice(void *device, const void *host, int offset, int size) {
   if (size < 0 || offset < 0) { setError(FCDEM_ERR_INVALID_VALUE); return; }
-  cudaStream_t s = curStream();
-  if (cudaOk(cudaMemcpyAsync((char *)device + offset, host, (size_t)size,
-                             cudaMemcpyHostToDevice, s)))
-    cudaOk(cudaStreamSynchronize(s));
+  uploadNow((char *)device + offset, host, (size_t)size);
 }
 
 void registerGLBufferObject(uint, struct cudaGraphicsResource **) {

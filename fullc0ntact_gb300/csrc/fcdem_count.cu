@@ -851,12 +851,14 @@ bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsi
       if (!optional) setError(FCDEM_ERR_ALLOC);
       return false;
     }
-    bytes = need;
-    cells = numCells;
-    if (!cudaOk(cudaMemset(buf, 0, need))) return false;  // cnt starts at zero
-    // no tile's offsets are known yet (see scanTile)
+    // cnt starts at zero, and no tile's offsets are known yet (see scanTile);
+    // done when this returns, so that any stream may use the buffer next
     const size_t prevAt = 2 * al(m * 4) + 2 * al((size_t)(tiles + 1) * 4);
-    if (!cudaOk(cudaMemset((char *)buf + prevAt, 0xff, (size_t)(tiles + 1) * 4))) return false;
+    if (!clearNow(buf, 0, need) ||
+        !clearNow((char *)buf + prevAt, 0xff, (size_t)(tiles + 1) * 4))
+      return false;
+    bytes = need;  // the buffer counts from here on
+    cells = numCells;
   }
   // The arrays that must stay zero between calls (cnt, tileCnt) sit first,
   // at offsets that depend on the cell count only, so that a call with

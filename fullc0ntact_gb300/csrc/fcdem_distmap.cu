@@ -227,10 +227,10 @@ fcdemDistanceMap *fcdemDistMapCreate(const float *distance, const float *contact
     for (size_t v = 0; v < nv; ++v)
       h[v] = make_float4(distance[v], contactPoints[3 * v], contactPoints[3 * v + 1],
                          contactPoints[3 * v + 2]);
-    cudaOk(cudaMemcpy(m->vert, h, nv * sizeof(float4), cudaMemcpyHostToDevice));
+    uploadNow(m->vert, h, nv * sizeof(float4));
     std::free(h);
   } else {
-    cudaOk(cudaMemset(m->vert, 0, nv * sizeof(float4)));
+    clearNow(m->vert, 0, nv * sizeof(float4));
   }
   return m;
 }
@@ -315,7 +315,7 @@ void fcdemDistMapGeometry(const fcdemDistanceMap *m, float vmin[3], float vmax[3
 void fcdemDistMapVertices(const fcdemDistanceMap *m, float *vertices4) {
   if (!m || !vertices4) { setError(FCDEM_ERR_INVALID_VALUE); return; }
   const size_t nv = (size_t)(m->cells[0] + 1) * (m->cells[1] + 1) * (m->cells[2] + 1);
-  cudaOk(cudaMemcpy(vertices4, m->vert, nv * sizeof(float4), cudaMemcpyDeviceToHost));
+  downloadNow(vertices4, m->vert, nv * sizeof(float4));
 }
 
 void fcdemDistMapQuery(const fcdemDistanceMap *m, const float *queries4, unsigned n,

@@ -112,9 +112,7 @@ void cuda_init(i3d::HashGrid<float, i3d::cpu> &hg, i3d::ParticleWorld<float, i3d
       !deviceAlloc(pw.sortedPos_, 4 * n) || !deviceAlloc(pw.sortedVel_, 4 * n))
     return;
   i3d::SimulationParameters<float> *dev = nullptr;
-  if (!deviceAlloc(dev, 1) || !cudaOk(cudaMemcpy(dev, pw.params_, sizeof(*dev),
-                                                 cudaMemcpyHostToDevice)))
-    return;
+  if (!deviceAlloc(dev, 1) || !uploadNow(dev, pw.params_, sizeof(*dev))) return;
   params = dev;
   {
     std::lock_guard<std::mutex> lock(g_i3dMutex);
@@ -151,8 +149,8 @@ void cuda_init(i3d::HashGrid<float, i3d::cpu> &hg, i3d::ParticleWorld<float, i3d
         pos[4 * i + 3] = 1.0f;
       }
   if (n) {
-    cudaOk(cudaMemcpy(pw.pos_, pos.data(), 16 * n, cudaMemcpyHostToDevice));
-    cudaOk(cudaMemcpy(pw.vel_, vel.data(), 16 * n, cudaMemcpyHostToDevice));
+    uploadNow(pw.pos_, pos.data(), 16 * n);
+    uploadNow(pw.vel_, vel.data(), 16 * n);
   }
 }
 

@@ -92,6 +92,14 @@ bool cudaOk(cudaError_t e);
 // Checks (and counts) the launch that was just issued.
 bool launchOk();
 
+// Copies and clears that are complete when they return, ordered after the work
+// on the library stream.  (cudaMemset, and cudaMemcpy from pageable memory, go
+// to the legacy default stream and may return before they have run; a
+// non-blocking stream does not wait for it.)
+bool uploadNow(void *device, const void *host, size_t bytes);
+bool downloadNow(void *host, const void *device, size_t bytes);
+bool clearNow(void *device, int byte, size_t bytes);
+
 // Chained launches.  launchChained(true, ...) issues a kernel that may start
 // while the kernel before it on the stream is still running (programmatic
 // stream serialisation), so that its launch latency and its prologue overlap

@@ -495,7 +495,7 @@ extern "C" fcdemDistanceMap *fcdemDistMapFromMesh(const float *vertices3, uint n
     return nullptr;
   }
   const bool ok =
-      cudaOk(cudaMemcpy(dTri, tri.data(), tri.size() * sizeof(float4), cudaMemcpyHostToDevice)) &&
+      uploadNow(dTri, tri.data(), tri.size() * sizeof(float4)) &&
       meshMap(m, dTri, numTriangles, vertices3, numVertices, triangles3, lo, hi);
   cudaFree(dTri);
   if (!ok) {

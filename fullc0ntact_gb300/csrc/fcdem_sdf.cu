@@ -1145,7 +1145,7 @@ bool uploadParams(fcdemSdfNet *net, const std::vector<float> &p) {
   const size_t bytes = sizeof(float) * p.size();
   net->w16Fresh = false;
   net->version++;
-  return cudaOk(cudaMemcpy(net->params, p.data(), bytes, cudaMemcpyHostToDevice));
+  return uploadNow(net->params, p.data(), bytes);
 }
 
 template <int H, int L>
@@ -1359,7 +1359,7 @@ unsigned char *sdfHints(fcdemSdfNet *net, unsigned tiles) {
     net->hints = nullptr;
     return nullptr;
   }
-  if (!cudaOk(cudaMemset(net->hints, 0, tiles))) return nullptr;
+  if (!clearNow(net->hints, 0, tiles)) return nullptr;
   net->hintTiles = tiles;
   return net->hints;
 }
@@ -1542,8 +1542,7 @@ fcdemSdfNet *fcdemSdfCreate(int inputs, int hidden, int hiddenLayers, unsigned l
   fill(ly.w0, (unsigned)(ly.H * ly.D), 3);
   for (int l = 1; l < ly.L; ++l) fill(ly.wh[l - 1], (unsigned)(ly.H * ly.H), ly.H);
   fill(ly.wo, (unsigned)ly.H, ly.H);
-  if (!uploadParams(net, p) || !cudaOk(cudaMemset(net->m, 0, bytes)) ||
-      !cudaOk(cudaMemset(net->v, 0, bytes))) {
+  if (!uploadParams(net, p) || !clearNow(net->m, 0, bytes) || !clearNow(net->v, 0, bytes)) {
     freeNet(net);
     return nullptr;
   }
@@ -1556,7 +1555,7 @@ uint fcdemSdfNumParams(const fcdemSdfNet *net) { return net ? net->lay.total : 0
 
 void fcdemSdfGetParams(const fcdemSdfNet *net, float *host) {
   if (!net || !host) { setError(FCDEM_ERR_INVALID_VALUE); return; }
-  cudaOk(cudaMemcpy(host, net->params, sizeof(float) * net->lay.total, cudaMemcpyDeviceToHost));
+  downloadNow(host, net->params, sizeof(float) * net->lay.total);
 }
 
 void fcdemSdfSetParams(fcdemSdfNet *net, const float *host) {
@@ -1622,9 +1621,8 @@ float fcdemSdfGradient(fcdemSdfNet *net, const float *samples4, const int *shape
       !reducePartials(net, parts, -1.0f))
     return 0.0f;
   float loss = 0.0f;
-  cudaOk(cudaStreamSynchronize(curStream()));
-  cudaOk(cudaMemcpy(&loss, net->loss, sizeof(float), cudaMemcpyDeviceToHost));
-  if (gradHost) cudaOk(cudaMemcpy(gradHost, net->grad, bytes, cudaMemcpyDeviceToHost));
+  downloadNow(&loss, net->loss, sizeof(float));
+  if (gradHost) downloadNow(gradHost, net->grad, bytes);
   return loss;
 }
 
@@ -1653,8 +1651,7 @@ float fcdemSdfTrainSamples(fcdemSdfNet *net, const float *samples4, const int *s
         return 0.0f;
     }
     if (e + 1 == epochs) {
-      cudaOk(cudaStreamSynchronize(curStream()));
-      cudaOk(cudaMemcpy(&last, net->loss, sizeof(float), cudaMemcpyDeviceToHost));
+      downloadNow(&last, net->loss, sizeof(float));
       last /= (float)batches;
     }
   }

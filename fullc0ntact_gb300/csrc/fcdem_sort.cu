@@ -487,7 +487,7 @@ unsigned char *noAllocScratch() {
       setError(FCDEM_ERR_CUDA);
       return nullptr;
     }
-    if (!cudaOk(cudaMemset(statusIn((unsigned char *)p), 0, sizeof(unsigned)))) return nullptr;
+    if (!clearNow(statusIn((unsigned char *)p), 0, sizeof(unsigned))) return nullptr;
     g_noAllocPtr[dev] = (unsigned char *)p;
   }
   return g_noAllocPtr[dev];
