@@ -148,7 +148,7 @@ unsigned numSms() {
   return 152u;  // GB300 (not reached on a working device)
 }
 
-void *scratch(Context &c, size_t bytes) {
+void *scratch(Context &c, size_t bytes, bool optional) {
   if (bytes <= c.scratchBytes) return c.scratch;
   // Work already queued (on any stream) may still use the old block.
   if (!cudaOk(cudaDeviceSynchronize())) return nullptr;
@@ -159,7 +159,7 @@ void *scratch(Context &c, size_t bytes) {
   if (cudaMalloc(&c.scratch, grown) != cudaSuccess) {
     cudaGetLastError();
     c.scratch = nullptr;
-    setError(FCDEM_ERR_ALLOC);
+    if (!optional) setError(FCDEM_ERR_ALLOC);
     return nullptr;
   }
   c.scratchBytes = grown;

@@ -830,7 +830,7 @@ static bool countBuffers(Context &c, unsigned n, unsigned numCells, CountBuffers
 }
 
 bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsigned numCells,
-                    CountBuffers &b, size_t workBytes, bool mayAllocate, bool optional) {
+                    CountBuffers &b) {
   const size_t m = (size_t)numCells + 1;
   const unsigned tiles = (unsigned)((m + kScanTile - 1) / kScanTile);
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
@@ -838,9 +838,8 @@ bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsi
   const unsigned tileBlocks = (tiles + kTileBlock - 1) / kTileBlock;
   const size_t need = 2 * al(m * 4) + al((size_t)n * 4) + al((size_t)n * 16) + 3 * al((size_t)(tiles + 1) * 4) +
                       al(((size_t)largeCap + 1) * 4) + al((size_t)tileBlocks * 4) +
-                      al((size_t)kBitmapSlots * 2 * bitmapWords(n) * 4) + al(workBytes);
+                      al((size_t)kBitmapSlots * 2 * bitmapWords(n) * 4);
   if (buf == nullptr || bytes < need || cells != numCells) {
-    if (!mayAllocate) return false;
     if (!cudaOk(cudaDeviceSynchronize())) return false;
     if (buf) cudaFree(buf);
     buf = nullptr;
@@ -848,7 +847,7 @@ bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsi
     if (cudaMalloc(&buf, need) != cudaSuccess) {
       cudaGetLastError();
       buf = nullptr;
-      if (!optional) setError(FCDEM_ERR_ALLOC);
+      setError(FCDEM_ERR_ALLOC);
       return false;
     }
     // cnt starts at zero, and no tile's offsets are known yet (see scanTile);
@@ -884,8 +883,7 @@ bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsi
   b.tileBlockSum = (unsigned *)p;
   p += al((size_t)tileBlocks * 4);
   b.bitmaps = (unsigned *)p;  // cleared where used (kFixupLarge)
-  p += al((size_t)kBitmapSlots * 2 * bitmapWords(n) * 4);
-  b.work = p;
+  b.work = nullptr;
   b.scanTiles = tiles;
   return true;
 }
@@ -970,10 +968,68 @@ bool countPipelineSort(Context &c, const CountBuffers &b, const unsigned *origOf
   return launchOk();
 }
 
-// Keys of at most this many bits are counted: 4096 tiles, whose counts
-// kScanCellsOwn sums itself.
-constexpr int kCountSortBits = 24;
+static_assert(((1u << kCountSortBits) >> kTileShift) + 1 <= kTilesOwnPrefix, "tiles of a key width");
 constexpr unsigned kCountSortMax = 1u << 21;  // pairs
+
+// Buffers of countSortPairs.  A recorded graph may hold their addresses, so
+// they live as long as those of the radix sort: each key width has its own
+// cell tables (8 * 2^bits bytes: 134 MB at 24 bits, twice that over all
+// widths), which are got once and never moved, and what belongs to the pairs is
+// in the scratch block, which only grows with the number of pairs.  That block
+// is taken large enough for the radix sort too, which can then step in while a
+// graph is captured at a key width that has no tables yet.  False, without an
+// error: nothing to be had (or to be got during a capture).
+static bool sortBuffers(Context &c, unsigned n, int bits, CountBuffers &b) {
+  auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t m = ((size_t)1 << bits) + 1;
+  const unsigned tiles = (unsigned)((m + kScanTile - 1) / kScanTile);
+  const unsigned largeCap = largeCapacity(n);
+  const size_t cellBytes = al(m * 4), tileBytes = al((size_t)tiles * 4);
+  const size_t rankBytes = al((size_t)n * 4), slotBytes = al((size_t)n * 16),
+               largeBytes = al(((size_t)largeCap + 1) * 4);
+  const size_t pairBytes = std::max(rankBytes + 2 * slotBytes + largeBytes +
+                                        (size_t)kBitmapSlots * 2 * bitmapWords(n) * 4,
+                                    radixScratchBytes(n));
+  void *&tables = c.sortTables[bits];
+  if (!tables || c.scratchBytes < pairBytes) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(curStream(), &cap) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    if (cap != cudaStreamCaptureStatusNone) return false;
+  }
+  if (!tables) {
+    void *got = nullptr;
+    if (cudaMalloc(&got, 2 * (cellBytes + tileBytes)) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    // the counts start at zero, and no tile's offsets are known yet (scanTile)
+    if (!clearNow(got, 0, 2 * cellBytes + tileBytes) ||
+        !clearNow((char *)got + 2 * cellBytes + tileBytes, 0xff, tileBytes)) {
+      cudaFree(got);
+      return false;
+    }
+    tables = got;
+  }
+  char *p = (char *)scratch(c, pairBytes, true);
+  if (!p) return false;
+  char *t = (char *)tables;
+  b = CountBuffers{};
+  b.cnt = (unsigned *)t;
+  b.off = (unsigned *)(t + cellBytes);
+  b.tileCnt = (unsigned *)(t + 2 * cellBytes);
+  b.tileOffPrev = (unsigned *)(t + 2 * cellBytes + tileBytes);
+  b.scanTiles = tiles;
+  b.slots = (uint4 *)p;
+  b.work = p + slotBytes;
+  b.rank = (unsigned *)(p + 2 * slotBytes);
+  b.large = (unsigned *)(p + 2 * slotBytes + rankBytes);
+  b.largeCap = largeCap;
+  b.bitmaps = (unsigned *)(p + 2 * slotBytes + rankBytes + largeBytes);
+  return true;
+}
 
 // sortParticles' stable sort of n (key, value) pairs by the low `bits` bits as
 // a counting sort over 2^bits cells, in place; keys with higher bits raise
@@ -983,21 +1039,13 @@ constexpr unsigned kCountSortMax = 1u << 21;  // pairs
 // bits, whose chain over the tiles is what they wait for.  A staged step with
 // it / with the radix sort: 5,000 spheres 39 / 60 us, 100,003 75 / 89, 1M in
 // lattice order 159 / 204, 1M in random order 245 / 252, 4.2M 901 / 892 (hence
-// the bound).  Its buffers are its own (a fused step
-// on another stream keeps its counts); while a graph is captured they are not
-// grown.
+// the bound).  The fused step's buffers are others: it may run on another
+// stream.
 bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int bits) {
   if (bits > kCountSortBits || n > kCountSortMax) return false;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(curStream(), &cap) != cudaSuccess) {
-    cudaGetLastError();
-    cap = cudaStreamCaptureStatusActive;
-  }
   const unsigned cells = 1u << bits, mask = cells - 1u;
   CountBuffers b;
-  if (!countBuffersIn(c.sortBuf, c.sortBytes, c.sortCells, n, cells, b, 16 * (size_t)n,
-                      cap == cudaStreamCaptureStatusNone, true))
-    return false;
+  if (!sortBuffers(c, n, bits, b)) return false;
   const unsigned blocks = (n + 255) / 256;
   const bool tiles = n <= kTileAtomicsMax;
   launchChained(true, tiles ? kCountKeys<true> : kCountKeys<false>, blocks, 256, 0, keys, n, mask,

@@ -44,6 +44,10 @@ struct KParams {
 };
 
 // Per-device library state.
+// sortParticles counts keys of at most this many bits: 4096 tiles of cells,
+// whose counts kScanCellsOwn sums itself.
+constexpr int kCountSortBits = 24;
+
 struct Context {
   int device = -1;
   bool haveParams = false;
@@ -57,9 +61,9 @@ struct Context {
   void *countBuf = nullptr;     // counting-sort pipeline of fcdemUpdate
   size_t countBytes = 0;
   unsigned countCells = 0;
-  void *sortBuf = nullptr;      // counting sort of sortParticles
-  size_t sortBytes = 0;
-  unsigned sortCells = 0;
+  // counting sort of sortParticles: cell tables per key width, never freed
+  // (what belongs to the pairs is in scratch)
+  void *sortTables[kCountSortBits + 1] = {};
   void *crowdBuf = nullptr;     // collide: groups of crowded particles
   unsigned crowdCap = 0;        // particles the group list covers
 };
@@ -140,7 +144,8 @@ inline void launchChained(bool chained, void (*kernel)(Params...), unsigned bloc
 void stageBegin(int stage);
 void stageEnd(int stage);
 // Returns scratch of at least `bytes` bytes (256-byte aligned) or nullptr.
-void *scratch(Context &c, size_t bytes);
+// optional: no error when it cannot be had.
+void *scratch(Context &c, size_t bytes, bool optional = false);
 
 KParams kparams(const Context &c);
 // Flags of the library's parameter copies, in maxParticlesPerCell (unused by
@@ -166,6 +171,8 @@ inline int keyBits(unsigned numCells) {
 // are 0..n-1 and are not read.  Defined in fcdem_sort.cu.
 void radixSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n,
                     int bits, bool identityVals = false);
+// The most scratch that n pairs can need there.
+size_t radixScratchBytes(unsigned n);
 
 // Cell-table fill (cellStart = 0xffffffff).  Defined in fcdem_stages.cu.
 void fillU32(Context &c, unsigned *p, size_t count, unsigned value);
@@ -244,7 +251,7 @@ struct CountBuffers {
   unsigned *tileOffPrev;        // per tile: the constant its offsets hold, or 0xffffffff
   unsigned *large;              // [0] = count, [1..largeCap] = cells too full for the re-rank
   unsigned *tileBlockSum;       // per 1024 tiles: their total (many-tile scans)
-  void *work;                   // countBuffersIn's extra work space
+  void *work;                   // countSortPairs: 16 bytes of work space per pair
   unsigned *bitmaps;            // kFixupLarge: per-CTA bitmap + word prefix of particle indices
   unsigned scanTiles, largeCap;
 };
@@ -252,11 +259,8 @@ bool countPipelineBegin(Context &c, float4 *pos, float4 *vel, float dt, unsigned
                         unsigned n, unsigned numCells, const KParams &kp, CountBuffers &b);
 // Buffers over explicit storage (a batch owns its own); cnt/tileCnt must be
 // zero on first use.
-// workBytes: extra work space (CountBuffers::work).  mayAllocate false: only
-// buffers that are there already.  optional: no error when they cannot be had.
 bool countBuffersIn(void *&buf, size_t &bytes, unsigned &cells, unsigned n, unsigned numCells,
-                    CountBuffers &b, size_t workBytes = 0, bool mayAllocate = true,
-                    bool optional = false);
+                    CountBuffers &b);
 // sortParticles' counting sort; false: not taken (fcdem_count.cu).
 bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int bits);
 // First step of a batch: integrate in each scene's box + hash + count.

@@ -371,6 +371,29 @@ inline size_t alignUp(size_t v) { return (v + 255) & ~(size_t)255; }
 
 }  // namespace
 
+// The parts of the radix sort's scratch for n pairs and `passes` passes with
+// tiles of `tileKeys` keys.
+struct RadixScratch {
+  size_t arr, hist, lookback;
+  int buffers;  // extra key/value pairs
+  RadixScratch(unsigned n, int passes, int tileKeys)
+      : arr(alignUp((size_t)n * 4)),
+        hist(alignUp(kMaxPasses * kRadix * 4 + kMaxPasses * 4)),
+        lookback(alignUp((size_t)passes * ((n + tileKeys - 1) / tileKeys) * kRadix * 4)),
+        buffers(passes % 2 == 1 ? 2 : 1) {}
+  size_t total() const { return (size_t)buffers * 2 * arr + hist + lookback; }
+};
+
+size_t radixScratchBytes(unsigned n) {
+  size_t most = 0;
+  for (int passes = 1; passes <= kMaxPasses; ++passes)
+    for (const PassConfig &pc : kPassConfigs) {
+      const size_t b = RadixScratch(n, passes, pc.tile()).total();
+      if (b > most) most = b;
+    }
+  return most;
+}
+
 void radixSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n,
                     int bits, bool identityVals) {
   if (n < 2) return;
@@ -381,12 +404,10 @@ void radixSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n,
   const PassConfig &pc = chooseConfig(n);
   if (!prepareConfig(pc)) return;
   const unsigned tiles = (n + pc.tile() - 1) / pc.tile();
-  const size_t arr = alignUp((size_t)n * 4);
-  const size_t histBytes = alignUp(kMaxPasses * kRadix * 4 + kMaxPasses * 4);
-  const size_t lbBytes = alignUp((size_t)passes * tiles * kRadix * 4);
-  const int buffers = (passes % 2 == 1) ? 2 : 1;  // extra key/value pairs
-  const size_t total = (size_t)buffers * 2 * arr + histBytes + lbBytes;
-  char *s = (char *)scratch(c, total);
+  const RadixScratch r(n, passes, pc.tile());
+  const size_t arr = r.arr, histBytes = r.hist, lbBytes = r.lookback;
+  const int buffers = r.buffers;
+  char *s = (char *)scratch(c, r.total());
   if (!s) return;
   unsigned *kB = (unsigned *)s, *vB = (unsigned *)(s + arr);
   unsigned *kC = buffers > 1 ? (unsigned *)(s + 2 * arr) : nullptr;

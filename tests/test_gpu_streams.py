@@ -83,3 +83,60 @@ def test_maps_and_networks_made_on_a_side_stream(side):
         mesh, dem.DistanceMap.from_mesh(*scenes.torus_mesh(0.3, 0.1, 48, 24), 48, 0.05).vertices())
     np.testing.assert_array_equal(a, sdf.SdfNet(3, 64, 3, seed=5).get_params())
     dem.set_stream(side)
+
+
+def _cpu(keys, vals):
+    o = np.argsort(keys, kind="stable")
+    return keys[o], vals[o]
+
+
+def test_sorts_of_alternating_cell_counts():
+    """Two grids in one process, and sizes that grow and shrink between them."""
+    rng = np.random.default_rng(17)
+    for n, cells in [(3000, 2 ** 12), (70_000, 2 ** 20), (3000, 2 ** 20), (300_000, 2 ** 12),
+                     (70_000, 2 ** 15), (300_000, 2 ** 20), (10, 2 ** 12), (300_000, 2 ** 12),
+                     (300_001, 3 * 2 ** 18), (70_000, 2 ** 20), (5000, 1), (300_000, 2 ** 15)]:
+        keys = rng.integers(0, cells, n).astype(np.uint32)
+        vals = rng.permutation(n).astype(np.uint32)
+        k, v = _sort(keys, vals, cells)
+        rk, rv = _cpu(keys, vals)
+        np.testing.assert_array_equal(k, rk)
+        np.testing.assert_array_equal(v, rv)
+
+
+@pytest.mark.parametrize("n", [4000, 60_000, 300_000])
+@pytest.mark.parametrize("warm", [2 ** 19, 2 ** 14])
+def test_captured_sort_outlives_sorts_of_other_cell_counts(side, n, warm):
+    """A recorded sortParticles replays correctly after sorts with smaller and
+    larger cell counts.  warm = 2^14: the key width is first met (or not) during
+    the capture, after a warm-up call at another one."""
+    from fullc0ntact_gb300 import dem
+    from fullc0ntact_gb300.params import make_params
+    cells = 2 ** 19 if n != 4000 else 2 ** 17
+    rng = np.random.default_rng(n + warm)
+    draw = lambda: (rng.integers(0, cells, n).astype(np.uint32), rng.permutation(n).astype(np.uint32))
+    dev = lambda a: torch.from_numpy(a.view(np.int32)).cuda()
+    warm = min(warm, cells)
+    _sort(rng.integers(0, warm, n).astype(np.uint32), np.arange(n, dtype=np.uint32), warm)
+    P = make_params(n, (2, 2, 2), 0.01)
+    P.numCells = cells
+    dem.set_parameters(P)
+    keys, vals = draw()
+    k, v = dev(keys), dev(vals)
+    side.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=side):
+        dem.sort_particles(k, v, n)
+    for other in (2 ** 9, 2 ** 21, cells):
+        ok, ov = rng.integers(0, other, n).astype(np.uint32), np.arange(n, dtype=np.uint32)
+        gk, gv = _sort(ok, ov, other)
+        np.testing.assert_array_equal(gv, _cpu(ok, ov)[1])
+        keys, vals = draw()
+        k.copy_(dev(keys))
+        v.copy_(dev(vals))
+        g.replay()
+        side.synchronize()
+        dem.check("replay")
+        rk, rv = _cpu(keys, vals)
+        np.testing.assert_array_equal(k.cpu().numpy().view(np.uint32), rk)
+        np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), rv)
