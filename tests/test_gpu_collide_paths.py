@@ -5,6 +5,7 @@ multi-row tiles, x-wrapping windows, crowded cells, inert particles and the
 polydisperse mode."""
 import numpy as np
 import pytest
+import torch
 
 pytestmark = pytest.mark.gpu
 
@@ -315,3 +316,52 @@ def test_row_scan_edges_match_oracle(grid, n, kind, poly, many):
         finally:
             dem.lib.fcdemSetCrowdPath(1)
             dem.set_radius_mode(False)
+
+
+@pytest.mark.parametrize("poly", [False, True])
+@pytest.mark.parametrize("n", [6000, 40_000])
+@pytest.mark.parametrize("grid", [(32, 32, 32), (8, 16, 32)])
+def test_particles_moved_across_a_face_after_the_sort(grid, n, poly):
+    """A staged host may move particles between calcHash and collide: the tables
+    then list a particle in a neighbour of the cell that its position gives
+    (every row and every part of a wrapped row).  It never meets itself there:
+    bit-exact against the oracle, with one thread and with nine lanes per
+    particle."""
+    from fullc0ntact_gb300 import dem, scenes
+    from oracle import oracle as O
+    cell = 1.0 / 16.0
+    sc = scenes.random_box(n, grid=grid, radius=1.0 / 64.0, seed=n + grid[0], cell=cell, poly=poly)
+    rng = np.random.default_rng(5)
+    pos, vel = sc["pos"], sc["vel"]
+    pos[:, :3] = -1.0 + rng.uniform(0.0, 1.0, (n, 3)) * np.array(grid) * cell
+    # a quarter of them just below a face on some axes, the world's edges among the
+    # faces, then just above it (by less than the margin of the cell culling)
+    some = rng.permutation(n)[: n // 4]
+    axes = rng.random((len(some), 3)) < 0.5
+    face = -1.0 + rng.integers(0, np.array(grid) + 1, (len(some), 3)) * cell
+    step = rng.uniform(1e-7, 1e-6, (2, len(some), 3))
+    moved = pos.copy()
+    pos[some, :3] = np.where(axes, face - step[0], pos[some, :3])
+    moved[some, :3] = np.where(axes, face + step[1], pos[some, :3])
+    P = O.SimParams.from_buffer_copy(bytes(sc["params"]))
+    with O.gpu_arithmetic():
+        h, x = O.sort_pairs(*O.calc_hash(P, pos))
+        cs, ce, sp, sv = O.reorder(h, x, moved, vel, P.numCells)
+        want = O.collide(P, sp, sv, x, cs, ce, radius_from_w=poly)
+    ds = dem.DeviceScene(sc)
+    ds.activate()
+    try:
+        dem.calc_hash(ds.hash, ds.index, ds.pos, n)
+        dem.sort_particles(ds.hash, ds.index, n)
+        ds.pos.copy_(torch.from_numpy(moved))
+        dem.reorder_data_and_find_cell_start(ds.cell_start, ds.cell_end, ds.sorted_pos,
+                                             ds.sorted_vel, ds.hash, ds.index, ds.pos, ds.vel, n,
+                                             ds.num_cells)
+        out = torch.empty_like(ds.vel)
+        dem.collide(out, ds.sorted_pos, ds.sorted_vel, ds.index, ds.cell_start, ds.cell_end, n,
+                    ds.num_cells)
+        dem.check("collide")
+    finally:
+        dem.set_radius_mode(False)
+    assert np.isfinite(want).all()
+    np.testing.assert_array_equal(out.cpu().numpy(), want)
