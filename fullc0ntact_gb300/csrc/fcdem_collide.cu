@@ -578,6 +578,18 @@ __device__ __forceinline__ unsigned neighbourhoodCount(int3 g, const CellRanges 
   return total;
 }
 
+// Whether the group of particle i, a member of cell h whose range begins at
+// slot a, is listed: its first member does that, if its position is in the cell
+// too (a staged host may have moved it out after the sort).
+template <bool kPrefix>
+__device__ __forceinline__ bool groupListed(unsigned i, unsigned a, unsigned h,
+                                            const float4 *sortedPos, const SimParams &P) {
+  if (kPrefix) return true;
+  const float4 q = sortedPos[i - ((i - a) & 31u)];
+  const int3 g = gridPos(q.x, q.y, q.z, P);
+  return gridHash(g.x, g.y, g.z, P) == h;
+}
+
 // One thread per sorted particle.  Bound by instruction issue, then by the L1
 // data path and its latency (4.2M spheres at 30% volume fraction: 76% issue
 // active, 17 of 32 lanes, L1 data 67%, ALU 44%, DRAM 7%).  So the scan spends 8 instructions on a candidate -- one 16-byte
@@ -623,8 +635,10 @@ kCollideGlobal(float4 *__restrict__ newVel, const float4 *__restrict__ sortedPos
     if (edge == 2) total = neighbourhoodCount<kPrefix>(g, cells, n, P);
     if (total > crowd.limit) {
       unsigned a, b;
-      cellRange<kPrefix>(gridHash(g.x, g.y, g.z, P), cells, n, a, b);
-      if (i >= a && i < b) {  // deferred to kCollideCrowd
+      const unsigned h = gridHash(g.x, g.y, g.z, P);
+      cellRange<kPrefix>(h, cells, n, a, b);
+      if (i >= a && i < b && groupListed<kPrefix>(i, a, h, sortedPos, P)) {
+        // deferred to kCollideCrowd
         if (((i - a) & 31u) == 0u) {
           const unsigned k = atomicAdd(crowd.count, 1u);
           if (k < crowd.cap) crowd.groups[k] = make_uint2(i, min(32u, b - i));
@@ -711,9 +725,10 @@ kCollideRows(float4 *newVel, const float4 *sortedPos, const float4 *sortedVel,
       for (int k = 0; k < 9; ++k) all += sTotal[warp][who][k];
     if (all > crowd.limit) {
       unsigned c0, c1;
-      cellRange<kPrefix, true>(gridHash(g.x, g.y, g.z, P), cells, n, c0, c1);
-      if (i >= c0 && i < c1) {  // deferred to kCollideCrowd
-        deferred = true;
+      const unsigned h = gridHash(g.x, g.y, g.z, P);
+      cellRange<kPrefix, true>(h, cells, n, c0, c1);
+      if (i >= c0 && i < c1 && groupListed<kPrefix>(i, c0, h, sortedPos, P)) {
+        deferred = true;  // to kCollideCrowd
         if (row == 0u && ((i - c0) & 31u) == 0u) {
           const unsigned k = atomicAdd(crowd.count, 1u);
           if (k < crowd.cap) crowd.groups[k] = make_uint2(i, min(32u, c1 - i));

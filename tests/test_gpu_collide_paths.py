@@ -365,3 +365,42 @@ def test_particles_moved_across_a_face_after_the_sort(grid, n, poly):
         dem.set_radius_mode(False)
     assert np.isfinite(want).all()
     np.testing.assert_array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("many", [0, 25_000])
+def test_crowded_cell_whose_first_members_moved_away(many):
+    """Members of a crowded cell that a staged host has moved across a face after
+    the sort, the first of many of its groups of 32 among them: every particle
+    gets its force, bit-exact against the oracle."""
+    from fullc0ntact_gb300 import dem, scenes
+    from oracle import oracle as O
+    m, cell = 700, 1.0 / 16.0
+    n = m + many
+    sc = scenes.random_box(n, grid=(32, 32, 32), radius=1.0 / 64.0, seed=3, cell=cell)
+    rng = np.random.default_rng(6)
+    pos, vel = sc["pos"], sc["vel"]
+    pos[m:, 0] = rng.uniform(0.0, 0.99, many)
+    pos[:m, :3] = -0.5 + rng.uniform(0.01, 0.99, (m, 3)) * cell
+    moved = pos.copy()
+    for first, axis in ((0, 0), (5, 1), (7, 2)):
+        some = np.arange(first, m, 8)
+        pos[some, axis] = -0.5 + cell - rng.uniform(1e-7, 1e-6, len(some))
+        moved[some, axis] = -0.5 + cell + rng.uniform(1e-7, 1e-6, len(some))
+    P = O.SimParams.from_buffer_copy(bytes(sc["params"]))
+    with O.gpu_arithmetic():
+        h, x = O.sort_pairs(*O.calc_hash(P, pos))
+        cs, ce, sp, sv = O.reorder(h, x, moved, vel, P.numCells)
+        want = O.collide(P, sp, sv, x, cs, ce)
+    ds = dem.DeviceScene(sc)
+    ds.activate()
+    dem.calc_hash(ds.hash, ds.index, ds.pos, n)
+    dem.sort_particles(ds.hash, ds.index, n)
+    ds.pos.copy_(torch.from_numpy(moved))
+    dem.reorder_data_and_find_cell_start(ds.cell_start, ds.cell_end, ds.sorted_pos, ds.sorted_vel,
+                                         ds.hash, ds.index, ds.pos, ds.vel, n, ds.num_cells)
+    out = torch.full_like(ds.vel, float("nan"))
+    dem.collide(out, ds.sorted_pos, ds.sorted_vel, ds.index, ds.cell_start, ds.cell_end, n,
+                ds.num_cells)
+    dem.check("collide")
+    assert np.isfinite(want).all()
+    np.testing.assert_array_equal(out.cpu().numpy(), want)
