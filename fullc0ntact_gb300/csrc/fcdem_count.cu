@@ -595,15 +595,16 @@ __device__ void largeRadixPass(const unsigned long long *src, unsigned long long
 // then gathered as in kFixupGather.  idBits = bits of the largest particle
 // index; bitmaps = kBitmapSlots slots of 2 * bitmapWords(n) words (the bits,
 // then the word prefix), or nullptr for the sort only.  kPairs: the members
-// of countSortPairs -- position and value in the slot, which are what the
-// outputs are; sortedPos is then 16 bytes of work space per pair.
+// of countSortPairs -- position and value in the slot; the keys, which may
+// have bits above the cell number, are found again by the position's `rank` in
+// the cell; sortedPos is then 16 bytes of work space per pair.
 template <bool kPairs>
 __global__ void __launch_bounds__(kLargeThreads)
 kFixupLarge(uint4 *slots, const unsigned *off, const unsigned *large,
             unsigned largeCap, unsigned *__restrict__ hashOut, unsigned *__restrict__ indexOut,
             float4 *__restrict__ sortedPos, float4 *__restrict__ sortedVel,
             const float4 *prevPos, const float4 *prevVel, unsigned n,
-            int idBits, unsigned *__restrict__ bitmaps) {
+            int idBits, unsigned *__restrict__ bitmaps, const unsigned *rank) {
   chainTrigger();
   chainWait();
   __shared__ LargeSmem sm;
@@ -676,6 +677,15 @@ kFixupLarge(uint4 *slots, const unsigned *off, const unsigned *large,
       A = B;
       B = tmp;
     }
+    if (kPairs) {
+      for (unsigned t = tid; t < c; t += kLargeThreads) {
+        const unsigned long long e = A[t];
+        hashOut[a + t] = slots[a + rank[(unsigned)(e >> 32)]].x;
+        indexOut[a + t] = (unsigned)e;
+      }
+      __syncthreads();
+      continue;
+    }
     for (unsigned t = tid; t < c; t += kLargeThreads) {
       const unsigned long long e = A[t];
       slots[a + t].y = (unsigned)(e >> 32);
@@ -684,11 +694,6 @@ kFixupLarge(uint4 *slots, const unsigned *off, const unsigned *large,
     __syncthreads();
     for (unsigned t = tid; t < c; t += kLargeThreads) {
       const unsigned me = slots[a + t].y, prev = slots[a + t].z;
-      if (kPairs) {
-        hashOut[a + t] = h;
-        indexOut[a + t] = prev;
-        continue;
-      }
       if (me >= n || prev >= n) continue;  // unfilled slot (reported by the scatter)
       hashOut[a + t] = h;
       indexOut[a + t] = me;
@@ -964,7 +969,7 @@ bool countPipelineSort(Context &c, const CountBuffers &b, const unsigned *origOf
   const unsigned largeCtas = b.largeCap < numSms() ? b.largeCap : numSms();  // one per SM at most
   launchChained(true, kFixupLarge<false>, largeCtas, kLargeThreads, 0, b.slots, b.off, b.large,
                 b.largeCap, hash, index, sortedPos, sortedVel, prevPos, prevVel, n,
-                keyBits(n), b.bitmaps);
+                keyBits(n), b.bitmaps, nullptr);
   return launchOk();
 }
 
@@ -1068,7 +1073,7 @@ bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int 
   const unsigned largeCtas = b.largeCap < numSms() ? b.largeCap : numSms();
   launchChained(true, kFixupLarge<true>, largeCtas, kLargeThreads, 0, b.slots, b.off, b.large,
                 b.largeCap, keys, vals, (float4 *)b.work, nullptr, nullptr, nullptr, n, keyBits(n),
-                b.bitmaps);
+                b.bitmaps, b.rank);
   launchOk();
   return true;
 }

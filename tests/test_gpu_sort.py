@@ -181,3 +181,33 @@ def test_counting_and_radix_sort_agree(n, cells):
         dem.lib.fcdemSetSortConfig(n, -1)
     np.testing.assert_array_equal(k, rk)
     np.testing.assert_array_equal(v, rv)
+
+
+@pytest.mark.parametrize("n,cells", [(200_000, 64), (60_000, 4), (300_000, 2 ** 12), (3000, 2)])
+def test_keys_above_the_width_are_kept(n, cells):
+    """Keys with bits above the sorted width are reported, and the pairs come back
+    whole, in stable order of their low bits, however large their cells are.
+    (The radix sort takes whole bytes of the key: its pairs are whole too.)"""
+    from fullc0ntact_gb300 import dem
+    from fullc0ntact_gb300.params import make_params
+    rng = np.random.default_rng(n)
+    keys = rng.integers(0, 2 ** 32, n, dtype=np.uint64).astype(np.uint32)
+    if cells == 2 ** 12:  # sparse members of crowded cells among many small ones
+        keys = np.where(rng.random(n) < 0.2, keys & np.uint32(0xfff0001f), keys)
+    vals = rng.integers(0, 2 ** 32, n, dtype=np.uint64).astype(np.uint32)
+    P = make_params(n, (2, 2, 2), 0.01)
+    P.numCells = cells
+    dem.set_parameters(P)
+    whole = 8 * -(-(cells - 1).bit_length() // 8)  # the radix sort's bits
+    for config, bits in ((-1, (cells - 1).bit_length()), (0, whole)):
+        dem.lib.fcdemSetSortConfig(n, config)
+        try:
+            k = torch.from_numpy(keys.view(np.int32).copy()).cuda()
+            v = torch.from_numpy(vals.view(np.int32).copy()).cuda()
+            dem.sort_particles(k, v, n)
+            assert dem.lib.fcdemGetLastError() == 6  # FCDEM_ERR_KEY_RANGE
+        finally:
+            dem.lib.fcdemSetSortConfig(n, -1)
+        o = np.argsort(keys & np.uint32((1 << bits) - 1), kind="stable")
+        np.testing.assert_array_equal(k.cpu().numpy().view(np.uint32), keys[o])
+        np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), vals[o])
