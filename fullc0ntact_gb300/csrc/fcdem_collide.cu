@@ -820,7 +820,7 @@ kCollideRows(float4 *newVel, const float4 *sortedPos, const float4 *sortedVel,
 // terms with the lanes that have queued partners, all from shared memory.
 template <int kMode, bool kRadiusFromW, bool kCollider, bool kForceOut, bool kPrefix>
 __global__ void __launch_bounds__(kCrowdWarps * 32)
-kCollideCrowd(float4 *__restrict__ newVel, const float4 *sortedPos,
+kCollideCrowd(float4 *newVel, const float4 *sortedPos,
               const float4 *sortedVel, const unsigned *index,
               CellRanges cells, unsigned n, KParams kp, CollideOut out, bool cull,
               CrowdList crowd, unsigned *status) {

@@ -57,8 +57,8 @@ __device__ __forceinline__ void resetLists(unsigned *largeCount, unsigned *crowd
 // tileOff[t] = sum of tileCnt[0..t), tileOff[tiles] = the total; tileCnt is
 // cleared for the next step.  One CTA of 1024 threads, tiles in chunks.
 __global__ void __launch_bounds__(1024)
-kScanTiles(unsigned *__restrict__ tileCnt, unsigned *__restrict__ tileOff, unsigned tiles,
-           unsigned *__restrict__ largeCount, unsigned *__restrict__ crowdCount) {
+kScanTiles(unsigned *tileCnt, unsigned *tileOff, unsigned tiles,
+           unsigned *largeCount, unsigned *crowdCount) {
   chainTrigger();
   chainWait();
   __shared__ unsigned sWarp[32];
@@ -111,9 +111,9 @@ constexpr unsigned kTilesOneCta = 8192;  // up to this many tiles kScanTiles run
 constexpr unsigned kTilesOwnPrefix = 4608;  // up to this many tiles kScanCellsOwn
 
 __global__ void __launch_bounds__(kTileBlock)
-kScanTileBlocks(unsigned *__restrict__ tileCnt, unsigned *__restrict__ tileOff, unsigned tiles,
-                unsigned *__restrict__ blockSum, unsigned *__restrict__ largeCount,
-                unsigned *__restrict__ crowdCount) {
+kScanTileBlocks(unsigned *tileCnt, unsigned *tileOff, unsigned tiles,
+                unsigned *blockSum, unsigned *largeCount,
+                unsigned *crowdCount) {
   chainTrigger();
   chainWait();
   __shared__ unsigned sWarp[32];
@@ -147,7 +147,7 @@ kScanTileBlocks(unsigned *__restrict__ tileCnt, unsigned *__restrict__ tileOff, 
 }
 
 __global__ void __launch_bounds__(kTileBlock)
-kAddTileBlocks(unsigned *__restrict__ tileOff, unsigned tiles,
+kAddTileBlocks(unsigned *tileOff, unsigned tiles,
                const unsigned *blockSum) {
   chainTrigger();
   chainWait();
@@ -601,10 +601,10 @@ __device__ void largeRadixPass(const unsigned long long *src, unsigned long long
 template <bool kPairs>
 __global__ void __launch_bounds__(kLargeThreads)
 kFixupLarge(uint4 *slots, const unsigned *off, const unsigned *large,
-            unsigned largeCap, unsigned *__restrict__ hashOut, unsigned *__restrict__ indexOut,
-            float4 *__restrict__ sortedPos, float4 *__restrict__ sortedVel,
+            unsigned largeCap, unsigned *hashOut, unsigned *indexOut,
+            float4 *sortedPos, float4 *sortedVel,
             const float4 *prevPos, const float4 *prevVel, unsigned n,
-            int idBits, unsigned *__restrict__ bitmaps, const unsigned *rank) {
+            int idBits, unsigned *bitmaps, const unsigned *rank) {
   chainTrigger();
   chainWait();
   __shared__ LargeSmem sm;
@@ -745,9 +745,9 @@ kCellTables(const unsigned *off, unsigned *cellStart, unsigned *cellEnd, unsigne
 // counts too; otherwise they follow in kTileReduce.
 template <bool kTiles>
 __global__ void __launch_bounds__(256)
-kIntegrateHashCount(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt,
-                    unsigned *__restrict__ hash, unsigned *__restrict__ rank,
-                    unsigned *__restrict__ cnt, unsigned *__restrict__ tileCnt, unsigned n,
+kIntegrateHashCount(float4 *pos, float4 *vel, float dt,
+                    unsigned *hash, unsigned *rank,
+                    unsigned *cnt, unsigned *tileCnt, unsigned n,
                     KParams kp) {
   chainTrigger();
   chainWait();
@@ -770,7 +770,7 @@ kIntegrateHashCount(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt
 // particle-order cells are scattered over the tiles: summing the counts once
 // is cheaper than one atomic per particle on the few tile counters).
 __global__ void __launch_bounds__(kScanThreads)
-kTileReduce(const unsigned *cnt, unsigned *__restrict__ tileCnt, unsigned m) {
+kTileReduce(const unsigned *cnt, unsigned *tileCnt, unsigned m) {
   chainTrigger();
   chainWait();
   __shared__ unsigned sWarp[kScanThreads / 32];
@@ -805,15 +805,15 @@ kTileReduce(const unsigned *cnt, unsigned *__restrict__ tileCnt, unsigned m) {
 // scene's box, global cell id = the scene's cellBase + local hash.
 template <bool kRadiusFromW>
 __global__ void __launch_bounds__(256)
-kBatchIntegrateHashCount(const BatchScene *__restrict__ scenes,
-                         const unsigned *__restrict__ sceneOf, float4 *__restrict__ pos,
-                         float4 *__restrict__ vel, float dt, unsigned *__restrict__ hash,
-                         unsigned *__restrict__ rank, unsigned *__restrict__ cnt, unsigned n) {
+kBatchIntegrateHashCount(const BatchScene *scenes,
+                         const unsigned *sceneOf, float4 *pos,
+                         float4 *vel, float dt, unsigned *hash,
+                         unsigned *rank, unsigned *cnt, unsigned n) {
   chainTrigger();
   chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const BatchScene &S = scenes[__ldg(sceneOf + i)];
+  const BatchScene &S = scenes[sceneOf[i]];
   const SimParams &P = S.p;
   float4 p4 = pos[i], v4 = vel[i];
   float3 p = make_float3(p4.x, p4.y, p4.z), v = make_float3(v4.x, v4.y, v4.z);

@@ -18,7 +18,7 @@ namespace {
 // kCount: also the next step's calcHash and cell count (counting pipeline).
 template <bool kCount>
 __global__ void __launch_bounds__(256)
-kIntegrateDistMap(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt, unsigned n,
+kIntegrateDistMap(float4 *pos, float4 *vel, float dt, unsigned n,
                   KParams kp, MapView M, int useMap, UmCount count) {
   chainTrigger();
   chainWait();

@@ -113,8 +113,9 @@ bool clearNow(void *device, int byte, size_t bytes);
 // then reads or writes what others touch: a kernel's completion thus still
 // implies that of all before it, the caller's included.  What earlier kernels
 // wrote is read with plain loads: a __ldg or a const __restrict__ parameter
-// tells the compiler that the value never changes, and it may then load it
-// before chainWait().  (kSdfTrain reads its samples before chainWait(); its
+// tells the compiler that the value never changes, and any __restrict__ one that
+// no other code, chainWait() included, changes it, and it may then load it
+// before chainWait(); so their parameters have none.  (kSdfTrain reads its samples before chainWait(); its
 // first launch of a call is not chained.)  Launched without the attribute the
 // two calls do nothing.
 __device__ __forceinline__ void chainTrigger() {

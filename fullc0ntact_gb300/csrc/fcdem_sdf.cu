@@ -179,9 +179,9 @@ struct TrainSmem {
 // writes the distance prediction to yOut.
 template <int H, int L, bool kBackward>
 __global__ void __launch_bounds__(4 * H, 1)
-kSdfTrain(SdfView net, const float4 *__restrict__ samples, const int *__restrict__ shapes,
-          unsigned n, float band, float invB, float *__restrict__ partial,
-          float *__restrict__ lossSum, float *__restrict__ yOut) {
+kSdfTrain(SdfView net, const float4 *samples, const int *shapes,
+          unsigned n, float band, float invB, float *partial,
+          float *lossSum, float *yOut) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   TrainSmem<H, L> &sm = *reinterpret_cast<TrainSmem<H, L> *>(smraw);
   constexpr int T = 4 * H, S = kTrainS, Q = H / 4;
@@ -398,8 +398,8 @@ kSdfTrain(SdfView net, const float4 *__restrict__ samples, const int *__restrict
 constexpr int kReduceWarps = 8;
 template <bool kAdam>
 __global__ void __launch_bounds__(32 * kReduceWarps)
-kSdfReduce(const float *partial, unsigned parts, unsigned total, float *__restrict__ p,
-           float *__restrict__ grad, float *__restrict__ m, float *__restrict__ v,
+kSdfReduce(const float *partial, unsigned parts, unsigned total, float *p,
+           float *grad, float *m, float *v,
            float lr, float b1, float b2, float eps, float c1, float c2) {
   __shared__ float sSum[kReduceWarps][32];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;

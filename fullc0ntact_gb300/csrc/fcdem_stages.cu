@@ -11,7 +11,7 @@ constexpr unsigned kEmpty = 0xffffffffu;
 // integrate (particles_kernel.cu:39-75; launched by thrust::for_each in
 // particleSystem.cu:141-153).  One thread per particle, 128-bit loads/stores.
 __global__ void __launch_bounds__(256)
-kIntegrate(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt,
+kIntegrate(float4 *pos, float4 *vel, float dt,
            unsigned n, KParams kp) {
   chainTrigger();
   chainWait();
@@ -28,7 +28,7 @@ kIntegrate(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt,
 // ---------------------------------------------------------------------------
 // calcHash (particles_kernel.cu:97-115).
 __global__ void __launch_bounds__(256)
-kCalcHash(unsigned *__restrict__ hash, unsigned *__restrict__ index,
+kCalcHash(unsigned *hash, unsigned *index,
           const float4 *pos, unsigned n, KParams kp) {
   chainTrigger();
   chainWait();
@@ -63,7 +63,7 @@ kIntegrateHash(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt,
 // Fill (the cudaMemset of particleSystem.cu:198).  16-byte stores where the
 // pointer allows, grid-stride.
 __global__ void __launch_bounds__(256)
-kFill(unsigned *__restrict__ p, size_t count, unsigned value) {
+kFill(unsigned *p, size_t count, unsigned value) {
   chainTrigger();
   chainWait();
   size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -94,8 +94,8 @@ void fillU32(Context &, unsigned *p, size_t count, unsigned value) {
 // hash is read directly (adjacent threads share the cache line), the gathers
 // are 128-bit.
 __global__ void __launch_bounds__(256)
-kReorder(unsigned *__restrict__ cellStart, unsigned *__restrict__ cellEnd,
-         float4 *__restrict__ sortedPos, float4 *__restrict__ sortedVel,
+kReorder(unsigned *cellStart, unsigned *cellEnd,
+         float4 *sortedPos, float4 *sortedVel,
          const unsigned *hash, const unsigned *index,
          const float4 *oldPos, const float4 *oldVel,
          unsigned n, unsigned numCells, unsigned *status) {
