@@ -79,9 +79,9 @@ unsigned numSms();
 // Look-back rounds a sort tile may make before it gives up
 // (fcdemSetSortWaitLimit; default kSortWaitRounds).
 unsigned sortWaitLimit();
-// Whether a set look-back limit or a configuration chosen for n's size class
-// asks for the radix sort.
-bool radixSortAsked(unsigned n);
+// Whether a set look-back limit or a choice for n's size class and the key
+// width asks for the radix sort.
+bool radixSortAsked(unsigned n, int bits);
 // The status word of the allocation-free sort on the current device, or
 // nullptr when that sort has not been set up there (fcdem_sort.cu).
 unsigned *noAllocStatusWord();

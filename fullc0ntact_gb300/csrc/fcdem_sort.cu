@@ -330,8 +330,11 @@ const PassConfig kPassConfigs[] = {
 };
 constexpr int kNumPassConfigs = sizeof(kPassConfigs) / sizeof(kPassConfigs[0]);
 
-// Tuned choice per size class (log2 of the particle count); -1 = default.
+// Tuned choices per size class (log2 of the particle count): the radix sort's
+// shape (-1 = default), and the key widths at which sortParticles takes it where
+// the counting sort is open (a bit per width; all of them once a shape is set).
 int g_sortChoice[33];
+unsigned long long g_radixWidths[33] = {};
 bool g_sortChoiceInit = false;
 std::mutex g_sortChoiceMutex;
 
@@ -365,6 +368,20 @@ const PassConfig &chooseConfig(unsigned n) {
   }
   int k = g_sortChoice[sizeClass(n)];
   return kPassConfigs[k >= 0 && k < kNumPassConfigs ? k : 0];
+}
+
+void setShape(unsigned n, int shape) {
+  chooseConfig(n);  // initialises the table
+  std::lock_guard<std::mutex> lock(g_sortChoiceMutex);
+  g_sortChoice[sizeClass(n)] = shape;
+}
+
+// radix: the key widths of `widths` take the radix sort in n's size class;
+// otherwise the counting sort where it is open.
+void setRadixWidths(unsigned n, unsigned long long widths, bool radix) {
+  std::lock_guard<std::mutex> lock(g_sortChoiceMutex);
+  unsigned long long &w = g_radixWidths[sizeClass(n)];
+  w = radix ? (w | widths) : (w & ~widths);
 }
 
 inline size_t alignUp(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -529,11 +546,10 @@ unsigned *noAllocStatusWord() {
 
 unsigned sortWaitLimit() { return g_sortWaitRounds.load(std::memory_order_relaxed); }
 
-bool radixSortAsked(unsigned n) {
+bool radixSortAsked(unsigned n, int bits) {
   if (sortWaitLimit() != kSortWaitRounds) return true;
-  chooseConfig(n);  // initialises the table
   std::lock_guard<std::mutex> lock(g_sortChoiceMutex);
-  return g_sortChoice[sizeClass(n)] >= 0;
+  return (g_radixWidths[sizeClass(n)] >> bits) & 1ull;
 }
 
 }  // namespace fcdem
@@ -631,10 +647,9 @@ __global__ void kTuneKeys(unsigned *keys, unsigned *vals, unsigned n, unsigned m
 
 extern "C" int fcdemSetSortConfig(unsigned numParticles, int config) {
   using namespace fcdem;
-  if (config < -1 || config >= kNumPassConfigs) { setError(FCDEM_ERR_INVALID_VALUE); return -1; }
-  chooseConfig(numParticles);  // initialises the table
-  std::lock_guard<std::mutex> lock(g_sortChoiceMutex);
-  g_sortChoice[sizeClass(numParticles)] = config;
+  if (config < -1 || config > kNumPassConfigs) { setError(FCDEM_ERR_INVALID_VALUE); return -1; }
+  if (config < kNumPassConfigs) setShape(numParticles, config);
+  setRadixWidths(numParticles, ~0ull, config >= 0 && config < kNumPassConfigs);
   return kNumPassConfigs;
 }
 
@@ -663,7 +678,7 @@ extern "C" int fcdemAutotuneSort(unsigned numParticles, unsigned numCells, float
   int best = 0;
   float bestT = 3.4e38f;
   for (int k = 0; k < kNumPassConfigs; ++k) {
-    fcdemSetSortConfig(n, k);
+    setShape(n, k);
     float tot = 0.0f;
     for (int rep = 0; rep < 4; ++rep) {
       cudaMemcpyAsync(k1, k0, (size_t)n * 8, cudaMemcpyDeviceToDevice, st);
@@ -677,8 +692,9 @@ extern "C" int fcdemAutotuneSort(unsigned numParticles, unsigned numCells, float
     }
     if (tot < bestT) { bestT = tot; best = k; }
   }
-  fcdemSetSortConfig(n, best);
-  // the counting sort that sortParticles takes by default, timed alike
+  setShape(n, best);
+  // the counting sort that sortParticles takes by default, timed alike: where it
+  // is open, the choice between the two is this key width's alone
   float count = 0.0f;
   bool counted = true;
   for (int rep = 0; rep < 4 && counted; ++rep) {
@@ -691,9 +707,12 @@ extern "C" int fcdemAutotuneSort(unsigned numParticles, unsigned numCells, float
     cudaEventElapsedTime(&t, e0, e1);
     if (rep > 0) count += t;
   }
-  if (counted && count < bestT) {
-    bestT = count;
-    fcdemSetSortConfig(n, -1);
+  if (counted) {
+    setRadixWidths(n, 1ull << bits, bestT <= count);
+    if (count < bestT) {
+      bestT = count;
+      best = kNumPassConfigs;
+    }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);

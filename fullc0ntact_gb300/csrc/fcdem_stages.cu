@@ -261,7 +261,7 @@ void sortParticles(uint *dGridParticleHash, uint *dGridParticleIndex,
     return;
   }
   int bits = c.haveParams ? keyBits(c.params.numCells) : 32;
-  if (!radixSortAsked(numParticles) &&
+  if (!radixSortAsked(numParticles, bits) &&
       countSortPairs(c, dGridParticleHash, dGridParticleIndex, numParticles, bits))
     return;
   radixSortPairs(c, dGridParticleHash, dGridParticleIndex, numParticles, bits);

@@ -243,14 +243,16 @@ void fcdemSetCollidePath(int path);
 void fcdemSetSortWaitLimit(int rounds);
 
 /* Sort tuning.  The passes of the radix sort come in several block shapes
- * (threads x keys per thread); results are identical.  fcdemAutotuneSort
- * times each on numParticles uniform keys below numCells (allocating
- * temporary device memory), keeps the fastest for that size class
- * (power-of-two bucket of numParticles) and returns its index (-1 on error);
- * where sortParticles' default, the counting sort, is faster than all of
- * them, that stays the choice.  *bestMs receives the kept one's time.
+ * (threads x keys per thread), numbered from 0; the number after the last
+ * shape's stands for the counting sort.  Results are identical.
+ * fcdemAutotuneSort times each on numParticles uniform keys below numCells
+ * (allocating temporary device memory) and returns the number of the fastest
+ * (-1 on error); *bestMs receives its time.  It keeps the best shape for the
+ * size class (power-of-two bucket of numParticles) and, where the counting sort
+ * is open to these keys, whether sortParticles takes it at this key width.
  * fcdemSetSortConfig forces a shape, and with it the radix sort in
- * sortParticles (-1 = default), and returns the number of shapes. */
+ * sortParticles, or the counting sort where it is open (-1 = default: that and
+ * the first shape), for a size class, and returns the number of shapes. */
 int fcdemAutotuneSort(unsigned numParticles, unsigned numCells, float *bestMs);
 int fcdemSetSortConfig(unsigned numParticles, int config);
 

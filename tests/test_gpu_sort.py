@@ -1,5 +1,7 @@
 """sortParticles: the onesweep radix sort against a stable CPU sort, on the
 key distributions the step produces and on edge cases."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -211,3 +213,36 @@ def test_keys_above_the_width_are_kept(n, cells):
         o = np.argsort(keys & np.uint32((1 << bits) - 1), kind="stable")
         np.testing.assert_array_equal(k.cpu().numpy().view(np.uint32), keys[o])
         np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), vals[o])
+
+
+def _launches(n, cells):
+    """Kernel launches of one sortParticles of n pairs below cells."""
+    from fullc0ntact_gb300 import dem
+    dem.lib.fcdemGetLaunchCount.restype = ctypes.c_ulonglong
+    keys = np.random.default_rng(n).integers(0, cells, n).astype(np.uint32)
+    _sort_gpu(keys, np.arange(n, dtype=np.uint32), cells)  # (buffers)
+    before = dem.lib.fcdemGetLaunchCount()
+    _sort_gpu(keys, np.arange(n, dtype=np.uint32), cells)
+    return dem.lib.fcdemGetLaunchCount() - before
+
+
+@pytest.mark.parametrize("n,cells", [(200_000, 2 ** 24), (200_000, 2 ** 30), (2 ** 21 + 5, 2 ** 24)])
+def test_autotuned_index_names_the_kept_sort(n, cells):
+    """Setting the index that the tuner returned changes nothing, and a tuning
+    run leaves other key widths of the size class alone."""
+    from fullc0ntact_gb300 import dem
+    lib = dem.lib
+    shapes = lib.fcdemSetSortConfig(n, -1)
+    default = _launches(n, 2 ** 20)
+    counted = _launches(n, cells) == _launches(n, 2 ** 20) and n <= 2 ** 21
+    try:
+        t = ctypes.c_float()
+        best = lib.fcdemAutotuneSort(n, cells, ctypes.byref(t))
+        dem.check("autotune")
+        assert 0 <= best <= shapes and (best < shapes or (counted and cells <= 2 ** 24))
+        kept = _launches(n, cells)
+        assert _launches(n, 2 ** 20) == default
+        assert lib.fcdemSetSortConfig(n, best) == shapes
+        assert _launches(n, cells) == kept
+    finally:
+        lib.fcdemSetSortConfig(n, -1)
