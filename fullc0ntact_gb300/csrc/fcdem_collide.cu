@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(128, 9)
 kCollideGlobal(float4 *__restrict__ newVel, const float4 *__restrict__ sortedPos,
                const float4 *__restrict__ sortedVel, const unsigned *__restrict__ index,
                CellRanges cells, unsigned n, KParams kp, CollideOut out, bool cull,
-               CrowdList crowd, unsigned *status) {
+               CrowdList crowd, DeviceStatus *status) {
   __shared__ unsigned qj[kQueueLen * kQueueStride];
   __shared__ unsigned char qc[kQueueLen * kQueueStride];
   __shared__ uint2 sSeg[9 * kQueueStride];
@@ -620,7 +620,7 @@ kCollideGlobal(float4 *__restrict__ newVel, const float4 *__restrict__ sortedPos
   const float ri = kRadiusFromW ? p4.w : P.particleRadius;
   const int3 g = gridPos(pos.x, pos.y, pos.z, P);
   if (kRadiusFromW && !(ri <= P.particleRadius)) {
-    atomicOr(status, (unsigned)kStatusRadiusBound);  // the culling bound is broken
+    report(status, kStatusRadiusBound);  // the culling bound is broken
     cull = false;
   }
   uint2 *mySeg = sSeg + threadIdx.x;
@@ -680,7 +680,7 @@ template <int kMode, bool kRadiusFromW, bool kCollider, bool kForceOut, bool kPr
 __global__ void __launch_bounds__(32 * kRowsWarps)
 kCollideRows(float4 *newVel, const float4 *sortedPos, const float4 *sortedVel,
              const unsigned *index, CellRanges cells, unsigned n, KParams kp, CollideOut out,
-             bool cull, CrowdList crowd, unsigned *status) {
+             bool cull, CrowdList crowd, DeviceStatus *status) {
   __shared__ float sSum[kRowsWarps][3][3][28];  // [warp][particle][x, y, z][cell]
   __shared__ unsigned sTotal[kRowsWarps][3][9];
   const SimParams &P = kp.p;
@@ -696,7 +696,7 @@ kCollideRows(float4 *newVel, const float4 *sortedPos, const float4 *sortedVel,
   const float ri = kRadiusFromW ? p4.w : P.particleRadius;
   const int3 g = gridPos(pos.x, pos.y, pos.z, P);
   if (active && kRadiusFromW && !(ri <= P.particleRadius)) {
-    atomicOr(status, (unsigned)kStatusRadiusBound);  // the culling bound is broken
+    report(status, kStatusRadiusBound);  // the culling bound is broken
     cull = false;
   }
   const CellCull cc = makeCull(pos, g, ri + P.particleRadius, P);
@@ -823,7 +823,7 @@ __global__ void __launch_bounds__(kCrowdWarps * 32)
 kCollideCrowd(float4 *newVel, const float4 *sortedPos,
               const float4 *sortedVel, const unsigned *index,
               CellRanges cells, unsigned n, KParams kp, CollideOut out, bool cull,
-              CrowdList crowd, unsigned *status) {
+              CrowdList crowd, DeviceStatus *status) {
   __shared__ float4 sPos[kCrowdWarps][32];
   __shared__ float4 sVel[kCrowdWarps][32];
   __shared__ unsigned char sQ[kCrowdWarps][32][32];  // [warp][entry][lane]
@@ -855,7 +855,7 @@ kCollideCrowd(float4 *newVel, const float4 *sortedPos,
     const bool scan = valid && !inertPos(pos);  // an inert member's force is +0.0
     bool lcull = cull;
     if (valid && kRadiusFromW && !(ri <= P.particleRadius)) {
-      atomicOr(status, (unsigned)kStatusRadiusBound);
+      report(status, kStatusRadiusBound);
       lcull = false;
     }
     const CellCull cc = makeCull(pos, g, ri + P.particleRadius, P);
@@ -1004,7 +1004,7 @@ template <int kMode, bool kRadiusFromW, bool kCollider, bool kForceOut>
 __global__ void __launch_bounds__(kTileThreads)
 kCollideTiled(float4 *__restrict__ newVel, const float4 *__restrict__ sortedPos,
               const float4 *__restrict__ sortedVel, const unsigned *__restrict__ index,
-              CellRanges cells, unsigned n, KParams kp, CollideOut out, unsigned *status) {
+              CellRanges cells, unsigned n, KParams kp, CollideOut out, DeviceStatus *status) {
   const unsigned *__restrict__ cellStart = cells.start;
   const unsigned *__restrict__ cellEnd = cells.end;
   __shared__ TileSmem sm;
@@ -1116,7 +1116,7 @@ kCollideTiled(float4 *__restrict__ newVel, const float4 *__restrict__ sortedPos,
     const bool staged = stageable && sm.staged;
     if (staged) {
       if (!mbarWait(&sm.bar, phase)) {
-        atomicOr(status, (unsigned)kStatusTimeout);
+        report(status, kStatusTimeout);
         // wait (bounded) for the copies in flight before touching the
         // buffer again or leaving
         mbarWait(&sm.bar, phase);
@@ -1255,7 +1255,7 @@ __global__ void __launch_bounds__(128)
 kCollideBatch(const BatchScene *__restrict__ scenes, const unsigned *__restrict__ sceneOf,
               float4 *__restrict__ newVel, const float4 *__restrict__ sortedPos,
               const float4 *__restrict__ sortedVel, const unsigned *__restrict__ index,
-              const unsigned *__restrict__ off, unsigned n, CollideOut out, unsigned *status) {
+              const unsigned *__restrict__ off, unsigned n, CollideOut out, DeviceStatus *status) {
   __shared__ unsigned qj[kQueueLen * kQueueStride];
   __shared__ unsigned char qc[kQueueLen * kQueueStride];
   __shared__ uint2 sSeg[9 * kQueueStride];
@@ -1270,7 +1270,7 @@ kCollideBatch(const BatchScene *__restrict__ scenes, const unsigned *__restrict_
   int3 g = gridPosDivide(pos.x, pos.y, pos.z, P);
   bool cull = S.cull != 0;
   if (kRadiusFromW && !(ri <= P.particleRadius)) {
-    atomicOr(status, (unsigned)kStatusRadiusBound);
+    report(status, kStatusRadiusBound);
     cull = false;
   }
   CellRanges cells;
@@ -1390,7 +1390,7 @@ void launchCollideBatch(int mode, bool radiusFromW, const BatchScene *scenes,
                         unsigned n, const CollideOut &out) {
   if (n == 0) return;
   const unsigned blocks = (n + 127) / 128;
-  unsigned *st = ctx().dStatus;
+  DeviceStatus *st = ctx().dStatus;
   if (mode == 2 && !radiusFromW)
     kCollideBatch<2, false><<<blocks, 128, 0, curStream()>>>(scenes, sceneOf, newVel, sp, sv,
                                                              index, off, n, out, st);

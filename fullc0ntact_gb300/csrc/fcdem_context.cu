@@ -99,14 +99,15 @@ Context &ctx() {
   if (c.device < 0) {
     std::lock_guard<std::mutex> lock(g_mutex);
     if (c.device < 0) {
-      // mapped host memory: kernels touch it on an error only, and
-      // fcdemGetLastError reads it without a copy
-      unsigned *status = nullptr;
-      if (cudaOk(cudaHostAlloc(&status, sizeof(unsigned),
-                               cudaHostAllocMapped | cudaHostAllocPortable))) {
-        *status = 0u;
-        c.hStatus = status;
-        if (!cudaOk(cudaHostGetDevicePointer(&c.dStatus, status, 0))) c.dStatus = nullptr;
+      unsigned *word = nullptr;
+      DeviceStatus s{0u, nullptr}, *status = nullptr;
+      if (cudaOk(cudaHostAlloc(&word, sizeof(unsigned),
+                               cudaHostAllocMapped | cudaHostAllocPortable)) &&
+          cudaOk(cudaHostGetDevicePointer(&s.host, word, 0)) &&
+          cudaOk(cudaMalloc(&status, sizeof(s))) && uploadNow(status, &s, sizeof(s))) {
+        *word = 0u;
+        c.hStatus = word;
+        c.dStatus = status;
       }
       c.device = dev;
     }
@@ -277,9 +278,10 @@ void recordStatus(unsigned status) {
   else if (status & kStatusCellOverflow) setError(FCDEM_ERR_CELL_OVERFLOW);
 }
 
-// Reads and clears a status word in device memory (synchronising the library
+// Reads and clears a status without a host word (synchronising the library
 // stream).
-void drainDeviceStatus(unsigned *word) {
+void drainDeviceStatus(DeviceStatus *s0) {
+  unsigned *word = &s0->bits;
   unsigned status = 0;
   cudaStream_t s = curStream();
   if (cudaMemcpyAsync(&status, word, sizeof(unsigned), cudaMemcpyDeviceToHost, s) ==
@@ -295,13 +297,15 @@ void drainDeviceStatus(unsigned *word) {
   }
 }
 
-// The same for the context's word, in mapped host memory.
+// The same for the context's, from its host word.  That is cleared first: a
+// report from another stream between the two clears is lost, but none after it.
 void drainStatus(Context &c) {
   if (!cudaOk(cudaStreamSynchronize(curStream()))) return;
   volatile unsigned *word = c.hStatus;
   const unsigned status = *word;
   if (status) {
     *word = 0u;
+    cudaOk(cudaMemsetAsync(&c.dStatus->bits, 0, sizeof(unsigned), curStream()));
     recordStatus(status);
   }
 }
@@ -312,8 +316,8 @@ extern "C" {
 int fcdemGetLastError(void) {
   Context &c = ctx();
   if (c.dStatus) drainStatus(c);
-  // the allocation-free sort keeps its own status word in its static scratch
-  if (unsigned *w = noAllocStatusWord()) drainDeviceStatus(w);
+  // the allocation-free sort keeps its own status in its static scratch
+  if (DeviceStatus *s = noAllocStatus()) drainDeviceStatus(s);
   return g_error.exchange(FCDEM_SUCCESS);
 }
 

@@ -322,7 +322,7 @@ kScanCellsMany(unsigned *cnt, unsigned *off, unsigned m, unsigned tiles, const u
 __global__ void __launch_bounds__(256)
 kScatterCells(const unsigned *hashN, const unsigned *rankN, const unsigned *origOf,
               const unsigned *off, uint4 *slots, unsigned n, unsigned numCells, unsigned *tileCnt,
-              unsigned tiles, unsigned *status) {
+              unsigned tiles, DeviceStatus *status) {
   chainTrigger();
   chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -331,12 +331,12 @@ kScatterCells(const unsigned *hashN, const unsigned *rankN, const unsigned *orig
   if (i >= n) return;
   unsigned h = hashN[i];
   if (h >= numCells) {
-    atomicOr(status, (unsigned)kStatusKeyRange);
+    report(status, kStatusKeyRange);
     return;
   }
   const unsigned a = off[h], s = a + rankN[i];
   if (s >= n) {
-    atomicOr(status, (unsigned)kStatusKeyRange);
+    report(status, kStatusKeyRange);
     return;
   }
   slots[s] = make_uint4(h, origOf ? origOf[i] : i, i, a);
@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(256)
 kFixupGather(const uint4 *slots, const unsigned *off, unsigned *hashOut, unsigned *indexOut,
              float4 *sortedPos, float4 *sortedVel, const float4 *prevPos, const float4 *prevVel,
              unsigned n, unsigned numCells, unsigned maxCell, unsigned *large, unsigned largeCap,
-             unsigned *status) {
+             DeviceStatus *status) {
   chainTrigger();
   chainWait();
   unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -380,7 +380,7 @@ kFixupGather(const uint4 *slots, const unsigned *off, unsigned *hashOut, unsigne
       if (k < largeCap)
         large[1 + k] = h;
       else
-        atomicOr(status, (unsigned)kStatusCellOverflow);
+        report(status, kStatusCellOverflow);
     }
     return;
   }
@@ -402,13 +402,13 @@ kFixupGather(const uint4 *slots, const unsigned *off, unsigned *hashOut, unsigne
 template <bool kTiles>
 __global__ void __launch_bounds__(256)
 kCountKeys(const unsigned *keys, unsigned n, unsigned mask, unsigned *rank, unsigned *cnt,
-           unsigned *tileCnt, unsigned *status) {
+           unsigned *tileCnt, DeviceStatus *status) {
   chainTrigger();
   chainWait();
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const unsigned k = keys[i], h = k & mask;
-  if (k != h) atomicOr(status, (unsigned)kStatusKeyRange);
+  if (k != h) report(status, kStatusKeyRange);
   rank[i] = atomicAdd(cnt + h, 1u);
   if (kTiles) countTile(tileCnt, h >> kTileShift);
 }
@@ -428,7 +428,7 @@ kScatterPairs(const unsigned *keys, const unsigned *vals, const unsigned *rankN,
 
 __global__ void __launch_bounds__(256)
 kFixupPairs(const uint4 *slots, const unsigned *off, unsigned *keys, unsigned *vals, unsigned n,
-            unsigned mask, unsigned maxCell, unsigned *large, unsigned largeCap, unsigned *status) {
+            unsigned mask, unsigned maxCell, unsigned *large, unsigned largeCap, DeviceStatus *status) {
   chainTrigger();
   chainWait();
   const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -442,7 +442,7 @@ kFixupPairs(const uint4 *slots, const unsigned *off, unsigned *keys, unsigned *v
       if (k < largeCap)
         large[1 + k] = h;
       else
-        atomicOr(status, (unsigned)kStatusCellOverflow);
+        report(status, kStatusCellOverflow);
     }
     return;
   }

@@ -26,7 +26,7 @@ static_assert(offsetof(SimParams, shear) == 92, "layout");
 static_assert(offsetof(SimParams, attraction) == 96, "layout");
 static_assert(offsetof(SimParams, boundaryDamping) == 100, "layout");
 
-// Device status bits (written by kernels with atomicOr, read by
+// Device status bits (written by kernels with report(), read by
 // fcdemGetLastError).
 enum : unsigned {
   kStatusTimeout = 1u,   // a bounded spin-wait gave up
@@ -34,6 +34,21 @@ enum : unsigned {
   kStatusRadiusBound = 4u,  // radius-from-w mode: a radius above particleRadius
   kStatusCellOverflow = 8u,  // counting sort: the list of crowded cells overflowed
 };
+
+// Where kernels report errors.  The first report of a bit since the last clear
+// also goes to `host` (mapped host memory, or nullptr), where fcdemGetLastError
+// sees it without a copy; every further one ends at the word in device memory,
+// with a load: a scene that breaks a bound in every particle and step crosses
+// the host link once (400,000 spheres with radii above particleRadius, four
+// steps: 406 us, 704 with an atomic on the host word per warp; within bounds 390).
+struct DeviceStatus {
+  unsigned bits;
+  unsigned *host;
+};
+__device__ __forceinline__ void report(DeviceStatus *s, unsigned bit) {
+  if (*(volatile unsigned *)&s->bits & bit) return;
+  if (!(atomicOr(&s->bits, bit) & bit) && s->host) atomicOr(s->host, bit);
+}
 
 // Everything a kernel needs from the parameter block, passed by value so
 // that every launch carries its own copy (no __constant__ upload, and graph
@@ -54,8 +69,8 @@ struct Context {
   SimParams params{};
   int radiusFromW = 0;
   int morton = 0;               // fcdemSetCellOrder
-  unsigned *dStatus = nullptr;  // one word of kStatus* bits (mapped host memory) ...
-  unsigned *hStatus = nullptr;  // ... as the host sees it
+  DeviceStatus *dStatus = nullptr;  // in device memory ...
+  unsigned *hStatus = nullptr;      // ... and its host word, as the host sees it
   void *scratch = nullptr;      // grown on demand, never shrunk
   size_t scratchBytes = 0;
   void *countBuf = nullptr;     // counting-sort pipeline of fcdemUpdate
@@ -82,9 +97,9 @@ unsigned sortWaitLimit();
 // Whether a set look-back limit or a choice for n's size class and the key
 // width asks for the radix sort.
 bool radixSortAsked(unsigned n, int bits);
-// The status word of the allocation-free sort on the current device, or
-// nullptr when that sort has not been set up there (fcdem_sort.cu).
-unsigned *noAllocStatusWord();
+// The status of the allocation-free sort on the current device (without a host
+// word), or nullptr when that sort has not been set up there (fcdem_sort.cu).
+DeviceStatus *noAllocStatus();
 // The stream this host thread issues work on (fcdemSetStream; default: the
 // legacy default stream, as the reference).
 cudaStream_t curStream();

@@ -769,7 +769,7 @@ template <int H> constexpr int inferLd() { return H == 64 ? 2 : 4; }
 template <int H, int L>
 __global__ void __launch_bounds__(128 * kInferTiles)
 kSdfInfer(SdfView net, const float4 *__restrict__ pts, const int *__restrict__ shapes,
-          unsigned n, float *__restrict__ dOut, unsigned *status) {
+          unsigned n, float *__restrict__ dOut, DeviceStatus *status) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   SdfTileSmem<H, L, kInferTiles> &sm =
       *reinterpret_cast<SdfTileSmem<H, L, kInferTiles> *>(smraw);
@@ -785,7 +785,7 @@ kSdfInfer(SdfView net, const float4 *__restrict__ pts, const int *__restrict__ s
     if (!sdfTileForward<H, L, inferLd<H>(), kInferTiles>(
             sm, net, (q.x - net.shift[0]) * net.scale[0], (q.y - net.shift[1]) * net.scale[1],
             (q.z - net.shift[2]) * net.scale[2], shape, phase, d)) {
-      if ((threadIdx.x & 127u) == 0) atomicOr(status, (unsigned)kStatusTimeout);
+      if ((threadIdx.x & 127u) == 0) report(status, kStatusTimeout);
       break;
     }
     if (valid) dOut[i] = d;
@@ -930,7 +930,7 @@ kIntegrateSdf(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt, unsi
               KParams kp, MapView M, SdfView net, float skin, unsigned *exact,
               unsigned *__restrict__ hashOut, unsigned *__restrict__ rankOut,
               unsigned *__restrict__ cnt, unsigned *__restrict__ tileCnt, TileHints hints,
-              unsigned *status) {
+              DeviceStatus *status) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   SdfTileSmem<H, L> &sm = *reinterpret_cast<SdfTileSmem<H, L> *>(smraw);
   sdfTileSetup<H, L>(sm, net);
@@ -958,7 +958,7 @@ kIntegrateSdf(float4 *__restrict__ pos, float4 *__restrict__ vel, float dt, unsi
         !sdfTileForward<H, L>(sm, net, (p.x - net.shift[0]) * net.scale[0],
                               (p.y - net.shift[1]) * net.scale[1],
                               (p.z - net.shift[2]) * net.scale[2], 0, phase, dPred)) {
-      if (threadIdx.x == 0) atomicOr(status, (unsigned)kStatusTimeout);
+      if (threadIdx.x == 0) report(status, kStatusTimeout);
       break;
     }
     const bool test = inBox && (!useNet || !(dPred > skin));
@@ -1007,7 +1007,7 @@ kBatchObstacle(const BatchScene *__restrict__ scenes, const unsigned *__restrict
                const MapView *__restrict__ maps, SdfView net, float skin,
                const float4 *__restrict__ inPos, float4 *__restrict__ pos,
                float4 *__restrict__ vel, float dt, unsigned n, UmCount count, int doCount,
-               unsigned *exact, TileHints hints, TileCull tc, unsigned *status) {
+               unsigned *exact, TileHints hints, TileCull tc, DeviceStatus *status) {
   extern __shared__ __align__(1024) unsigned char smraw[];
   SdfTileSmem<H, L> &sm = *reinterpret_cast<SdfTileSmem<H, L> *>(smraw);
   if (kNet) sdfTileSetup<H, L>(sm, net);
@@ -1039,7 +1039,7 @@ kBatchObstacle(const BatchScene *__restrict__ scenes, const unsigned *__restrict
           !sdfTileForward<H, L>(sm, net, (p.x - net.shift[0]) * net.scale[0],
                                 (p.y - net.shift[1]) * net.scale[1],
                                 (p.z - net.shift[2]) * net.scale[2], shape, phase, dPred)) {
-        if (threadIdx.x == 0) atomicOr(status, (unsigned)kStatusTimeout);
+        if (threadIdx.x == 0) report(status, kStatusTimeout);
         break;
       }
     }

@@ -102,7 +102,7 @@ constexpr int kUpWarps = kThreads / 32;
 constexpr int kUpKeys = 4;
 __global__ void __launch_bounds__(kThreads)
 kUpsweep(const unsigned *__restrict__ keys, unsigned n, int passes, int bits,
-         unsigned *__restrict__ hist, unsigned *__restrict__ status) {
+         unsigned *__restrict__ hist, DeviceStatus *status) {
   __shared__ unsigned sh[kUpWarps][kMaxPasses][kRadix];
   for (int k = threadIdx.x; k < kUpWarps * kMaxPasses * kRadix; k += kThreads)
     (&sh[0][0][0])[k] = 0;
@@ -138,7 +138,7 @@ kUpsweep(const unsigned *__restrict__ keys, unsigned n, int passes, int bits,
       }
     }
   }
-  if (bad) atomicOr(status, (unsigned)kStatusKeyRange);
+  if (bad) report(status, kStatusKeyRange);
   __syncthreads();
   for (int e = threadIdx.x; e < passes * kRadix; e += kThreads) {
     unsigned c = 0;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(THREADS, MINB)
 kOnesweep(const unsigned *__restrict__ keysIn, const unsigned *__restrict__ valsIn,
           unsigned *__restrict__ keysOut, unsigned *__restrict__ valsOut,
           unsigned n, int shift, const unsigned *__restrict__ hist,
-          unsigned *lookback, unsigned *tileCounter, unsigned *status, unsigned waitRounds) {
+          unsigned *lookback, unsigned *tileCounter, DeviceStatus *status, unsigned waitRounds) {
   static_assert(THREADS >= kRadix, "one thread per digit in the scan phases");
   constexpr int kWarps = THREADS / 32;
   constexpr int kTileKeys = THREADS * ITEMS;
@@ -242,7 +242,7 @@ kOnesweep(const unsigned *__restrict__ keysIn, const unsigned *__restrict__ vals
       bool done = false;
       for (unsigned round = 0; !done; ++round) {
         if (round >= waitRounds) {
-          atomicOr(status, (unsigned)kStatusTimeout);
+          report(status, kStatusTimeout);
           break;
         }
         unsigned w[kLookWindow];
@@ -311,7 +311,7 @@ struct PassConfig {
   int threads, items;
   size_t smem;
   void (*kernel)(const unsigned *, const unsigned *, unsigned *, unsigned *, unsigned, int,
-                 const unsigned *, unsigned *, unsigned *, unsigned *, unsigned);
+                 const unsigned *, unsigned *, unsigned *, DeviceStatus *, unsigned);
   int tile() const { return threads * items; }
 };
 
@@ -505,8 +505,8 @@ constexpr int kNoAllocMaxDevices = 64;
 std::mutex g_noAllocMutex;
 unsigned char *g_noAllocPtr[kNoAllocMaxDevices] = {};
 
-unsigned *statusIn(unsigned char *scratch) {
-  return (unsigned *)(scratch + 4 * kNoAllocArr + kNoAllocHist + kNoAllocLookback);
+DeviceStatus *statusIn(unsigned char *scratch) {
+  return (DeviceStatus *)(scratch + 4 * kNoAllocArr + kNoAllocHist + kNoAllocLookback);
 }
 
 // Device address of the scratch on the current device, looked up once per
@@ -525,7 +525,7 @@ unsigned char *noAllocScratch() {
       setError(FCDEM_ERR_CUDA);
       return nullptr;
     }
-    if (!clearNow(statusIn((unsigned char *)p), 0, sizeof(unsigned))) return nullptr;
+    if (!clearNow(statusIn((unsigned char *)p), 0, sizeof(DeviceStatus))) return nullptr;
     g_noAllocPtr[dev] = (unsigned char *)p;
   }
   return g_noAllocPtr[dev];
@@ -533,7 +533,7 @@ unsigned char *noAllocScratch() {
 
 }  // namespace
 
-unsigned *noAllocStatusWord() {
+DeviceStatus *noAllocStatus() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
     cudaGetLastError();
@@ -584,7 +584,7 @@ extern "C" void fcdemSortParticlesNoAlloc(uint *dGridParticleHash, uint *dGridPa
   unsigned *hist = (unsigned *)meta;
   unsigned *counters = hist + kMaxPasses * kRadix;
   unsigned *lookback = (unsigned *)(meta + kNoAllocHist);
-  unsigned *status = statusIn(s);
+  DeviceStatus *status = statusIn(s);
   cudaStream_t st = curStream();
   // The array keeps whatever the previous call left; the histograms, tile
   // counters and look-back flags must start at zero.  (The status word is

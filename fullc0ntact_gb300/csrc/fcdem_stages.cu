@@ -98,7 +98,7 @@ kReorder(unsigned *cellStart, unsigned *cellEnd,
          float4 *sortedPos, float4 *sortedVel,
          const unsigned *hash, const unsigned *index,
          const float4 *oldPos, const float4 *oldVel,
-         unsigned n, unsigned numCells, unsigned *status) {
+         unsigned n, unsigned numCells, DeviceStatus *status) {
   chainTrigger();
   chainWait();
   unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -108,7 +108,7 @@ kReorder(unsigned *cellStart, unsigned *cellEnd,
   // Hashes come from calcHash and are below numCells, indices below n; a
   // caller's array that breaks this is reported instead of written through.
   if (h >= numCells || s >= n) {
-    atomicOr(status, (unsigned)kStatusKeyRange);
+    report(status, kStatusKeyRange);
     return;
   }
   if (i == 0) {

@@ -86,6 +86,27 @@ def test_radius_bound_violation_is_reported():
         dem.check()
 
 
+@pytest.mark.parametrize("n", [5000, 40_000])
+def test_every_radius_out_of_bound_is_reported_after_each_clear(n):
+    """A scene that reports from every warp and step: the error is there after
+    each run, gone once read, and the states are those of the right bound."""
+    from fullc0ntact_gb300 import dem, scenes
+    sc = scenes.random_box(n, grid=(64, 64, 64), radius=1.0 / 64.0, seed=12, poly=True)
+    right, broken = dem.DeviceScene(sc), dem.DeviceScene(sc)
+    broken.params.particleRadius /= 4.0
+    try:
+        for steps in (1, 3):
+            right.update(steps)
+            assert dem.lib.fcdemGetLastError() == 0
+            broken.update(steps)
+            assert dem.lib.fcdemGetLastError() == 8  # FCDEM_ERR_RADIUS_BOUND
+            assert dem.lib.fcdemGetLastError() == 0
+            for a, b in ((right.pos, broken.pos), (right.vel, broken.vel)):
+                np.testing.assert_array_equal(a.cpu().numpy(), b.cpu().numpy())
+    finally:
+        dem.set_radius_mode(False)
+
+
 def _crowded_scene(kind):
     """Scenes with collapsed cells: thousands of particles in a few cells, the
     cells around them sparse or crowded too."""
