@@ -354,6 +354,8 @@ inline unsigned fixupMaxCell(unsigned n) { return n <= kFixupAllCells ? n : kFix
 // Capacity of the large-cell list: a listed cell has more than kFixupMaxCell
 // of the n particles, so at most n / (kFixupMaxCell + 1) cells are listed.
 inline unsigned largeCapacity(unsigned n) { return n / (kFixupMaxCell + 1) + 1; }
+// CTAs of kFixupLarge: one per SM at most.
+inline unsigned largeCtas(unsigned n) { return std::min(largeCapacity(n), numSms()); }
 
 // Stable order inside each cell + the reorder gather.  The particle of slot
 // s is re-ranked among its cell's members by particle index; its position and
@@ -398,37 +400,87 @@ kFixupGather(const uint4 *slots, const unsigned *off, unsigned *hashOut, unsigne
 // The same passes over (key, value) pairs: the key is the cell (its low `bits`
 // bits), the position in the arrays takes the particle index's place, and the
 // value travels in the slot, so the sort is stable and in place.
+//
+// Crowded cells.  A cell of at least `least` pairs (a giant: at most 256 of them)
+// would keep one CTA busy for long.  Its pairs are not ranked by slot but taken
+// in the order of the arrays: kScatterPairs leaves each one's slot in rank
+// (kGiantSlot set) and counts them per giant and part of the arrays, and
+// kFixupLarge scatters each part from there, one CTA each.  Sorts with giants /
+// before there were any / with the radix sort: 2M pairs of one key 139 / 5,936 /
+// 104 us, of four keys 140 / 1,500 / 104, 100,003 pairs of one key 35 / 305 / 58;
+// it costs a sort without giants about 1 us.  Cells between 1,025 pairs and a giant
+// stay with one CTA each, smaller ones with the ranking by slot: 2M pairs in cells
+// of 500, 1,000 and 20,000 take 241, 412 and 473 us (radix 110).
+constexpr unsigned kGiants = 256, kGiantSlot = 1u << 31;
+struct Giants {
+  unsigned *count;  // [giant][part]
+  unsigned *first;  // [giant]: first slot, or 0xffffffff
+  unsigned least;   // pairs in a giant
+  unsigned parts, part;  // parts of the arrays and their size
+  // giants begin at least `least` slots apart
+  __device__ __forceinline__ unsigned id(unsigned firstSlot) const { return firstSlot / least; }
+};
 
 template <bool kTiles>
 __global__ void __launch_bounds__(256)
 kCountKeys(const unsigned *keys, unsigned n, unsigned mask, unsigned *rank, unsigned *cnt,
-           unsigned *tileCnt, DeviceStatus *status) {
+           unsigned *tileCnt, Giants giants, DeviceStatus *status) {
   chainTrigger();
   chainWait();
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  for (unsigned k = i; k < kGiants * giants.parts; k += gridDim.x * blockDim.x) {
+    giants.count[k] = 0u;
+    if (k < kGiants) giants.first[k] = 0xffffffffu;
+  }
+  const unsigned live = __ballot_sync(0xffffffffu, i < n), lane = threadIdx.x & 31u;
   if (i >= n) return;
   const unsigned k = keys[i], h = k & mask;
   if (k != h) report(status, kStatusKeyRange);
-  rank[i] = atomicAdd(cnt + h, 1u);
+  // Where two lanes in a row share a cell, one atomic for the members of the warp
+  // that do: the pairs of a crowded cell would queue on its counter (2M pairs of
+  // one key: 5.8 ms the sort, with plain atomics and without giants; always
+  // looking for the members costs a sort of 1M pairs of many keys 4 us).
+  const unsigned up = __shfl_down_sync(live, h, 1);
+  if (__any_sync(live, lane < 31u && ((live >> (lane + 1u)) & 1u) && up == h)) {
+    const unsigned peers = __match_any_sync(live, h);
+    const int leader = __ffs((int)peers) - 1;
+    unsigned first = 0u;
+    if ((int)lane == leader) first = atomicAdd(cnt + h, (unsigned)__popc(peers));
+    rank[i] = __shfl_sync(live, first, leader) + __popc(peers & ((1u << lane) - 1u));
+  } else {
+    rank[i] = atomicAdd(cnt + h, 1u);
+  }
   if (kTiles) countTile(tileCnt, h >> kTileShift);
 }
 
 __global__ void __launch_bounds__(256)
-kScatterPairs(const unsigned *keys, const unsigned *vals, const unsigned *rankN,
-              const unsigned *off, uint4 *slots, unsigned n, unsigned mask, unsigned *tileCnt,
-              unsigned tiles) {
+kScatterPairs(const unsigned *keys, const unsigned *vals, unsigned *rankN, const unsigned *off,
+              uint4 *slots, unsigned n, unsigned mask, unsigned *tileCnt, unsigned tiles,
+              Giants giants) {
   chainTrigger();
   chainWait();
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   for (unsigned k = i; k < tiles; k += gridDim.x * blockDim.x) tileCnt[k] = 0u;
+  const unsigned live = __ballot_sync(0xffffffffu, i < n), lane = threadIdx.x & 31u;
   if (i >= n) return;
-  const unsigned k = keys[i], a = off[k & mask], s = a + rankN[i];
+  const unsigned k = keys[i], a = off[k & mask], b = off[(k & mask) + 1u], r = rankN[i], s = a + r;
   if (s < n) slots[s] = make_uint4(k, i, vals[i], a);
+  const bool giant = b - a >= giants.least;
+  const unsigned inGiants = __ballot_sync(live, giant);
+  if (!giant) return;
+  const unsigned id = giants.id(a), part = i / giants.part;
+  rankN[i] = kGiantSlot | s;
+  if (r == 0u) giants.first[id] = a;
+  // (a warp may lie in two parts)
+  const unsigned peers = __match_any_sync(inGiants, id * giants.parts + part);
+  if ((int)lane == __ffs((int)peers) - 1)
+    atomicAdd(giants.count + id * giants.parts + part, (unsigned)__popc(peers));
 }
 
 __global__ void __launch_bounds__(256)
 kFixupPairs(const uint4 *slots, const unsigned *off, unsigned *keys, unsigned *vals, unsigned n,
-            unsigned mask, unsigned maxCell, unsigned *large, unsigned largeCap, DeviceStatus *status) {
+            unsigned mask, unsigned maxCell, unsigned least, unsigned *large, unsigned largeCap,
+            DeviceStatus *status) {
   chainTrigger();
   chainWait();
   const unsigned s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -436,8 +488,8 @@ kFixupPairs(const uint4 *slots, const unsigned *off, unsigned *keys, unsigned *v
   const uint4 w = slots[s];
   const unsigned h = w.x & mask, a = w.w, b = min(off[h + 1], n);
   if (a > s) return;
-  if (b - a > maxCell) {
-    if (s == a) {
+  if (b - a > maxCell) {  // for kFixupLarge
+    if (s == a && b - a < least) {
       const unsigned k = atomicAdd(large, 1u);
       if (k < largeCap)
         large[1 + k] = h;
@@ -447,6 +499,7 @@ kFixupPairs(const uint4 *slots, const unsigned *off, unsigned *keys, unsigned *v
     return;
   }
   unsigned r = 0;
+#pragma unroll 32  // eight slots a line: several lines on their way
   for (unsigned t = a; t < b; ++t) r += slots[t].y < w.y ? 1u : 0u;
   if (a + r >= n) return;
   keys[a + r] = w.x;
@@ -526,22 +579,11 @@ __device__ void bitmapRanks(const uint4 *slots, unsigned a, unsigned c, unsigned
   __syncthreads();
 }
 
-// One stable pass of a block-wide LSD radix sort: src[0..c) -> dst[0..c)
-// by the 8-bit digit at bit `shift`.  Chunks of kLargeThreads entries go in
-// order; inside a chunk an entry's place is its digit's running base + the
-// count of that digit in earlier warps + its rank among its warp's peers.
-__device__ void largeRadixPass(const unsigned long long *src, unsigned long long *dst,
-                               unsigned c, int shift, LargeSmem &sm) {
+// Exclusive prefix sums of 256 counts (thread d < 256: digit d's).
+__device__ __forceinline__ unsigned digitScan(unsigned v, LargeSmem &sm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid < 256) sm.bin[tid] = 0u;
-  __syncthreads();
-  for (unsigned t = tid; t < c; t += kLargeThreads)
-    atomicAdd(&sm.bin[(unsigned)(src[t] >> shift) & 255u], 1u);
-  __syncthreads();
-  unsigned v = 0, x = 0;
-  if (tid < 256) {  // exclusive scan of the 256 digit counts, warps 0..7
-    v = sm.bin[tid];
-    x = v;
+  unsigned x = v;
+  if (tid < 256) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       unsigned y = __shfl_up_sync(0xffffffffu, x, o);
@@ -550,20 +592,29 @@ __device__ void largeRadixPass(const unsigned long long *src, unsigned long long
     if (lane == 31) sm.part[warp] = x;
   }
   __syncthreads();
-  if (tid < 256) {
-    unsigned before = 0;
+  unsigned before = 0;
+  if (tid < 256)
     for (int w = 0; w < warp; ++w) before += sm.part[w];
-    sm.bin[tid] = before + x - v;
-  }
   __syncthreads();
+  return before + x - v;
+}
+
+// Entries 0 .. c-1 in order, each to the next free place of its digit (sm.bin[d]
+// on entry).  load(t, e) returns the digit of entry t (256: leave it out) and the
+// entry in e.  Chunks of kLargeThreads entries go in order; inside a chunk an entry's place is its
+// digit's running base + the count of that digit in earlier warps + its rank
+// among its warp's peers.
+template <class Load, class Store>
+__device__ __forceinline__ void stableScatter(unsigned c, LargeSmem &sm, Load load, Store store) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const unsigned lt = (1u << lane) - 1u;
   for (unsigned base = 0; base < c; base += kLargeThreads) {
     for (int q = tid; q < kLargeWarps * 256; q += kLargeThreads) (&sm.warpCnt[0][0])[q] = 0u;
     __syncthreads();
     const unsigned t = base + tid;
-    const bool valid = t < c;
-    const unsigned long long e = valid ? src[t] : 0ull;
-    const unsigned d = valid ? ((unsigned)(e >> shift) & 255u) : 256u;
+    unsigned long long e = 0ull;
+    const unsigned d = t < c ? load(t, e) : 256u;
+    const bool valid = d < 256u;
     const unsigned peers = __match_any_sync(0xffffffffu, d);
     const unsigned rank = __popc(peers & lt);
     if (valid && rank == 0) sm.warpCnt[warp][d] = __popc(peers);
@@ -578,11 +629,33 @@ __device__ void largeRadixPass(const unsigned long long *src, unsigned long long
       sm.total[tid] = run;
     }
     __syncthreads();
-    if (valid) dst[sm.bin[d] + sm.warpCnt[warp][d] + rank] = e;
+    if (valid) store(sm.bin[d] + sm.warpCnt[warp][d] + rank, e);
     __syncthreads();
     if (tid < 256) sm.bin[tid] += sm.total[tid];
     __syncthreads();
   }
+}
+
+// One stable pass of a block-wide LSD radix sort: src[0..c) -> dst[0..c)
+// by the 8-bit digit at bit `shift`.
+__device__ void largeRadixPass(const unsigned long long *src, unsigned long long *dst,
+                               unsigned c, int shift, LargeSmem &sm) {
+  const int tid = threadIdx.x;
+  if (tid < 256) sm.bin[tid] = 0u;
+  __syncthreads();
+  for (unsigned t = tid; t < c; t += kLargeThreads)
+    atomicAdd(&sm.bin[(unsigned)(src[t] >> shift) & 255u], 1u);
+  __syncthreads();
+  const unsigned first = digitScan(tid < 256 ? sm.bin[tid] : 0u, sm);
+  if (tid < 256) sm.bin[tid] = first;
+  __syncthreads();
+  stableScatter(
+      c, sm,
+      [&](unsigned t, unsigned long long &e) {
+        e = src[t];
+        return (unsigned)(e >> shift) & 255u;
+      },
+      [&](unsigned at, unsigned long long e) { dst[at] = e; });
 }
 
 // The large cells listed by kFixupGather, one CTA per cell at a time.  A
@@ -604,10 +677,39 @@ kFixupLarge(uint4 *slots, const unsigned *off, const unsigned *large,
             unsigned largeCap, unsigned *hashOut, unsigned *indexOut,
             float4 *sortedPos, float4 *sortedVel,
             const float4 *prevPos, const float4 *prevVel, unsigned n,
-            int idBits, unsigned *bitmaps, const unsigned *rank) {
+            int idBits, unsigned *bitmaps, const unsigned *rank, Giants giants) {
   chainTrigger();
   chainWait();
   __shared__ LargeSmem sm;
+  if (kPairs) {
+    // this CTA's part of the arrays: the pairs in giants
+    const unsigned first = threadIdx.x < kGiants ? giants.first[threadIdx.x] : 0xffffffffu;
+    if (__syncthreads_or(first != 0xffffffffu)) {
+      if (threadIdx.x < kGiants) {
+        unsigned before = 0;
+        if (first != 0xffffffffu)
+          for (unsigned p = 0; p < blockIdx.x; ++p)
+            before += giants.count[threadIdx.x * giants.parts + p];
+        sm.bin[threadIdx.x] = first + before;
+      }
+      __syncthreads();
+      const unsigned lo = min(n, blockIdx.x * giants.part), c = min(n, lo + giants.part) - lo;
+      stableScatter(
+          c, sm,
+          [&](unsigned t, unsigned long long &e) {
+            const unsigned r = rank[lo + t];
+            if (!(r & kGiantSlot)) return 256u;
+            const uint4 w = slots[r & ~kGiantSlot];
+            e = ((unsigned long long)w.x << 32) | w.z;
+            return giants.id(w.w);
+          },
+          [&](unsigned at, unsigned long long e) {
+            if (at >= n) return;
+            hashOut[at] = (unsigned)(e >> 32);
+            indexOut[at] = (unsigned)e;
+          });
+    }
+  }
   const unsigned count = min(large[0], largeCap);
   const int tid = threadIdx.x;
   const size_t words = bitmapWords(n);
@@ -683,22 +785,21 @@ kFixupLarge(uint4 *slots, const unsigned *off, const unsigned *large,
         hashOut[a + t] = slots[a + rank[(unsigned)(e >> 32)]].x;
         indexOut[a + t] = (unsigned)e;
       }
+    } else {
+      for (unsigned t = tid; t < c; t += kLargeThreads) {
+        const unsigned long long e = A[t];
+        slots[a + t].y = (unsigned)(e >> 32);
+        slots[a + t].z = (unsigned)e;
+      }
       __syncthreads();
-      continue;
-    }
-    for (unsigned t = tid; t < c; t += kLargeThreads) {
-      const unsigned long long e = A[t];
-      slots[a + t].y = (unsigned)(e >> 32);
-      slots[a + t].z = (unsigned)e;
-    }
-    __syncthreads();
-    for (unsigned t = tid; t < c; t += kLargeThreads) {
-      const unsigned me = slots[a + t].y, prev = slots[a + t].z;
-      if (me >= n || prev >= n) continue;  // unfilled slot (reported by the scatter)
-      hashOut[a + t] = h;
-      indexOut[a + t] = me;
-      sortedPos[a + t] = prevPos[prev];
-      sortedVel[a + t] = prevVel[prev];
+      for (unsigned t = tid; t < c; t += kLargeThreads) {
+        const unsigned me = slots[a + t].y, prev = slots[a + t].z;
+        if (me >= n || prev >= n) continue;  // unfilled slot (reported by the scatter)
+        hashOut[a + t] = h;
+        indexOut[a + t] = me;
+        sortedPos[a + t] = prevPos[prev];
+        sortedVel[a + t] = prevVel[prev];
+      }
     }
     __syncthreads();
   }
@@ -966,15 +1067,17 @@ bool countPipelineSort(Context &c, const CountBuffers &b, const unsigned *origOf
   if (!launchOk()) return false;
   if (n <= kFixupAllCells) return true;  // no cell is left
   // Returns at once when the fix-up listed no cell (the common case).
-  const unsigned largeCtas = b.largeCap < numSms() ? b.largeCap : numSms();  // one per SM at most
-  launchChained(true, kFixupLarge<false>, largeCtas, kLargeThreads, 0, b.slots, b.off, b.large,
+  launchChained(true, kFixupLarge<false>, largeCtas(n), kLargeThreads, 0, b.slots, b.off, b.large,
                 b.largeCap, hash, index, sortedPos, sortedVel, prevPos, prevVel, n,
-                keyBits(n), b.bitmaps, nullptr);
+                keyBits(n), b.bitmaps, nullptr, Giants{});
   return launchOk();
 }
 
 static_assert(((1u << kCountSortBits) >> kTileShift) + 1 <= kTilesOwnPrefix, "tiles of a key width");
 constexpr unsigned kCountSortMax = 1u << 21;  // pairs
+// Pairs per cell.  Fuller tables are left to the radix sort, whatever the keys: 2M
+// pairs over 512 cells 484 us here, 85 there, 100,003 (195 a cell) 48 each.
+constexpr unsigned kCountSortFill = 64;
 
 // Buffers of countSortPairs.  A recorded graph may hold their addresses, so
 // they live as long as those of the radix sort: each key width has its own
@@ -991,8 +1094,9 @@ static bool sortBuffers(Context &c, unsigned n, int bits, CountBuffers &b) {
   const unsigned largeCap = largeCapacity(n);
   const size_t cellBytes = al(m * 4), tileBytes = al((size_t)tiles * 4);
   const size_t rankBytes = al((size_t)n * 4), slotBytes = al((size_t)n * 16),
-               largeBytes = al(((size_t)largeCap + 1) * 4);
-  const size_t pairBytes = std::max(rankBytes + 2 * slotBytes + largeBytes +
+               largeBytes = al(((size_t)largeCap + 1) * 4),
+               giantBytes = (size_t)kGiants * (largeCtas(n) + 1) * 4;
+  const size_t pairBytes = std::max(rankBytes + 2 * slotBytes + largeBytes + giantBytes +
                                         (size_t)kBitmapSlots * 2 * bitmapWords(n) * 4,
                                     radixScratchBytes(n));
   void *&tables = c.sortTables[bits];
@@ -1032,14 +1136,16 @@ static bool sortBuffers(Context &c, unsigned n, int bits, CountBuffers &b) {
   b.rank = (unsigned *)(p + 2 * slotBytes);
   b.large = (unsigned *)(p + 2 * slotBytes + rankBytes);
   b.largeCap = largeCap;
-  b.bitmaps = (unsigned *)(p + 2 * slotBytes + rankBytes + largeBytes);
+  b.giants = (unsigned *)(p + 2 * slotBytes + rankBytes + largeBytes);
+  b.bitmaps = (unsigned *)(p + 2 * slotBytes + rankBytes + largeBytes + giantBytes);
   return true;
 }
 
 // sortParticles' stable sort of n (key, value) pairs by the low `bits` bits as
 // a counting sort over 2^bits cells, in place; keys with higher bits raise
-// kStatusKeyRange.  False (nothing done): more than kCountSortBits bits or
-// kCountSortMax pairs, or no buffers -- the radix sort then takes the pairs.
+// kStatusKeyRange.  False (nothing done): more than kCountSortBits bits,
+// kCountSortMax pairs or kCountSortFill pairs per cell, or no buffers -- the radix
+// sort then takes the pairs.
 // Five short passes instead of a histogram and three look-back passes of eight
 // bits, whose chain over the tiles is what they wait for.  A staged step with
 // it / with the radix sort: 5,000 spheres 39 / 60 us, 100,003 75 / 89, 1M in
@@ -1047,14 +1153,23 @@ static bool sortBuffers(Context &c, unsigned n, int bits, CountBuffers &b) {
 // the bound).  The fused step's buffers are others: it may run on another
 // stream.
 bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int bits) {
-  if (bits > kCountSortBits || n > kCountSortMax) return false;
+  if (bits > kCountSortBits || n > kCountSortMax || (n >> bits) > kCountSortFill) return false;
   const unsigned cells = 1u << bits, mask = cells - 1u;
   CountBuffers b;
   if (!sortBuffers(c, n, bits, b)) return false;
   const unsigned blocks = (n + 255) / 256;
-  const bool tiles = n <= kTileAtomicsMax;
+  const bool tiles = n <= kTileAtomicsMax, large = n > kFixupAllCells;
+  Giants giants{};
+  giants.least = ~0u;
+  if (large) {
+    giants.parts = largeCtas(n);
+    giants.part = (n + giants.parts - 1) / giants.parts;
+    giants.count = b.giants;
+    giants.first = b.giants + kGiants * giants.parts;
+    giants.least = std::max((n + kGiants - 1) / kGiants, kFixupMaxCell + 1);
+  }
   launchChained(true, tiles ? kCountKeys<true> : kCountKeys<false>, blocks, 256, 0, keys, n, mask,
-                b.rank, b.cnt, b.tileCnt, c.dStatus);
+                b.rank, b.cnt, b.tileCnt, giants, c.dStatus);
   if (!launchOk()) return true;  // recorded
   if (!tiles) {
     launchChained(true, kTileReduce, b.scanTiles, kScanThreads, 0, b.cnt, b.tileCnt, cells + 1);
@@ -1064,16 +1179,14 @@ bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int 
                 b.tileOffPrev, b.large, nullptr);
   if (!launchOk()) return true;
   launchChained(true, kScatterPairs, blocks, 256, 0, keys, vals, b.rank, b.off, b.slots, n, mask,
-                b.tileCnt, b.scanTiles);
+                b.tileCnt, b.scanTiles, giants);
   if (!launchOk()) return true;
   launchChained(true, kFixupPairs, blocks, 256, 0, b.slots, b.off, keys, vals, n, mask,
-                fixupMaxCell(n), b.large,
-                b.largeCap, c.dStatus);
-  if (!launchOk() || n <= kFixupAllCells) return true;
-  const unsigned largeCtas = b.largeCap < numSms() ? b.largeCap : numSms();
-  launchChained(true, kFixupLarge<true>, largeCtas, kLargeThreads, 0, b.slots, b.off, b.large,
+                fixupMaxCell(n), giants.least, b.large, b.largeCap, c.dStatus);
+  if (!launchOk() || !large) return true;
+  launchChained(true, kFixupLarge<true>, largeCtas(n), kLargeThreads, 0, b.slots, b.off, b.large,
                 b.largeCap, keys, vals, (float4 *)b.work, nullptr, nullptr, nullptr, n, keyBits(n),
-                b.bitmaps, b.rank);
+                b.bitmaps, b.rank, giants);
   launchOk();
   return true;
 }

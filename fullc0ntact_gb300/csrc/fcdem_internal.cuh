@@ -268,6 +268,7 @@ struct CountBuffers {
   unsigned *large;              // [0] = count, [1..largeCap] = cells too full for the re-rank
   unsigned *tileBlockSum;       // per 1024 tiles: their total (many-tile scans)
   void *work;                   // countSortPairs: 16 bytes of work space per pair
+  unsigned *giants;             // countSortPairs: counts and first slots of its giant cells
   unsigned *bitmaps;            // kFixupLarge: per-CTA bitmap + word prefix of particle indices
   unsigned scanTiles, largeCap;
 };

@@ -185,7 +185,8 @@ def test_counting_and_radix_sort_agree(n, cells):
     np.testing.assert_array_equal(v, rv)
 
 
-@pytest.mark.parametrize("n,cells", [(200_000, 64), (60_000, 4), (300_000, 2 ** 12), (3000, 2)])
+@pytest.mark.parametrize("n,cells", [(200_000, 64), (60_000, 4), (300_000, 2 ** 12), (3000, 2),
+                                     (100_000, 2 ** 9)])
 def test_keys_above_the_width_are_kept(n, cells):
     """Keys with bits above the sorted width are reported, and the pairs come back
     whole, in stable order of their low bits, however large their cells are.
@@ -200,8 +201,9 @@ def test_keys_above_the_width_are_kept(n, cells):
     P = make_params(n, (2, 2, 2), 0.01)
     P.numCells = cells
     dem.set_parameters(P)
-    whole = 8 * -(-(cells - 1).bit_length() // 8)  # the radix sort's bits
-    for config, bits in ((-1, (cells - 1).bit_length()), (0, whole)):
+    width = (cells - 1).bit_length()
+    whole = 8 * -(-width // 8)  # the radix sort's bits
+    for config in (-1, 0):  # the default and the radix sort
         dem.lib.fcdemSetSortConfig(n, config)
         try:
             k = torch.from_numpy(keys.view(np.int32).copy()).cuda()
@@ -210,9 +212,11 @@ def test_keys_above_the_width_are_kept(n, cells):
             assert dem.lib.fcdemGetLastError() == 6  # FCDEM_ERR_KEY_RANGE
         finally:
             dem.lib.fcdemSetSortConfig(n, -1)
-        o = np.argsort(keys & np.uint32((1 << bits) - 1), kind="stable")
-        np.testing.assert_array_equal(k.cpu().numpy().view(np.uint32), keys[o])
-        np.testing.assert_array_equal(v.cpu().numpy().view(np.uint32), vals[o])
+        got = k.cpu().numpy().view(np.uint32), v.cpu().numpy().view(np.uint32)
+        orders = [np.argsort(keys & np.uint32((1 << bits) - 1), kind="stable")
+                  for bits in ((width, whole) if config < 0 else (whole,))]
+        assert any(np.array_equal(got[0], keys[o]) and np.array_equal(got[1], vals[o])
+                   for o in orders)
 
 
 def _launches(n, cells):
@@ -246,3 +250,33 @@ def test_autotuned_index_names_the_kept_sort(n, cells):
         assert _launches(n, cells) == kept
     finally:
         lib.fcdemSetSortConfig(n, -1)
+
+
+@pytest.mark.parametrize("n,cells", [(3000, 64), (4096, 2 ** 20), (4097, 256), (5000, 2 ** 13),
+                                     (155_649, 2 ** 13), (300_001, 3 * 2 ** 18),
+                                     (2 ** 21 - 1, 2 ** 16), (2 ** 21, 2 ** 24)])
+def test_crowded_cells(n, cells):
+    """Cells on both sides of the sizes at which another kernel takes their pairs
+    (1,024 and n / 256 pairs), several of them, and cells of a few hundred, in
+    random order and in runs, against the CPU's stable sort."""
+    rng = np.random.default_rng(n + cells)
+    giant = max(-(-n // 256), 1025)
+    kinds = {
+        "one cell": np.full(n, cells - 1),
+        "half in one": np.where(rng.random(n) < 0.5, 7, rng.integers(0, cells, n)),
+        "three cells": rng.integers(0, 3, n) * (cells // 3),
+        "256 each": rng.integers(0, max(1, n // 256), n) % cells,
+        "257 each, in runs": (np.arange(n) // 257) % cells,
+        "as many giants as there can be": np.minimum(rng.permutation(n) // giant, cells - 1),
+    }
+    for members in {1024, 1025, giant - 1, giant, giant + 1}:
+        k = rng.integers(1, cells, n)
+        k[rng.permutation(n)[: min(members, n)]] = 0
+        kinds[f"a cell of {members}"] = k
+    vals = rng.integers(0, 2 ** 32, n, dtype=np.uint64).astype(np.uint32)
+    for name, keys in kinds.items():
+        keys = keys.astype(np.uint32)
+        k, v = _sort_gpu(keys, vals, cells)
+        rk, rv = _sort_cpu(keys, vals)
+        np.testing.assert_array_equal(k, rk, err_msg=name)
+        np.testing.assert_array_equal(v, rv, err_msg=name)
