@@ -19,7 +19,9 @@
 //     have the same one.  Each vertex points to such a neighbour with a lower
 //     index; the solid angles are summed at the vertices without one (the
 //     roots, a thin shell around the surface) and the others take their
-//     root's sign.  In a mesh with a boundary every vertex is a root.
+//     root's sign.  In a mesh with a boundary every vertex is a root, and where
+//     the roots' list and the distances beside it (13 bytes per vertex) cannot be
+//     had: a map needs no more device memory than its vertices and triangles.
 //
 // Both kernels are bound by instruction issue.  The 128-cell map of a torus
 // mesh of 32,768 triangles, host work and the vertices' copy to the host
@@ -172,8 +174,9 @@ __device__ __forceinline__ float gap(float lo, float hi, float a, float b) {
 // closestOnTriangle and of the box distances.
 constexpr int kNearWarps = 4;
 __global__ void __launch_bounds__(32 * kNearWarps)
-kMeshNearest(float4 *__restrict__ vert, float *__restrict__ dist, Lattice L, const float4 *__restrict__ tri, unsigned nt,
-             const float4 *__restrict__ box, float slack) {
+kMeshNearest(float4 *__restrict__ vert, float *__restrict__ dist, Lattice L,
+             const float4 *__restrict__ tri, unsigned nt, const float4 *__restrict__ box,
+             float slack) {
   __shared__ float4 sTri[kNearWarps][3 * kCluster];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const int bx = (L.vx + 3) / 4, by = (L.vy + 3) / 4, bz = (L.vz + 1) / 2;
@@ -271,15 +274,14 @@ kMeshNearest(float4 *__restrict__ vert, float *__restrict__ dist, Lattice L, con
     const long long v = ((long long)k * L.vy + j) * L.vx + i;
     const float d = sqrtf(best);
     vert[v] = make_float4(d, bestCp.x, bestCp.y, bestCp.z);
-    dist[v] = d;
+    if (dist) dist[v] = d;
   }
 }
 
 // The lower neighbour whose sign vertex v shares, or -1 (v is a root): the
 // segment between the two is shorter than one end's distance to the mesh.
 __device__ __forceinline__ long long signParent(const float *__restrict__ dist, const Lattice &L,
-                                                long long v, bool closed) {
-  if (!closed) return -1;
+                                                long long v) {
   const float step = L.cs * 1.001f;
   const long long sy = L.vx, sz = (long long)L.vx * L.vy;
   const float d = __ldg(dist + v);
@@ -292,11 +294,11 @@ __device__ __forceinline__ long long signParent(const float *__restrict__ dist, 
 
 // Lists the roots.
 __global__ void __launch_bounds__(256)
-kMeshRoots(const float *__restrict__ dist, Lattice L, bool closed, long long *__restrict__ list,
+kMeshRoots(const float *__restrict__ dist, Lattice L, long long *__restrict__ list,
            unsigned long long *__restrict__ count) {
   const long long total = (long long)L.vx * L.vy * L.vz;
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool root = v < total && signParent(dist, L, v, closed) < 0;
+  const bool root = v < total && signParent(dist, L, v) < 0;
   const unsigned lane = threadIdx.x & 31u, m = __ballot_sync(0xffffffffu, root);
   unsigned long long at = 0;
   if (lane == 0 && m) at = atomicAdd(count, (unsigned long long)__popc(m));
@@ -305,20 +307,22 @@ kMeshRoots(const float *__restrict__ dist, Lattice L, bool closed, long long *__
 }
 
 // inside[v] of the listed roots: 32 roots per CTA at a time, one a lane, the
-// triangles shared out over the warps.
+// triangles shared out over the warps.  kAll: the sign of every vertex instead.
 constexpr int kWindWarps = 8;
+template <bool kAll>
 __global__ void __launch_bounds__(32 * kWindWarps)
 kMeshWinding(Lattice L, const float4 *__restrict__ tri, unsigned nt,
              const long long *__restrict__ list, const unsigned long long *__restrict__ count,
-             unsigned char *__restrict__ inside) {
+             unsigned char *__restrict__ inside, float4 *__restrict__ vert) {
   __shared__ float4 sTri[kWindWarps][3 * kCluster];
   __shared__ float sOmega[kWindWarps][32];
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  const unsigned long long n = *count;
+  const unsigned long long n = kAll ? (unsigned long long)L.vx * L.vy * L.vz : *count;
   const unsigned clusters = (nt + kCluster - 1) / kCluster;
   float4 *s = sTri[warp];
   for (unsigned long long base = blockIdx.x * 32u; base < n; base += gridDim.x * 32u) {
-    const long long v = __ldg(list + min(base + lane, n - 1ull));
+    const unsigned long long at = min(base + lane, n - 1ull);
+    const long long v = kAll ? (long long)at : __ldg(list + at);
     const float3 p = latticePoint(L, (int)(v % L.vx), (int)(v / L.vx % L.vy),
                                   (int)(v / ((long long)L.vx * L.vy)));
     float omega = 0.0f;
@@ -337,7 +341,11 @@ kMeshWinding(Lattice L, const float4 *__restrict__ tri, unsigned nt,
     __syncthreads();
     if (warp == 0 && base + lane < n) {
       for (int w = 1; w < kWindWarps; ++w) omega += sOmega[w][lane];
-      inside[v] = omega > 2.0f * 3.14159265358979f;  // winding number > 1/2
+      const bool in = omega > 2.0f * 3.14159265358979f;  // winding number > 1/2
+      if (!kAll)
+        inside[v] = in;
+      else if (in)
+        vert[v].x = -vert[v].x;
     }
     __syncthreads();
   }
@@ -346,13 +354,13 @@ kMeshWinding(Lattice L, const float4 *__restrict__ tri, unsigned nt,
 // The sign of every vertex, from its root (parents are found from the
 // unsigned distances).
 __global__ void __launch_bounds__(256)
-kMeshSign(float4 *__restrict__ vert, const float *__restrict__ dist, Lattice L, bool closed,
+kMeshSign(float4 *__restrict__ vert, const float *__restrict__ dist, Lattice L,
           const unsigned char *__restrict__ inside) {
   const long long total = (long long)L.vx * L.vy * L.vz;
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= total) return;
   long long r = v;
-  for (long long q = v; q >= 0; q = signParent(dist, L, r, closed)) r = q;
+  for (long long q = v; q >= 0; q = signParent(dist, L, r)) r = q;
   if (inside[r]) vert[v].x = -__ldg(dist + v);
 }
 
@@ -401,17 +409,22 @@ bool meshMap(fcdemDistanceMap *m, const float4 *tri, unsigned nt, const float *v
                listAt = boxAt + al((size_t)clusters * 32), distAt = listAt + al((size_t)total * 8),
                insideAt = distAt + al((size_t)total * 4), countAt = insideAt + al((size_t)total);
   char *buf = nullptr;
-  if (cudaMalloc(&buf, countAt + 256) != cudaSuccess) {
+  // without the per-vertex part every vertex is a root
+  bool roots = cudaMalloc(&buf, countAt + 256) == cudaSuccess;
+  if (!roots) {
     cudaGetLastError();
-    setError(FCDEM_ERR_ALLOC);
-    return false;
+    if (cudaMalloc(&buf, listAt) != cudaSuccess) {
+      cudaGetLastError();
+      setError(FCDEM_ERR_ALLOC);
+      return false;
+    }
   }
   unsigned *key = (unsigned *)buf, *order = key + nt;
-  long long *list = (long long *)(buf + listAt);
-  unsigned long long *count = (unsigned long long *)(buf + countAt);
   float4 *sorted = (float4 *)(buf + sortedAt), *box = (float4 *)(buf + boxAt);
-  float *dist = (float *)(buf + distAt);
-  unsigned char *inside = (unsigned char *)(buf + insideAt);
+  long long *list = roots ? (long long *)(buf + listAt) : nullptr;
+  float *dist = roots ? (float *)(buf + distAt) : nullptr;
+  unsigned char *inside = roots ? (unsigned char *)(buf + insideAt) : nullptr;
+  unsigned long long *count = roots ? (unsigned long long *)(buf + countAt) : nullptr;
   float3 scale;
   auto per = [&](int a) { return hi[a] > lo[a] ? 1024.0f / (hi[a] - lo[a]) : 0.0f; };
   scale = make_float3(per(0), per(1), per(2));
@@ -420,22 +433,29 @@ bool meshMap(fcdemDistanceMap *m, const float4 *tri, unsigned nt, const float *v
     extent = std::fmax(extent, std::fmax(std::fabs(m->vmin[a]), std::fabs(m->vmax[a])));
   const unsigned vBlocks = (unsigned)((total + 255) / 256);
   const long long bricks = (long long)((L.vx + 3) / 4) * ((L.vy + 3) / 4) * ((L.vz + 1) / 2);
-  bool ok = cudaOk(cudaMemsetAsync(count, 0, 8, st));
+  bool ok = !roots || cudaOk(cudaMemsetAsync(count, 0, 8, st));
   kMeshKeys<<<(nt + 255) / 256, 256, 0, st>>>(tri, nt, make_float3(lo[0], lo[1], lo[2]), scale, key,
                                              order);
   ok = ok && launchOk();
-  if (ok) radixSortPairs(ctx(), key, order, nt, 30);
+  // (in the caller's order the clusters are wide, and as right)
+  if (ok && scratch(ctx(), radixScratchBytes(nt), true)) radixSortPairs(ctx(), key, order, nt, 30);
   kMeshClusters<<<(clusters * 32 + 255) / 256, 256, 0, st>>>(tri, order, nt, sorted, box);
   ok = ok && launchOk();
   kMeshNearest<<<(unsigned)((bricks + kNearWarps - 1) / kNearWarps), 32 * kNearWarps, 0, st>>>(
       m->vert, dist, L, sorted, nt, box, 1e-5f * extent);
   ok = ok && launchOk();
-  const bool closed = meshClosed(vertices3, nv, triangles3, nt);  // meanwhile
-  kMeshRoots<<<vBlocks, 256, 0, st>>>(dist, L, closed, list, count);
-  ok = ok && launchOk();
-  kMeshWinding<<<numSms() * 4, 32 * kWindWarps, 0, st>>>(L, sorted, nt, list, count, inside);
-  ok = ok && launchOk();
-  kMeshSign<<<vBlocks, 256, 0, st>>>(m->vert, dist, L, closed, inside);
+  roots = meshClosed(vertices3, nv, triangles3, nt) && roots;  // meanwhile
+  if (roots) {
+    kMeshRoots<<<vBlocks, 256, 0, st>>>(dist, L, list, count);
+    ok = ok && launchOk();
+    kMeshWinding<false><<<numSms() * 4, 32 * kWindWarps, 0, st>>>(L, sorted, nt, list, count,
+                                                                  inside, nullptr);
+    ok = ok && launchOk();
+    kMeshSign<<<vBlocks, 256, 0, st>>>(m->vert, dist, L, inside);
+  } else {
+    kMeshWinding<true><<<numSms() * 4, 32 * kWindWarps, 0, st>>>(L, sorted, nt, nullptr, nullptr,
+                                                                 nullptr, m->vert);
+  }
   ok = ok && launchOk() && cudaOk(cudaStreamSynchronize(st));
   cudaFree(buf);
   return ok;
