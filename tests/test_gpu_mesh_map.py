@@ -73,3 +73,31 @@ def test_mesh_map_forms_match_fp64_oracle(nu, nv, cells, form):
     assert np.abs(np.linalg.norm(coords - gcp, axis=1) - np.abs(d)).max() <= 2e-6
     on, _ = mo.mesh_distance(gcp, verts, tris)
     assert np.abs(on).max() <= 2e-6
+
+
+def test_mesh_map_that_leaves_no_room_for_its_roots():
+    """Device memory for the map and less than the sign roots' list beside it: the
+    same map, every vertex's sign from its own solid angles."""
+    import torch
+    from fullc0ntact_gb300 import dem, scenes
+    verts, tris = scenes.torus_mesh(0.3, 0.1, 24, 10)
+    cells = 240
+    dem.DistanceMap.from_mesh(verts, tris[: len(tris) * 2 // 3], 24, 0.05)  # loads both ways' kernels
+    want = dem.DistanceMap.from_mesh(verts, tris, cells, 0.05).vertices()
+    nv = want.shape[0]  # 16 bytes a vertex for the map, 13 for the list and the distances
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    hog = torch.empty(free - nv * 16 - nv * 7, dtype=torch.uint8, device="cuda")
+    try:
+        if torch.cuda.mem_get_info()[0] >= nv * 29:
+            pytest.skip("another process gave memory back")
+        m = dem.DistanceMap.from_mesh(verts, tris, cells, 0.05)
+        dem.check("mesh map")
+        got = m.vertices()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    np.testing.assert_array_equal(np.abs(got), np.abs(want))
+    sure = np.abs(want[:, 0]) > 1e-5
+    np.testing.assert_array_equal(got[sure], want[sure])
