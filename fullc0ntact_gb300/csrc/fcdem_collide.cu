@@ -600,10 +600,12 @@ __device__ __forceinline__ bool groupListed(unsigned i, unsigned a, unsigned h,
 // collide: 4.2M spheres 490 against 748 us, 1M in piles 245 against 395, 1M
 // falling monodisperse 67 against 121.  All lanes scan the same row at a time:
 // skipping a lane's empty rows costs L1 hits (+13%).  56 registers (9 CTAs
-// per SM) against 72: -4%; 48 are slower again.  Shared memory is kept small because L1 gets the
+// per SM) against 72: -4%; 48 are slower again.  In Morton order, where every
+// particle takes the general loop, 72 (kBlocks = 7) are better: 100,000 packed
+// spheres, four updates 271 against 288 us.  Shared memory is kept small because L1 gets the
 // rest of the 256 KB (31 KB per CTA instead of 17: +6%).
-template <int kMode, bool kRadiusFromW, bool kCollider, bool kForceOut, bool kPrefix>
-__global__ void __launch_bounds__(128, 9)
+template <int kMode, bool kRadiusFromW, bool kCollider, bool kForceOut, bool kPrefix, int kBlocks>
+__global__ void __launch_bounds__(128, kBlocks)
 kCollideGlobal(float4 *__restrict__ newVel, const float4 *__restrict__ sortedPos,
                const float4 *__restrict__ sortedVel, const unsigned *__restrict__ index,
                CellRanges cells, unsigned n, KParams kp, CollideOut out, bool cull,
@@ -688,7 +690,10 @@ kCollideRows(float4 *newVel, const float4 *sortedPos, const float4 *sortedVel,
   const unsigned who = lane / 9u, row = lane % 9u;
   const unsigned i = (blockIdx.x * kRowsWarps + warp) * 3u + who;
   const bool active = who < 3u && i < n;
-  chainTrigger();
+  // With a crowd list the next kernel is kCollideCrowd, whose few busy CTAs would
+  // be placed, several to an SM, where this kernel's first CTAs leave (16,384
+  // spheres in eight cells, two updates: 8.0 against 4.8 ms): it starts after them.
+  if (!crowd.groups) chainTrigger();
   chainWait();
   const float4 p4 = active ? sortedPos[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   const float4 v4 = active ? sortedVel[i] : p4;
@@ -819,7 +824,7 @@ kCollideRows(float4 *newVel, const float4 *sortedPos, const float4 *sortedVel,
 // near partners in order; the drain then runs the exact test and the contact
 // terms with the lanes that have queued partners, all from shared memory.
 template <int kMode, bool kRadiusFromW, bool kCollider, bool kForceOut, bool kPrefix>
-__global__ void __launch_bounds__(kCrowdWarps * 32)
+__global__ void __launch_bounds__(kCrowdWarps * 32, 1)  // (left out: 64 registers, +4%)
 kCollideCrowd(float4 *newVel, const float4 *sortedPos,
               const float4 *sortedVel, const unsigned *index,
               CellRanges cells, unsigned n, KParams kp, CollideOut out, bool cull,
@@ -918,7 +923,7 @@ kCollideCrowd(float4 *newVel, const float4 *sortedPos,
             const float cd = kRadiusFromW ? ri + q4.w : cdMono;
             if (dist < cd) {
               const float4 w4 = cVel[t];
-              const float3 f = contactTerm(rel, dist, cd, vel, make_float3(w4.x, w4.y, w4.z),
+              const float3 f = contactTerm<true>(rel, dist, cd, vel, make_float3(w4.x, w4.y, w4.z),
                                            P.attraction, P);
               cf.x = cf.x + f.x;
               cf.y = cf.y + f.y;
@@ -1232,13 +1237,20 @@ void launchT(bool tiled, bool cull, unsigned n, float4 *newVel, const float4 *sp
       launchChained(true, kCollideRows<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix>,
                     (n + 3 * kRowsWarps - 1) / (3 * kRowsWarps), 32 * kRowsWarps, 0, newVel, sp, sv,
                     index, cells, n, kp, out, cull, crowd, ctx().dStatus);
+    else if (kp.p.maxParticlesPerCell & kMortonOrder)
+      kCollideGlobal<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix, 7>
+          <<<blocks, 128, 0, curStream()>>>(newVel, sp, sv, index, cells, n, kp, out, cull, crowd,
+                                            ctx().dStatus);
     else  // not chained: read-only loads (gas of 4.2M spheres -2%, box batches -4%)
-      kCollideGlobal<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix>
+      kCollideGlobal<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix, 9>
           <<<blocks, 128, 0, curStream()>>>(newVel, sp, sv, index, cells, n, kp, out, cull, crowd,
                                             ctx().dStatus);
     if (crowd.groups && launchOk()) {
-      // groups have up to 32 members: no more warps than that can be busy
-      const unsigned most = (n + 32 * kCrowdWarps - 1) / (32 * kCrowdWarps);
+      // Groups have up to 32 members, and each crowded cell one that may have
+      // fewer: with a warp for every 32 particles the last few groups of 1,000 or
+      // 16,384 spheres in eight cells had to wait for a second round, which
+      // doubled the time.
+      const unsigned most = 4u * ((n + 32 * kCrowdWarps - 1) / (32 * kCrowdWarps));
       const unsigned all = numSms() * g_crowdCtasPerSm;
       launchChained(true, kCollideCrowd<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix>,
                     most < all ? most : all, kCrowdWarps * 32, 0, newVel, sp, sv, index, cells, n,

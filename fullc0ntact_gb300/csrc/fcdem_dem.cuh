@@ -140,16 +140,19 @@ __device__ __forceinline__ void integrateOneBox(float3 &p, float3 &v, float dt, 
 
 // The force of particles_kernel.cu:185-218 (collideSpheres) once the
 // distance test has passed: rel = pB - pA, dist = |rel|, cd = rA + rB.
-// norm = rel / dist (as rel * (1 / dist), the correctly rounded reciprocal); tanVel = relVel - dot(relVel,
+// norm = rel / dist (as rel * (1 / dist), the correctly rounded reciprocal; kDivide:
+// from a division, the same bits, which suits kCollideCrowd: 24,577 spheres in
+// eight cells 5.26 against 5.46 ms; box batches take 2% longer with it); tanVel = relVel - dot(relVel,
 // norm) * norm; force = -spring (cd - dist) norm + damping relVel + shear
 // tanVel + attraction rel.  The fusions are the ones nvcc forms from the
 // reference's expressions: in `a * b + c * d` the left product is fused
 // with the right one as addend; in `x + a * b` the product is fused.
+template <bool kDivide = false>
 __device__ __forceinline__ float3 contactTerm(float3 rel, float dist, float cd,
                                               float3 vA, float3 vB,
                                               float attraction,
                                               const SimParams &P) {
-  const float inv = __frcp_rn(dist);
+  const float inv = kDivide ? __fdiv_rn(1.0f, dist) : __frcp_rn(dist);
   const float3 nrm = make_float3(__fmul_rn(rel.x, inv), __fmul_rn(rel.y, inv),
                                  __fmul_rn(rel.z, inv));
   const float3 rv = make_float3(__fsub_rn(vB.x, vA.x), __fsub_rn(vB.y, vA.y),
