@@ -4,7 +4,8 @@
 // above 1/2), and that closest point as the contact point -- what
 // DistanceMapMesh::ComputeDistance (distancegridcgal.hpp:36-69) stores.
 //
-// Neither part looks at every pair of a lattice vertex and a triangle:
+// Beyond a few triangles (kMeshFew) neither part looks at every pair of a lattice
+// vertex and a triangle:
 //
 //   * closest point: the triangles are put in Morton order of their centroids
 //     and cut into clusters of 32 with a bounding box each.  A warp takes a
@@ -278,6 +279,45 @@ kMeshNearest(float4 *__restrict__ vert, float *__restrict__ dist, Lattice L,
   }
 }
 
+// Few triangles: one thread per lattice vertex evaluates all of them, from shared
+// memory.  There the sort, the clusters and the sign's passes cost more than they
+// save.  One map, few / clusters: 18 triangles on 8 and 128 cells 72 / 142 and 331 /
+// 826 us, 128 on 128 cells 873 / 924, 256 on 32 and 128 cells 164 / 210 and 1,464 /
+// 973, 480 on 32 cells 259 / 267, 1,024 on 8 cells 403 / 397.  So it takes up to 128
+// triangles, and up to 512 on lattices of at most 65,536 vertices.
+constexpr unsigned kFewTriangles = 512;
+__host__ inline bool fewTriangles(unsigned nt, long long vertices) {
+  return nt <= 128u || (nt <= kFewTriangles && vertices <= 65536);
+}
+__global__ void __launch_bounds__(128)
+kMeshFew(float4 *__restrict__ vert, Lattice L, const float4 *__restrict__ tri, unsigned nt) {
+  __shared__ float4 sTri[3 * kFewTriangles];
+  for (unsigned e = threadIdx.x; e < 3 * nt; e += blockDim.x) sTri[e] = __ldg(tri + e);
+  __syncthreads();
+  const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= (long long)L.vx * L.vy * L.vz) return;
+  const float3 p = latticePoint(L, (int)(v % L.vx), (int)(v / L.vx % L.vy),
+                                (int)(v / ((long long)L.vx * L.vy)));
+  float best = 3.4e38f, omega = 0.0f;
+  float3 bestCp = p;
+  for (unsigned q = 0; q < nt; ++q) {
+    const float4 a4 = sTri[3 * q], b4 = sTri[3 * q + 1], c4 = sTri[3 * q + 2];
+    const float3 a = make_float3(a4.x, a4.y, a4.z), b = make_float3(b4.x, b4.y, b4.z),
+                 c = make_float3(c4.x, c4.y, c4.z);
+    const float3 cp = closestOnTriangle(p, a, b, c);
+    const float dx = p.x - cp.x, dy = p.y - cp.y, dz = p.z - cp.z;
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    if (d2 < best) {  // (of equal distances the first triangle's)
+      best = d2;
+      bestCp = cp;
+    }
+    omega += solidAngle(p, a, b, c);
+  }
+  const float d = sqrtf(best);
+  const bool inside = omega > 2.0f * 3.14159265358979f;  // winding number > 1/2
+  vert[v] = make_float4(inside ? -d : d, bestCp.x, bestCp.y, bestCp.z);
+}
+
 // The lower neighbour whose sign vertex v shares, or -1 (v is a root): the
 // segment between the two is shorter than one end's distance to the mesh.
 __device__ __forceinline__ long long signParent(const float *__restrict__ dist, const Lattice &L,
@@ -402,8 +442,12 @@ bool meshMap(fcdemDistanceMap *m, const float4 *tri, unsigned nt, const float *v
   const Lattice L{m->cells[0] + 1, m->cells[1] + 1, m->cells[2] + 1,
                   make_float3(m->vmin[0], m->vmin[1], m->vmin[2]), m->cellSize};
   const long long total = (long long)L.vx * L.vy * L.vz;
-  const unsigned clusters = (nt + kCluster - 1) / kCluster;
   cudaStream_t st = curStream();
+  if (fewTriangles(nt, total)) {
+    kMeshFew<<<(unsigned)((total + 127) / 128), 128, 0, st>>>(m->vert, L, tri, nt);
+    return launchOk() && cudaOk(cudaStreamSynchronize(st));
+  }
+  const unsigned clusters = (nt + kCluster - 1) / kCluster;
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const size_t sortedAt = al((size_t)nt * 8), boxAt = sortedAt + al((size_t)nt * 48),
                listAt = boxAt + al((size_t)clusters * 32), distAt = listAt + al((size_t)total * 8),

@@ -75,6 +75,32 @@ def test_mesh_map_forms_match_fp64_oracle(nu, nv, cells, form):
     assert np.abs(on).max() <= 2e-6
 
 
+@pytest.mark.parametrize("cells", [12, 44, 80])
+@pytest.mark.parametrize("nu,nv", [(3, 3), (8, 8), (13, 5), (16, 16), (43, 6)])
+def test_meshes_of_few_triangles(nu, nv, cells):
+    """18, 128, 130, 512 and 516 triangles on lattices below and above 65,536
+    vertices, closed and with a boundary: both kernels' maps against the FP64
+    oracle at a sample of the vertices."""
+    from fullc0ntact_gb300 import dem, scenes
+    from oracle import mesh_oracle as mo
+    from oracle import oracle as O
+    verts, tris = scenes.torus_mesh(0.3, 0.1, nu, nv)
+    for part in (len(tris), len(tris) - 2):
+        m = dem.DistanceMap.from_mesh(verts, tris[:part], cells, 0.05)
+        dem.check("mesh map")
+        coords = O.lattice_coords(m.vmin, m.cell_size, m.cells).astype(np.float64)
+        pick = np.random.default_rng(nu).permutation(len(coords))[:4000]
+        v, x = m.vertices()[pick], coords[pick]
+        d, _ = mo.mesh_distance(x, verts, tris[:part])
+        assert np.abs(np.abs(v[:, 0]) - np.abs(d)).max() <= 2e-6
+        V = verts.astype(np.float64)[tris[:part]]
+        wind = mo.winding_number(x, V[:, 0], V[:, 1], V[:, 2])
+        sure = (np.abs(d) > 1e-5) & (np.abs(wind - 0.5) > 1e-3)
+        assert np.all((v[sure, 0] < 0) == (wind[sure] > 0.5))
+        gap = np.linalg.norm(x - v[:, 1:].astype(np.float64), axis=1) - np.abs(d)
+        assert np.abs(gap).max() <= 2e-6
+
+
 def test_mesh_map_that_leaves_no_room_for_its_roots():
     """Device memory for the map and less than the sign roots' list beside it: the
     same map, every vertex's sign from its own solid angles."""
