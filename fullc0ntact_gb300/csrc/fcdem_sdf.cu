@@ -152,7 +152,11 @@ kSdfSamples(MapView M, float4 *__restrict__ out, int *__restrict__ shapeOut, int
 // same bits every time; the loss alone is summed sample by sample).  3 -> 64 ->
 // 64 -> 64 -> 1, batches of 2,048 samples: 17 us a batch against 67 us with
 // tiles of 64 samples (32 CTAs), weights read from L2 and a gradient added with
-// 277,000 atomics.
+// 277,000 atomics.  With more tiles than SMs the eight warps of a width-64 CTA
+// leave the SM idle in every layer's latency, and two CTAs share it (kCtas, 128
+// registers a thread): three layers, one batch of 262,144 samples 781 against 981
+// us.  With a tile each the registers' spills would cost more (two layers, 32
+// batches of 2,048 samples 457 against 353 us).
 constexpr int kTrainS = 16;
 
 // Floats of one row of gradient sums: the parameters, rounded up to 16 bytes
@@ -177,8 +181,8 @@ struct TrainSmem {
 // kBackward: the CTA's sums of invB * the gradient of sum_s w (y - t)^2 go to
 // partial[blockIdx.x] and the loss terms are added to *lossSum; otherwise
 // writes the distance prediction to yOut.
-template <int H, int L, bool kBackward>
-__global__ void __launch_bounds__(4 * H, 1)
+template <int H, int L, bool kBackward, int kCtas>
+__global__ void __launch_bounds__(4 * H, kCtas)
 kSdfTrain(SdfView net, const float4 *samples, const int *shapes,
           unsigned n, float band, float invB, float *partial,
           float *lossSum, float *yOut) {
@@ -1095,7 +1099,7 @@ struct fcdemSdfNet {
   float shift[3] = {0.0f, 0.0f, 0.0f}, scale[3] = {1.0f, 1.0f, 1.0f}, outScale = 1.0f;
   float *params = nullptr, *grad = nullptr, *m = nullptr, *v = nullptr;
   float *loss = nullptr;  // one device float
-  float *partial = nullptr;  // kSdfTrain: numSms() rows of gradient sums (first training call)
+  float *partial = nullptr;  // kSdfTrain: rows of gradient sums (first training call)
   __nv_bfloat16 *w16 = nullptr;
   bool w16Fresh = false;
   unsigned adamStep = 0;
@@ -1181,8 +1185,10 @@ bool runTrainKernel(fcdemSdfNet *net, bool backward, const float4 *samples, cons
                     unsigned n, float band, float invB, float *yOut, unsigned *parts = nullptr,
                     bool chained = false) {
   const unsigned sms = numSms();
+  const int H = net->lay.H, L = net->lay.L;
+  const unsigned rows = H == 64 ? 2u * sms : sms;  // CTAs of a backward pass at most
   if (backward && !net->partial &&
-      cudaMalloc(&net->partial, sizeof(float) * (size_t)sms * partialRow(net->lay.total)) !=
+      cudaMalloc(&net->partial, sizeof(float) * (size_t)rows * partialRow(net->lay.total)) !=
           cudaSuccess) {
     cudaGetLastError();
     net->partial = nullptr;
@@ -1190,25 +1196,32 @@ bool runTrainKernel(fcdemSdfNet *net, bool backward, const float4 *samples, cons
     return false;
   }
   const SdfView v = sdfView(net);
-  const int H = net->lay.H, L = net->lay.L;
   const unsigned tiles = (n + kTrainS - 1) / kTrainS;
-  // one CTA per SM (its row of partial sums); two of the narrow ones forward
-  const unsigned most = backward || H != 64 ? sms : 2u * sms;
+  // one CTA per SM, two of the narrow ones forward and where there are tiles for
+  // them (kTrainS)
+  const bool two = H == 64 && tiles > sms;
+  const unsigned most = H == 64 ? 2u * sms : sms;
   const unsigned blocks = tiles < most ? tiles : most;
   if (parts) *parts = blocks;
 #define FCDEM_SDF_TRAIN(HH, LL)                                                               \
   if (H == HH && L == LL) {                                                                   \
     constexpr int smem = (int)sizeof(TrainSmem<HH, LL>);                                      \
     static_assert(smem <= 227 * 1024, "shared memory of a CTA");                              \
-    if (backward) {                                                                           \
+    if (backward && two) {                                                                    \
       static std::atomic<unsigned long long> ready{0};                                        \
-      if (!smemReady(kSdfTrain<HH, LL, true>, smem, ready)) return false;                     \
-      launchChained(chained, kSdfTrain<HH, LL, true>, blocks, 4 * HH, smem, v, samples,       \
+      constexpr int kCtas = HH == 64 ? 2 : 1;                                                 \
+      if (!smemReady(kSdfTrain<HH, LL, true, kCtas>, smem, ready)) return false;              \
+      launchChained(chained, kSdfTrain<HH, LL, true, kCtas>, blocks, 4 * HH, smem, v,         \
+                    samples, shapes, n, band, invB, net->partial, net->loss, nullptr);        \
+    } else if (backward) {                                                                    \
+      static std::atomic<unsigned long long> ready{0};                                        \
+      if (!smemReady(kSdfTrain<HH, LL, true, 1>, smem, ready)) return false;                  \
+      launchChained(chained, kSdfTrain<HH, LL, true, 1>, blocks, 4 * HH, smem, v, samples,    \
                     shapes, n, band, invB, net->partial, net->loss, nullptr);                 \
     } else {                                                                                  \
       static std::atomic<unsigned long long> ready{0};                                        \
-      if (!smemReady(kSdfTrain<HH, LL, false>, smem, ready)) return false;                    \
-      launchChained(false, kSdfTrain<HH, LL, false>, blocks, 4 * HH, smem, v, samples,        \
+      if (!smemReady(kSdfTrain<HH, LL, false, 1>, smem, ready)) return false;                 \
+      launchChained(false, kSdfTrain<HH, LL, false, 1>, blocks, 4 * HH, smem, v, samples,     \
                     shapes, n, band, invB, nullptr, nullptr, yOut);                           \
     }                                                                                         \
     return launchOk();                                                                        \
