@@ -693,7 +693,9 @@ kCollideRows(float4 *newVel, const float4 *sortedPos, const float4 *sortedVel,
   // With a crowd list the next kernel is kCollideCrowd, whose few busy CTAs would
   // be placed, several to an SM, where this kernel's first CTAs leave (16,384
   // spheres in eight cells, two updates: 8.0 against 4.8 ms): it starts after them.
-  if (!crowd.groups) chainTrigger();
+  // (In a call's last step of few particles, where most SMs are free anyway, the
+  // overlap is worth a microsecond.)
+  if (!crowd.groups || (kMode == 3 && n <= 4096u)) chainTrigger();
   chainWait();
   const float4 p4 = active ? sortedPos[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   const float4 v4 = active ? sortedVel[i] : p4;
