@@ -825,8 +825,11 @@ kCollideRows(float4 *newVel, const float4 *sortedPos, const float4 *sortedVel,
 // with broadcast loads, tests the squared distance and queues each lane's
 // near partners in order; the drain then runs the exact test and the contact
 // terms with the lanes that have queued partners, all from shared memory.
-template <int kMode, bool kRadiusFromW, bool kCollider, bool kForceOut, bool kPrefix>
-__global__ void __launch_bounds__(kCrowdWarps * 32, 1)  // (left out: 64 registers, +4%)
+// kFew: three CTAs per SM hold all groups, so 76 registers are free; otherwise the
+// compiler's 64 are better (two updates of 24,577 spheres in eight cells 7.24 / 7.55
+// ms, of 100,000 in a ball 1.18 / 1.29, of 200,000 4.25 / 3.45).
+template <int kMode, bool kRadiusFromW, bool kCollider, bool kForceOut, bool kPrefix, bool kFew>
+__global__ void __launch_bounds__(kCrowdWarps * 32, kFew ? 1 : 0)
 kCollideCrowd(float4 *newVel, const float4 *sortedPos,
               const float4 *sortedVel, const unsigned *index,
               CellRanges cells, unsigned n, KParams kp, CollideOut out, bool cull,
@@ -925,8 +928,8 @@ kCollideCrowd(float4 *newVel, const float4 *sortedPos,
             const float cd = kRadiusFromW ? ri + q4.w : cdMono;
             if (dist < cd) {
               const float4 w4 = cVel[t];
-              const float3 f = contactTerm<true>(rel, dist, cd, vel, make_float3(w4.x, w4.y, w4.z),
-                                           P.attraction, P);
+              const float3 f = contactTerm<kFew>(
+                  rel, dist, cd, vel, make_float3(w4.x, w4.y, w4.z), P.attraction, P);
               cf.x = cf.x + f.x;
               cf.y = cf.y + f.y;
               cf.z = cf.z + f.z;
@@ -1254,7 +1257,10 @@ void launchT(bool tiled, bool cull, unsigned n, float4 *newVel, const float4 *sp
       // doubled the time.
       const unsigned most = 4u * ((n + 32 * kCrowdWarps - 1) / (32 * kCrowdWarps));
       const unsigned all = numSms() * g_crowdCtasPerSm;
-      launchChained(true, kCollideCrowd<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix>,
+      const bool few = n <= 3u * 32u * kCrowdWarps * numSms();
+      launchChained(true,
+                    few ? kCollideCrowd<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix, true>
+                        : kCollideCrowd<kMode, kRadiusFromW, kCollider, kForceOut, kPrefix, false>,
                     most < all ? most : all, kCrowdWarps * 32, 0, newVel, sp, sv, index, cells, n,
                     kp, out, cull, crowd, ctx().dStatus);
     }

@@ -141,8 +141,8 @@ __device__ __forceinline__ void integrateOneBox(float3 &p, float3 &v, float dt, 
 // The force of particles_kernel.cu:185-218 (collideSpheres) once the
 // distance test has passed: rel = pB - pA, dist = |rel|, cd = rA + rB.
 // norm = rel / dist (as rel * (1 / dist), the correctly rounded reciprocal; kDivide:
-// from a division, the same bits, which suits kCollideCrowd: 24,577 spheres in
-// eight cells 5.26 against 5.46 ms; box batches take 2% longer with it); tanVel = relVel - dot(relVel,
+// from a division, the same bits, which suits the crowded kernel of small scenes:
+// 24,577 spheres in eight cells 5.26 against 5.46 ms; box batches take 2% longer); tanVel = relVel - dot(relVel,
 // norm) * norm; force = -spring (cd - dist) norm + damping relVel + shear
 // tanVel + attraction rel.  The fusions are the ones nvcc forms from the
 // reference's expressions: in `a * b + c * d` the left product is fused

@@ -425,3 +425,27 @@ def test_crowded_cell_whose_first_members_moved_away(many):
     dem.check("collide")
     assert np.isfinite(want).all()
     np.testing.assert_array_equal(out.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("poly", [False, True])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_crowded_kernel_of_few_and_of_many_groups(extra, poly):
+    """The largest scene of the form for few groups and the smallest of the other,
+    many of its neighbourhoods crowded: the same bits as without the crowded path."""
+    from fullc0ntact_gb300 import dem, scenes
+    n = 3 * 256 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    sc = scenes.random_box(n, grid=(64, 64, 64), radius=1.0 / 64.0, seed=1, cell=1.0 / 32.0, poly=poly)
+    sc["pos"][:, :3] = np.random.default_rng(n).uniform(-0.3, -0.05, (n, 3))
+    got = []
+    for on in (1, 0):
+        dem.lib.fcdemSetCrowdPath(on)
+        try:
+            ds = dem.DeviceScene(sc)
+            ds.update(2)
+            dem.check("update")
+            got.append((ds.pos.cpu().numpy(), ds.vel.cpu().numpy()))
+        finally:
+            dem.lib.fcdemSetCrowdPath(1)
+            dem.set_radius_mode(False)
+    for a, b in zip(*got):
+        np.testing.assert_array_equal(a.view(np.uint32), b.view(np.uint32))
