@@ -1148,10 +1148,12 @@ static bool sortBuffers(Context &c, unsigned n, int bits, CountBuffers &b) {
 // sort then takes the pairs.
 // Five short passes instead of a histogram and three look-back passes of eight
 // bits, whose chain over the tiles is what they wait for.  A staged step with
-// it / with the radix sort: 5,000 spheres 39 / 60 us, 100,003 75 / 89, 1M in
-// lattice order 159 / 204, 1M in random order 245 / 252, 4.2M 901 / 892 (hence
-// the bound).  The fused step's buffers are others: it may run on another
-// stream.
+// it / with the radix sort: 3,000 spheres in a 64^3 grid 59 / 73 us, 100,003 packed
+// in a 128^3 grid 87 / 106, 1M falling in a 256^3 grid 188 / 210 (shuffled 198 /
+// 204), 2M packed there 427 / 437 (shuffled 449 / 448), 4.2M 901 / 892 (hence the
+// bound).  Spheres all over a 256^3 grid touch all of its 4,097 tiles: 300,000 take
+// 187 / 171 us, 1M 293 / 260; in a 128^3 grid 105 / 126 and 213 / 234.  The fused
+// step's buffers are others: it may run on another stream.
 bool countSortPairs(Context &c, unsigned *keys, unsigned *vals, unsigned n, int bits) {
   if (bits > kCountSortBits || n > kCountSortMax || (n >> bits) > kCountSortFill) return false;
   const unsigned cells = 1u << bits, mask = cells - 1u;

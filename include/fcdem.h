@@ -110,13 +110,13 @@ void calcHash(uint *gridParticleHash, uint *gridParticleIndex, float *pos,
 /* particleSystem.cu:265-270: stable ascending sort of (hash, index) in place.
  * Keys are expected below 2^ceil(log2(numCells)) of the current parameters;
  * a larger key records FCDEM_ERR_KEY_RANGE (the pairs stay whole, in an order
- * of their keys' low bits).  Up to 2,097,152 pairs with keys
- * of at most 24 bits, no more than 64 pairs per cell, are counted (a counting
- * sort over the cells), others take the radix sort.  The library keeps its buffers: some 40 bytes per pair
- * of the largest call, and 8 bytes per cell for each key width that was
- * counted (134 MB at 24 bits); where these cannot be had, the radix sort, which
- * needs about 17 bytes per pair, takes the call.  A captured graph that holds
- * the call is valid until a call with more pairs than any before it. */
+ * of their keys' low bits).  Up to 2,097,152 pairs with keys of at most 24
+ * bits and no more than 64 pairs per cell are counted (a counting sort over the
+ * cells), others take the radix sort.  The library keeps its buffers: some 40
+ * bytes per pair of the largest call, and 8 bytes per cell for each key width
+ * that was counted (134 MB at 24 bits); where these cannot be had, the radix
+ * sort, which needs about 17 bytes per pair, takes the call.  A captured graph
+ * that holds the call is valid until a call with more pairs than any before it. */
 void sortParticles(uint *dGridParticleHash, uint *dGridParticleIndex,
                    uint numParticles);
 
