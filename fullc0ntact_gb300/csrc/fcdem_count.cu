@@ -414,7 +414,7 @@ kFixupGather(const uint4 *slots, const unsigned *off, unsigned *hashOut, unsigne
 constexpr unsigned kGiants = 256, kGiantSlot = 1u << 31;
 struct Giants {
   unsigned *count;  // [giant][part]
-  unsigned *first;  // [giant]: first slot, or 0xffffffff
+  unsigned *first;  // [giant]: first slot, or 0xffffffff; [kGiants]: whether there are any
   unsigned least;   // pairs in a giant
   unsigned parts, part;  // parts of the arrays and their size
   // giants begin at least `least` slots apart
@@ -428,13 +428,14 @@ kCountKeys(const unsigned *keys, unsigned n, unsigned mask, unsigned *rank, unsi
   chainTrigger();
   chainWait();
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  for (unsigned k = i; k < kGiants * giants.parts; k += gridDim.x * blockDim.x) {
-    giants.count[k] = 0u;
-    if (k < kGiants) giants.first[k] = 0xffffffffu;
+  const unsigned k = i < n ? keys[i] : 0u, h = k & mask;
+  for (unsigned c = i; c < kGiants * giants.parts; c += gridDim.x * blockDim.x) {
+    giants.count[c] = 0u;
+    if (c < kGiants) giants.first[c] = 0xffffffffu;
+    if (c == 0u) giants.first[kGiants] = 0u;
   }
   const unsigned live = __ballot_sync(0xffffffffu, i < n), lane = threadIdx.x & 31u;
   if (i >= n) return;
-  const unsigned k = keys[i], h = k & mask;
   if (k != h) report(status, kStatusKeyRange);
   // Where two lanes in a row share a cell, one atomic for the members of the warp
   // that do: the pairs of a crowded cell would queue on its counter (2M pairs of
@@ -470,7 +471,10 @@ kScatterPairs(const unsigned *keys, const unsigned *vals, unsigned *rankN, const
   if (!giant) return;
   const unsigned id = giants.id(a), part = i / giants.part;
   rankN[i] = kGiantSlot | s;
-  if (r == 0u) giants.first[id] = a;
+  if (r == 0u) {
+    giants.first[id] = a;
+    giants.first[kGiants] = 1u;
+  }
   // (a warp may lie in two parts)
   const unsigned peers = __match_any_sync(inGiants, id * giants.parts + part);
   if ((int)lane == __ffs((int)peers) - 1)
@@ -681,11 +685,12 @@ kFixupLarge(uint4 *slots, const unsigned *off, const unsigned *large,
   chainTrigger();
   chainWait();
   __shared__ LargeSmem sm;
+  const unsigned count = min(large[0], largeCap);
   if (kPairs) {
     // this CTA's part of the arrays: the pairs in giants
-    const unsigned first = threadIdx.x < kGiants ? giants.first[threadIdx.x] : 0xffffffffu;
-    if (__syncthreads_or(first != 0xffffffffu)) {
+    if (giants.first[kGiants]) {
       if (threadIdx.x < kGiants) {
+        const unsigned first = giants.first[threadIdx.x];
         unsigned before = 0;
         if (first != 0xffffffffu)
           for (unsigned p = 0; p < blockIdx.x; ++p)
@@ -710,7 +715,6 @@ kFixupLarge(uint4 *slots, const unsigned *off, const unsigned *large,
           });
     }
   }
-  const unsigned count = min(large[0], largeCap);
   const int tid = threadIdx.x;
   const size_t words = bitmapWords(n);
   unsigned *bits = blockIdx.x < (unsigned)kBitmapSlots && bitmaps
@@ -1095,7 +1099,7 @@ static bool sortBuffers(Context &c, unsigned n, int bits, CountBuffers &b) {
   const size_t cellBytes = al(m * 4), tileBytes = al((size_t)tiles * 4);
   const size_t rankBytes = al((size_t)n * 4), slotBytes = al((size_t)n * 16),
                largeBytes = al(((size_t)largeCap + 1) * 4),
-               giantBytes = (size_t)kGiants * (largeCtas(n) + 1) * 4;
+               giantBytes = al(((size_t)kGiants * (largeCtas(n) + 1) + 1) * 4);
   const size_t pairBytes = std::max(rankBytes + 2 * slotBytes + largeBytes + giantBytes +
                                         (size_t)kBitmapSlots * 2 * bitmapWords(n) * 4,
                                     radixScratchBytes(n));
