@@ -503,8 +503,13 @@ kFixupPairs(const uint4 *slots, const unsigned *off, unsigned *keys, unsigned *v
     return;
   }
   unsigned r = 0;
+  if (b - a < 32u) {
+#pragma unroll 4
+    for (unsigned t = a; t < b; ++t) r += slots[t].y < w.y ? 1u : 0u;
+  } else {
 #pragma unroll 32  // eight slots a line: several lines on their way
-  for (unsigned t = a; t < b; ++t) r += slots[t].y < w.y ? 1u : 0u;
+    for (unsigned t = a; t < b; ++t) r += slots[t].y < w.y ? 1u : 0u;
+  }
   if (a + r >= n) return;
   keys[a + r] = w.x;
   vals[a + r] = w.z;
