@@ -152,11 +152,12 @@ kSdfSamples(MapView M, float4 *__restrict__ out, int *__restrict__ shapeOut, int
 // same bits every time; the loss alone is summed sample by sample).  3 -> 64 ->
 // 64 -> 64 -> 1, batches of 2,048 samples: 17 us a batch against 67 us with
 // tiles of 64 samples (32 CTAs), weights read from L2 and a gradient added with
-// 277,000 atomics.  With more tiles than SMs the eight warps of a width-64 CTA
-// leave the SM idle in every layer's latency, and two CTAs share it (kCtas, 128
-// registers a thread): three layers, one batch of 262,144 samples 781 against 981
-// us.  With a tile each the registers' spills would cost more (two layers, 32
-// batches of 2,048 samples 457 against 353 us).
+// 277,000 atomics.  In large batches the eight warps of a width-64 CTA leave the
+// SM idle in every layer's latency, and two CTAs share it (kCtas, 128 registers a
+// thread): one batch of 262,144 samples, two layers, 460 against 598 us, three layers
+// 783 against 981.  That is from 16 tiles per SM on; smaller batches keep the order of
+// their sums.  (With a tile each the registers' spills cost more: two layers, 32
+// batches of 2,048 samples 457 against 353 us.)
 constexpr int kTrainS = 16;
 
 // Floats of one row of gradient sums: the parameters, rounded up to 16 bytes
@@ -1197,10 +1198,9 @@ bool runTrainKernel(fcdemSdfNet *net, bool backward, const float4 *samples, cons
   }
   const SdfView v = sdfView(net);
   const unsigned tiles = (n + kTrainS - 1) / kTrainS;
-  // one CTA per SM, two of the narrow ones forward and where there are tiles for
-  // them (kTrainS)
-  const bool two = H == 64 && tiles > sms;
-  const unsigned most = H == 64 ? 2u * sms : sms;
+  // one CTA per SM, two of the narrow ones forward and in large batches (kTrainS)
+  const bool two = H == 64 && tiles > 16u * sms;
+  const unsigned most = H == 64 && (!backward || two) ? 2u * sms : sms;
   const unsigned blocks = tiles < most ? tiles : most;
   if (parts) *parts = blocks;
 #define FCDEM_SDF_TRAIN(HH, LL)                                                               \

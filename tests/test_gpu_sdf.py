@@ -125,6 +125,34 @@ def test_training_tiles_match_fp64_oracle(cfg, n):
     assert float((net.eval_f32(s, shapes) - ref).abs().max()) <= tol
 
 
+@pytest.mark.parametrize("cfg", [(3, 64, 2), (3, 64, 3), (11, 64, 3)])
+@pytest.mark.parametrize("more", [0, 1])
+def test_training_with_two_ctas_per_sm_matches_fp64_oracle(cfg, more):
+    """The largest batch of one CTA per SM and the smallest of two.  Tolerances of
+    the tests above; twice the same call gives the same gradient bits."""
+    from fullc0ntact_gb300 import sdf
+    n = 16 * 16 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    dmap = _torus()
+    net = _net(*cfg, dmap, jitter=0.05)
+    s = sdf.samples(dmap, n, 0.5, 0.05, seed=n)
+    shapes = None
+    if cfg[0] > 3:
+        shapes = (torch.arange(n, device="cuda") % (cfg[0] - 3)).to(torch.int32)
+    loss, g = net.gradient(s, shapes, 0.02)
+    shift, scale, out_scale = net.normalization()
+    lref, gref = so.loss_and_grad(net.get_params().astype(np.float64), so.layout(*cfg),
+                                  s.cpu().numpy().astype(np.float64),
+                                  None if shapes is None else shapes.cpu().numpy(),
+                                  0.02, shift, scale, out_scale)
+    # the loss is summed one by one in FP32: half a unit in the last place of the
+    # sum each time, in no fixed order
+    assert abs(loss - lref) <= n * 2.0 ** -24 * abs(lref)
+    err = np.abs(g.astype(np.float64) - gref)
+    assert np.max(err) <= 1e-4 * np.max(np.abs(gref))
+    assert np.linalg.norm(err) <= 1e-4 * np.linalg.norm(gref)
+    np.testing.assert_array_equal(net.gradient(s, shapes, 0.02)[1], g)
+
+
 @pytest.mark.parametrize("cfg", CONFIGS)
 def test_fp32_forward_matches_torch(cfg):
     from fullc0ntact_gb300 import sdf
