@@ -58,11 +58,11 @@ struct KParams {
   int radiusFromW;
 };
 
-// Per-device library state.
 // sortParticles counts keys of at most this many bits: 4096 tiles of cells,
 // whose counts kScanCellsOwn sums itself.
 constexpr int kCountSortBits = 24;
 
+// Per-device library state.
 struct Context {
   int device = -1;
   bool haveParams = false;
@@ -130,9 +130,9 @@ bool clearNow(void *device, int byte, size_t bytes);
 // wrote is read with plain loads: a __ldg or a const __restrict__ parameter
 // tells the compiler that the value never changes, and any __restrict__ one that
 // no other code, chainWait() included, changes it, and it may then load it
-// before chainWait(); so their parameters have none.  (kSdfTrain reads its samples before chainWait(); its
-// first launch of a call is not chained.)  Launched without the attribute the
-// two calls do nothing.
+// before chainWait(); so their parameters have none.  (kSdfTrain reads its
+// samples before chainWait(); its first launch of a call is not chained.)
+// Launched without the attribute the two calls do nothing.
 __device__ __forceinline__ void chainTrigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
